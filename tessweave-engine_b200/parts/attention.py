@@ -110,10 +110,21 @@ class PagedSoftmaxMixer(Mixer):
         if ops.tensor_core_attention_supported(self.runtime.dtype, self.head_dim, self.v_dim) and q.stride(0) % 8 == 0:
             self._attend_tensor_cores(ctx, out, q, cache, gate)
             return
+        only_single = None
+        longest = 0 if ctx.fixed_shape else max(ctx.host_q_len, default=0)     # (a captured step knows no row counts)
+        if ops.prefer_fp32_tiles(self.runtime.dtype, self.head_dim, self.v_dim, longest, max(ctx.host_kv_len, default=0)):
+            # requests with several tokens in tiles; those with one, if there are any, with the kernel below
+            ops.attention_fp32_tiles(out, q, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.seq_slot, cache.block_table,
+                                     cache.k_pages, cache.v_pages, ctx.n_seqs, longest, self.n_heads, self.n_kv_heads,
+                                     self.head_dim, self.reach, self.scale, ctx.status, sink=self.sink,
+                                     bias_by_distance=self.bias_by_distance, gate=gate)
+            if all(n > 1 for n in ctx.host_q_len):
+                return
+            only_single = ctx.seq_q_len
         ops.attention_generic(out, q, ctx.positions, ctx.seq_of_token, ctx.seq_slot, cache.block_table,
                               cache.k_pages, cache.v_pages, ctx.n_tokens, self.n_heads, self.n_kv_heads,
                               self.head_dim, self.reach, self.scale, ctx.status, sink=self.sink,
-                              bias_by_distance=self.bias_by_distance, gate=gate)
+                              bias_by_distance=self.bias_by_distance, gate=gate, only_single=only_single)
 
 
 @register_part("mixer", "gqa_attention")

@@ -177,6 +177,61 @@ def test_attention_generic_ragged_rows(dtype, hq, hkv, d, window):
         cursor += len(r)
 
 
+@pytest.mark.parametrize("hq,hkv,d", [(14, 2, 64), (4, 4, 32), (28, 4, 128), (5, 1, 100), (3, 3, 4)])
+@pytest.mark.parametrize("reach,terms", [(0, False), (70, False), (-48, False), (0, True)])
+def test_attention_fp32_tiles(hq, hkv, d, reach, terms):
+    """The 32-bit tile kernel against a dense softmax in 64 bits: portions that end at, before and behind the edges of the
+    64-row and 64-key tiles, portions behind a prefix, a request of one row (left alone), windows, chunks, and the terms.
+    The last position's value is infinite: rows that do not see it must not notice."""
+    lens, held = [2, 65, 1, 64, 130], [0, 63, 40, 64, 7]
+    totals = [a + b for a, b in zip(lens, held)]
+    setup = paged_setup(totals, 16, hkv, d, torch.float32, seed=hq + d)
+    g = torch.Generator().manual_seed(9)
+    n = sum(lens)
+    q = torch.randn(n, hq * d, generator=g)
+    sink = torch.randn(hq, generator=g) if terms else None
+    bias = torch.randn(40, hq, generator=g) if terms else None
+    gate = torch.rand(n, hq, generator=g) if terms else None
+    last = totals[4] - 1
+    setup["v_pages"][int(setup["table"][setup["slots"][4], last // 16]), :, last % 16] = float("inf")
+    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))                               # noqa: E731
+    out = torch.full((n, hq * d), -7.0, device="cuda")
+    st = status()
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    ops().attention_fp32_tiles(out, dev(q), i32(starts), i32(lens), i32(totals), i32(setup["slots"]), setup["table"],
+                               setup["k_pages"], setup["v_pages"], len(lens), max(lens), hq, hkv, d, reach, d ** -0.5, st,
+                               sink=dev(sink) if terms else None, bias_by_distance=dev(bias) if terms else None,
+                               gate=dev(gate) if terms else None)
+    assert int(st) == 0
+    for i, (a, m, h) in enumerate(zip(starts, lens, held)):
+        got = out[a:a + m].cpu().double().view(m, hq, d)
+        if m == 1:
+            assert torch.all(got == -7.0)
+            continue
+        kk, vv = (t.double().repeat_interleave(hq // hkv, 1) for t in (setup["k"][i], setup["v"][i]))
+        pos, key = (h + torch.arange(m))[:, None], torch.arange(totals[i])[None, :]
+        seen = key <= pos
+        if reach > 0:
+            seen &= key > pos - reach
+        if reach < 0:
+            seen &= key >= pos - pos % -reach
+        s = torch.einsum("rhd,nhd->hrn", q[a:a + m].double().view(m, hq, d), kk) * d ** -0.5
+        if terms:
+            s = s + bias.double()[(pos - key).clamp(0, bias.shape[0] - 1)].permute(2, 0, 1)
+        s = s.masked_fill(~seen, float("-inf"))
+        if terms:
+            s = torch.cat([s, sink.double()[:, None, None].expand(-1, m, 1)], -1)
+        p = torch.softmax(s, -1)[..., :totals[i]]
+        want = torch.einsum("hrn,nhd->rhd", p, vv)
+        if terms:
+            want = want * gate[a:a + m].double()[:, :, None]
+        if i == 4:
+            assert not torch.isfinite(got[-1]).any()
+            got, want = got[:-1], want[:-1]
+        # scores of size 1 from sums of up to 128 products, sums of up to 137 probabilities: some 2^-24 x 40 in all
+        assert float((got - want).abs().max()) < 4e-6, f"request {i}"
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("where", ["first_of_page", "last_of_page", "position_zero", "window_edge_inside", "window_edge_outside"])
 def test_attention_finds_one_far_key(dtype, where):
