@@ -68,6 +68,7 @@ struct RecArgs {
     const int* positions;
     const int* seq_slot; const int* seq_q_start; const int* seq_q_len;
     int H, Dv, write_state;
+    int below;                  // requests with this many rows or more are left alone (0: none are)
     int cols_per_block;         // columns of S a block owns (its first `cols_per_block` threads; all threads stage rows)
 };
 
@@ -92,7 +93,7 @@ linear_recurrence_kernel(RecArgs a) {
     tw_grid_launch_dependents();
     const int h = blockIdx.x, s = blockIdx.y;
     const int len = a.seq_q_len[s];
-    if (len <= 0) return;
+    if (len <= 0 || (a.below > 0 && len >= a.below)) return;
     const int start = a.seq_q_start[s];
     const int Dv = a.Dv, cols = MODE == TW_REC_MLSTM ? Dv + 1 : Dv;
     const int per = a.cols_per_block;
@@ -527,6 +528,7 @@ static int launch_recurrence(const RecArgs& a, int n_seqs, bool long_portions, c
     return launch_split<T, MODE, TW_REC_SHARES>(a, n_seqs, long_portions, stream);
 }
 
+// `below` > 0: requests with that many rows or more are left alone (recurrence_chunks.cu serves them).
 TW_EXPORT int tw_linear_recurrence(int mode, float* out, float* den, const void* q, int q_stride, const void* k, int k_stride,
                                    const void* v, int v_stride, const float* wpre, int wpre_stride, const float* p0,
                                    const float* p1, const float* p2, const float* bpre, int bpre_stride, int channel_decay, int qk_group,
@@ -534,7 +536,7 @@ TW_EXPORT int tw_linear_recurrence(int mode, float* out, float* den, const void*
                                    float cap, float* state, long long state_stride, const void* tail_src, int tail_stride,
                                    int tail_width, long long tail_offset, const int* positions, const int* seq_slot,
                                    const int* seq_q_start, const int* seq_q_len, int n_seqs, int H, int Dk, int Dv,
-                                   int write_state, int max_q_len, int dtype, cudaStream_t stream) {
+                                   int write_state, int max_q_len, int below, int dtype, cudaStream_t stream) {
     if (n_seqs <= 0 || H <= 0) return 0;
     const bool lp = max_q_len > TW_REC_CHUNK;
     if (Dk != TW_DK || Dv <= 0 || Dv > 256 || rot_dims < 0 || rot_dims > Dk || (rot_dims & 1)) return (int)cudaErrorInvalidValue;
@@ -546,7 +548,7 @@ TW_EXPORT int tw_linear_recurrence(int mode, float* out, float* den, const void*
     a.k_scale = k_scale; a.q_scale = q_scale; a.cap = cap; a.state = state; a.state_stride = state_stride;
     a.tail_src = tail_src; a.tail_stride = tail_stride; a.tail_width = tail_width; a.tail_offset = tail_offset;
     a.positions = positions; a.seq_slot = seq_slot; a.seq_q_start = seq_q_start; a.seq_q_len = seq_q_len;
-    a.H = H; a.Dv = Dv; a.write_state = write_state; a.cols_per_block = 0;
+    a.H = H; a.Dv = Dv; a.write_state = write_state; a.cols_per_block = 0; a.below = below;
     const bool f32 = dtype == TW_F32;
     switch (mode) {
     case TW_REC_RETENTION:

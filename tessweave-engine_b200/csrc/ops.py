@@ -1603,7 +1603,7 @@ def linear_recurrence(mode: int, out: torch.Tensor, den: torch.Tensor | None, q:
                       inv_freq: torch.Tensor | None = None, rot_dims: int = 0, q_scale: float = 1.0, k_scale: float = 1.0,
                       cap: float = 1.0, tail: torch.Tensor | None = None, tail_offset: int = 0, max_q_len: int = 1 << 30,
                       write_pre: torch.Tensor | None = None, channel_decay: bool = False, qk_group: int = 1,
-                      p2: torch.Tensor | None = None) -> None:
+                      p2: torch.Tensor | None = None, below: int = 0) -> None:
     """Walk every request's rows of the step through its matrix state (csrc/linear_recurrence.cu): ``out`` fp32
     [rows, heads * value_dim] receives the raw outputs, ``den`` fp32 [rows, heads] the mLSTM denominators.  q, k, v are
     column slices of the projected rows (heads side by side).  ``pre``: fp32 rows the rule needs beside them (wkv:
@@ -1617,7 +1617,8 @@ def linear_recurrence(mode: int, out: torch.Tensor, den: torch.Tensor | None, q:
     share a head of q and k.  Gated linear attention takes ``pre`` the projected decay [rows, heads * key_dim], ``p0`` its
     bias and ``cap`` the exponent 1 / tau of the sigmoid.  The state-space rule takes q, k, v that are ready to use,
     ``pre`` the projected step size [rows, heads], ``p0`` the log of each head's rate, ``p1`` the step size's bias and ``p2``
-    the skip, each [heads]; ``qk_group`` as in the delta rule."""
+    the skip, each [heads]; ``qk_group`` as in the delta rule.  ``below`` > 0: requests with that many rows or more are left
+    alone."""
     _cuda(out, den, q, k, v, state, positions, seq_slot, seq_q_start, seq_q_len, pre, p0, p1, p2, inv_freq, tail, write_pre)
     _need(mode != RECURRENCE_SSD or (pre is not None and pre.stride(1) == 1 and pre.shape[1] >= heads
                                      and all(p is not None and p.numel() == heads and p.is_contiguous() for p in (p0, p1, p2))
@@ -1650,8 +1651,58 @@ def linear_recurrence(mode: int, out: torch.Tensor, den: torch.Tensor | None, q:
         c_float(q_scale), c_float(k_scale), c_float(cap), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(tail),
         c_int(0 if tail is None else tail.stride(0)), c_int(0 if tail is None else tail.shape[1]), ctypes.c_longlong(tail_offset),
         _ptr(positions), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(key_dim),
-        c_int(value_dim), c_int(1 if write_state else 0), c_int(max_q_len), c_int(dtype_code(q.dtype)), _stream())
+        c_int(value_dim), c_int(1 if write_state else 0), c_int(max_q_len), c_int(below), c_int(dtype_code(q.dtype)), _stream())
     _check(code, "linear_recurrence")
+
+
+RECURRENCE_CHUNK = 64                   # tokens of a chunk (csrc/recurrence_chunks.cu)
+# Where a portion goes through the chunks' three launches.  14 heads of 128 x 128, mLSTM / retention: 26 / 33 us for up to 256
+# tokens (one wave of blocks), token by token 30 / 28 us for 96, 38 / 37 for 128, 71 for 256 (6 heads of 64: 18 and 36 for 128).
+RECURRENCE_CHUNK_MIN_TOKENS = 128
+
+
+def recurrence_chunks_supported(mode: int, dtype: torch.dtype, key_dim: int, value_dim: int, rot_dims: int = 0) -> bool:
+    """Whether csrc/recurrence_chunks.cu can take the long portions of a step."""
+    return (dtype == torch.bfloat16 and mode in (RECURRENCE_RETENTION, RECURRENCE_MLSTM) and key_dim in (32, 64, 128)
+            and value_dim in (64, 128) and rot_dims % 4 == 0)
+
+
+def recurrence_chunk_count(rows: int, n_seqs: int) -> int:
+    """The most chunks that portions of at least ``RECURRENCE_CHUNK_MIN_TOKENS`` rows, ``rows`` in all, are cut into."""
+    return rows // RECURRENCE_CHUNK + min(n_seqs, rows // RECURRENCE_CHUNK_MIN_TOKENS)
+
+
+def recurrence_chunks(mode: int, out: torch.Tensor, den: torch.Tensor | None, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
+                      state: torch.Tensor, positions: torch.Tensor, seq_slot: torch.Tensor, seq_q_start: torch.Tensor,
+                      seq_q_len: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int, max_q_len: int,
+                      chunk_state: torch.Tensor, chunk_gate: torch.Tensor, chunk_max: torch.Tensor, write_state: bool = True,
+                      pre: torch.Tensor | None = None, p0: torch.Tensor | None = None, inv_freq: torch.Tensor | None = None,
+                      rot_dims: int = 0, q_scale: float = 1.0, k_scale: float = 1.0, cap: float = 1.0) -> None:
+    """``linear_recurrence`` of the requests that bring ``RECURRENCE_CHUNK_MIN_TOKENS`` rows or more, in chunks on the tensor
+    cores (csrc/recurrence_chunks.cu): same operands and state, bfloat16 q, k, v.  The other requests are left alone.
+    ``chunk_state`` fp32 [chunks, heads * (key_dim * value_dim + key_dim)], ``chunk_gate`` fp64 [chunks, heads, 2] and
+    ``chunk_max`` fp32 [chunks, heads] are scratch for ``recurrence_chunk_count`` chunks."""
+    _cuda(out, den, q, k, v, state, positions, seq_slot, seq_q_start, seq_q_len, pre, p0, inv_freq, chunk_state, chunk_gate, chunk_max)
+    _need(recurrence_chunks_supported(mode, q.dtype, key_dim, value_dim, rot_dims if inv_freq is not None else 0),
+          "recurrence: the chunk kernels do not take this rule or these sizes")
+    _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == heads * value_dim, "recurrence: out must be fp32 [rows, H * Dv]")
+    _need(q.dtype == k.dtype == v.dtype and q.stride(1) == k.stride(1) == v.stride(1) == 1
+          and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)), "recurrence: q, k, v of one type, rows on 16-byte boundaries")
+    _need(state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1, "recurrence: state must be fp32 [slots, numel]")
+    for t in (pre, p0, inv_freq, den, chunk_state, chunk_max):
+        _need(t is None or t.dtype == torch.float32, "recurrence: constants, gates and denominators are fp32")
+    _need(p0 is not None and (mode != RECURRENCE_MLSTM or (den is not None and pre is not None)), "recurrence: gates and constants are missing")
+    chunks = recurrence_chunk_count(out.shape[0], n_seqs)
+    _need(chunk_gate.dtype == torch.float64 and chunk_state.numel() >= chunks * heads * key_dim * (value_dim + 1)
+          and chunk_gate.numel() >= chunks * heads * 2 and chunk_max.numel() >= chunks * heads, "recurrence: the chunks' scratch is too small")
+    code = _fn("recurrence_chunks", "tw_recurrence_chunks", {"TW_DK": key_dim})(
+        c_int(mode), _ptr(out), _ptr(den), _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), _ptr(v), c_int(v.stride(0)),
+        _ptr(pre), c_int(0 if pre is None else pre.stride(0)), _ptr(p0), _ptr(inv_freq), c_int(rot_dims), c_float(q_scale),
+        c_float(k_scale), c_float(cap), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(positions), _ptr(seq_slot),
+        _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(key_dim), c_int(value_dim),
+        c_int(RECURRENCE_CHUNK_MIN_TOKENS), c_int(max_q_len), c_int(1 if write_state else 0), _ptr(chunk_state), _ptr(chunk_gate),
+        _ptr(chunk_max), _stream())
+    _check(code, "recurrence_chunks")
 
 
 STATE_SPACE_CHUNK_STATES = (16, 32, 64, 128, 256)

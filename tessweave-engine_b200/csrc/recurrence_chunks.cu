@@ -1,0 +1,739 @@
+// Prompt portions of two of linear_recurrence.cu's rules -- retention (a constant decay per head, q and k rotated) and mLSTM
+// (exponential gates with a running maximum) -- in chunks of 64 tokens, on the tensor cores and in parallel over the chunks.
+//
+// With c(t, s) what token s contributes to the state a token t of its chunk reads, in(t) what is left there of the state S
+// before the chunk, and w(s), keep the same at the chunk's end,
+//
+//   o_t = in(t) S^T q_t + sum over s <= t of c(t, s) (q_t . k_s) v_s          S' = keep S + sum over s of w(s) k_s v_s^T
+//
+// Three launches: (1) every chunk's own sum of w k v^T; (2) the walk over the chunks, element by element of S, which
+// leaves the state before each chunk and the new one in the request's slot; (3) every chunk's outputs.
+//
+// What bounds the walk token by token is a chain of dependent steps (0.25 us each), whatever the GPU could do beside it;
+// here the chain is one multiply-add per chunk and element.  14 heads of 128 x 128 over
+// 2,048 tokens: mLSTM 522 us token by token, 66 in chunks (22 + 11 + 33 for the three launches); retention 472 and 85
+// (23 + 9 + 53).  A chunk's state takes 64 KB, 29 MB in all for these sizes, which stays in L2 between the launches.  64
+// tokens: at 32 the states' traffic doubles, at 128 the triangle of q . k does and its coefficients fill shared memory.
+//
+// Precision: nothing that was held in 32 bits is rounded to 16.  bf16 inputs enter a product as they are; what has 32 bits
+// (the state, the coefficients, rotated q and k) enters as the sum of three bf16 numbers, which hold its 24 bits, with a
+// product for each pair of terms that matters (mma.sync m16n8k16, fp32 sums).  2,048 tokens against 64 bits: outputs 2.1e-7
+// (token by token 2.2e-7) for mLSTM, 1.8e-7 (5.9e-7) for retention, its state 2.2e-7 (7.3e-7).  Exponents of coefficients are differences
+// of sums over a chunk; those sums are formed and kept in 64 bits, powers of a constant decay are multiplied up in 64 bits.
+#include "attention_common.cuh"
+
+#ifndef TW_DK
+#define TW_DK 128
+#endif
+
+namespace {
+
+typedef __nv_bfloat16 bf16;
+using tw_attn::ldmatrix_x4;
+using tw_attn::ldmatrix_x4_trans;
+using tw_attn::mma_bf16;
+
+enum : int { RC_RETENTION = 0, RC_MLSTM = 1 };
+constexpr int L = 64, DK = TW_DK, KT = DK / 16, RS = DK + 8, MS = L + 8, THREADS = 256, WARPS = 8;
+static_assert(DK == 32 || DK == 64 || DK == 128, "key sizes");
+
+struct RcArgs {
+    float* out; float* den;
+    const bf16* q; const bf16* k; const bf16* v; int q_stride, k_stride, v_stride;
+    const float* pre; int pre_stride;       // mlstm: [rows, 2 H] (input | forget)
+    const float* p0;                        // retention: decay [H]; mlstm: biases [2 H]
+    const float* inv_freq; int rot_dims;
+    float q_scale, k_scale, cap;
+    float* state; long long state_stride;
+    const int* positions; const int* seq_slot; const int* seq_q_start; const int* seq_q_len;
+    int n_seqs, H, min_len, write_state;
+    float* chunk_state;                     // [chunks, H][DV / 8][KT][32 lanes][4], then [DK] (mlstm): sums, then the state before
+    double2* chunk_gate;                    // [chunks, H] mlstm: (the forget gates' sum, the largest of i - that sum so far)
+    float* chunk_max;                       // [chunks, H] mlstm: the running maximum before the chunk
+};
+
+// (x, y) as three pairs of bf16 whose sum is the pair to 24 bits
+__device__ __forceinline__ void split3(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const float2 hf = __bfloat1622float2(h);
+    x -= hf.x; y -= hf.y;
+    const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
+    const float2 mf = __bfloat1622float2(m);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x - mf.x, y - mf.y);
+    a = *reinterpret_cast<const uint32_t*>(&h);
+    b = *reinterpret_cast<const uint32_t*>(&m);
+    c = *reinterpret_cast<const uint32_t*>(&l);
+}
+// A product of the leading terms: sixteen products summed by the tensor core, added to the running sum by an fp32 addition
+// that rounds to nearest (the tensor core's own additions truncate: chained over a whole sum they left errors of 2 to 3 times
+// the token kernel's).  The products of the smaller terms are chained (mma_bf16), in sums of their own or before the others.
+__device__ __forceinline__ void mma_top(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    float t[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_bf16(t, a, b0, b1);
+    d[0] += t[0]; d[1] += t[1]; d[2] += t[2]; d[3] += t[3];
+}
+
+// Chunks of the requests before s that are served here: where the request's own chunks start.
+__device__ __forceinline__ int first_chunk(const int* seq_q_len, int s, int min_len) {
+    int n = 0;
+    for (int r = threadIdx.x & 31; r < s; r += 32) {
+        const int len = seq_q_len[r];
+        n += len >= min_len ? (len + L - 1) / L : 0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    return n;
+}
+
+__device__ __forceinline__ float logsigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
+
+// The gates of a chunk, by the first warp (lane: tokens `lane` and `lane + 32`): F, the sum of the forget gates up to a
+// token, and G = i - F.  A token behind the chunk's last has f = 0 and i = -infinity.
+struct Gates { double f0, f1, g0, g1, m0, m1; };      // m: the largest G up to the token
+__device__ __forceinline__ Gates chunk_gates(const RcArgs& a, int h, size_t row0, int ct) {
+    const int lane = threadIdx.x & 31;
+    double f[2], i[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int t = lane + 32 * e;
+        float li = -INFINITY, lf = 0.f;
+        if (t < ct) {
+            const float* g = a.pre + (row0 + t) * a.pre_stride;
+            li = a.cap * tanhf((g[h] + a.p0[h]) / a.cap);
+            lf = logsigmoid(a.cap * tanhf((g[a.H + h] + a.p0[a.H + h]) / a.cap));
+        }
+        f[e] = lf; i[e] = li;
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double u0 = __shfl_up_sync(0xffffffffu, f[0], o), u1 = __shfl_up_sync(0xffffffffu, f[1], o);
+        if (lane >= o) { f[0] += u0; f[1] += u1; }
+    }
+    f[1] += __shfl_sync(0xffffffffu, f[0], 31);
+    Gates r;
+    r.f0 = f[0]; r.f1 = f[1]; r.g0 = i[0] - f[0]; r.g1 = i[1] - f[1];
+    double m0 = r.g0, m1 = r.g1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double u0 = __shfl_up_sync(0xffffffffu, m0, o), u1 = __shfl_up_sync(0xffffffffu, m1, o);
+        if (lane >= o) { m0 = fmax(m0, u0); m1 = fmax(m1, u1); }
+    }
+    m1 = fmax(m1, __shfl_sync(0xffffffffu, m0, 31));
+    r.m0 = m0; r.m1 = m1;
+    return r;
+}
+// powers 0 .. 64 of a head's decay, by the first warp
+__device__ __forceinline__ void decay_powers(float* pw, float decay) {
+    const int lane = threadIdx.x & 31;
+    double base = decay, p = 1.0;                       // decay^lane by squaring
+    for (int b = lane; b; b >>= 1) { if (b & 1) p *= base; base *= base; }
+    double p32 = 1.0, b32 = decay;
+    for (int b = 32; b; b >>= 1) { if (b & 1) p32 *= b32; b32 *= b32; }
+    pw[lane] = (float)p; pw[lane + 32] = (float)(p * p32);
+    if (lane == 0) pw[64] = (float)(p32 * p32);
+}
+
+// bf16 rows of a chunk (rows from `ct` on are zeros), 16 bytes per thread and step, all loads under way at once.
+template <int W>
+struct Rows {
+    static constexpr int N = L * (W / 8) / THREADS;
+    static_assert(N * THREADS == L * (W / 8), "rows divide evenly");
+    uint4 v[N];
+    __device__ __forceinline__ static int token(int e) { return (threadIdx.x + e * THREADS) / (W / 8); }
+    __device__ __forceinline__ static int channel(int e) { return (threadIdx.x + e * THREADS) % (W / 8) * 8; }
+    __device__ __forceinline__ void load(const bf16* src, int stride, int ct) {
+#pragma unroll
+        for (int e = 0; e < N; ++e)
+            v[e] = token(e) < ct ? *reinterpret_cast<const uint4*>(src + (size_t)token(e) * stride + channel(e)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    __device__ __forceinline__ void store(bf16* dst, int stride) const {
+#pragma unroll
+        for (int e = 0; e < N; ++e) *reinterpret_cast<uint4*>(dst + token(e) * stride + channel(e)) = v[e];
+    }
+    // values that are not finite become zeros; returns whether there were any
+    __device__ __forceinline__ bool keep_finite() {
+        bool found = false;
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            uint32_t* w = reinterpret_cast<uint32_t*>(&v[e]);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                if ((w[x] & 0x7f80u) == 0x7f80u) { w[x] &= 0xffff0000u; found = true; }
+                if ((w[x] & 0x7f800000u) == 0x7f800000u) { w[x] &= 0xffffu; found = true; }
+            }
+        }
+        return found;
+    }
+};
+__device__ __forceinline__ float2 pair_of(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+
+// Rows of q or k, scaled (and, for retention, rotated), times `weight` of the token, as three bf16 terms [3][L][RS].
+__device__ __forceinline__ void put3(bf16* dst, int t, int i, float x, float y) {
+    uint32_t hi, mid, lo;
+    split3(x, y, hi, mid, lo);
+    *reinterpret_cast<uint32_t*>(dst + t * RS + i) = hi;
+    *reinterpret_cast<uint32_t*>(dst + (L + t) * RS + i) = mid;
+    *reinterpret_cast<uint32_t*>(dst + (2 * L + t) * RS + i) = lo;
+}
+__device__ __forceinline__ void stage_plain(bf16* dst, const Rows<DK>& rows, float scale, const float* weight) {
+#pragma unroll
+    for (int e = 0; e < Rows<DK>::N; ++e) {
+        const int t = Rows<DK>::token(e), i = Rows<DK>::channel(e);
+        const float w = weight ? weight[t] : 1.f;
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(&rows.v[e]);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const float2 f = pair_of(p[x]);
+            put3(dst, t, i + 2 * x, f.x * scale * w, f.y * scale * w);
+        }
+    }
+}
+// Rotated: channels i, i + 1 with their partners i + half, i + half + 1 (rot_dims is a multiple of 4); channels from rot_dims
+// on are not rotated.
+__device__ __forceinline__ void stage_rotated(bf16* dst, const RcArgs& a, const bf16* src, int stride, size_t row0, int ct, float scale,
+                                              const float* weight) {
+    const int half = a.rot_dims >> 1, per = half / 2;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < L * per; e += THREADS) {
+        const int t = e / per, i = (e - t * per) * 2;
+        float x1 = 0.f, x2 = 0.f, y1 = 0.f, y2 = 0.f;
+        if (t < ct) {
+            const bf16* r = src + (size_t)t * stride;
+            const float2 lo = pair_of(*reinterpret_cast<const uint32_t*>(r + i)), hi = pair_of(*reinterpret_cast<const uint32_t*>(r + i + half));
+            const float pos = (float)a.positions[row0 + t], w = weight ? weight[t] : 1.f;
+            float sn, cs;
+            sincosf(pos * a.inv_freq[i], &sn, &cs);
+            x1 = (lo.x * cs - hi.x * sn) * scale * w; y1 = (hi.x * cs + lo.x * sn) * scale * w;
+            sincosf(pos * a.inv_freq[i + 1], &sn, &cs);
+            x2 = (lo.y * cs - hi.y * sn) * scale * w; y2 = (hi.y * cs + lo.y * sn) * scale * w;
+        }
+        put3(dst, t, i, x1, x2);
+        put3(dst, t, i + half, y1, y2);
+    }
+    const int first = a.rot_dims, plain = (DK - first) / 2;
+    for (int e = threadIdx.x; e < L * plain; e += THREADS) {
+        const int t = e / plain, i = first + (e - t * plain) * 2;
+        float2 v = make_float2(0.f, 0.f);
+        if (t < ct) v = pair_of(*reinterpret_cast<const uint32_t*>(src + (size_t)t * stride + i));
+        const float w = scale * (weight ? weight[t] : 1.f);
+        put3(dst, t, i, v.x * w, v.y * w);
+    }
+}
+
+// ---- (1) a chunk's own sum of w(s) k_s v_s^T, transposed: rows are columns of the state.  The weighted keys are staged as
+// three bf16 terms (3 x 64 x DK), the values as they are; a warp owns 16 values and all or half of the key channels.  Its
+// accumulators hold pairs of neighbouring key channels of one value, which is how (3) wants the state as an operand:
+// they go to memory in that order, 512 bytes per warp and store.
+template <int RULE, int DV>
+__global__ void __launch_bounds__(THREADS, 2) chunk_sums_kernel(RcArgs a) {
+    constexpr int VS = DV + 8, MT = DV / 16, WPM = WARPS / MT, PAIRS = KT / WPM;
+    static_assert(MT * WPM == WARPS && PAIRS * WPM == KT, "warps divide the state evenly");
+    extern __shared__ __align__(16) unsigned char rc_smem[];
+    bf16* kw = reinterpret_cast<bf16*>(rc_smem);            // [3][L][RS]
+    bf16* vs = kw + 3 * L * RS;                             // [L][VS]
+    __shared__ float weight[L];
+    __shared__ float pw[L + 1];
+    tw_grid_wait();
+    tw_grid_launch_dependents();
+    const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
+    const int len = a.seq_q_len[s];
+    if (len < a.min_len || c * L >= len) return;
+    const int ct = min(L, len - c * L);
+    const size_t row0 = (size_t)a.seq_q_start[s] + c * L;
+    const size_t at = (size_t)(first_chunk(a.seq_q_len, s, a.min_len) + c) * a.H + h;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bf16* krows = a.k + row0 * a.k_stride + (size_t)h * DK;
+    const bool rotate = RULE == RC_RETENTION && a.rot_dims > 0;
+    Rows<DV> vrows;
+    Rows<DK> kplain;
+    vrows.load(a.v + row0 * a.v_stride + (size_t)h * DV, a.v_stride, ct);
+    if (!rotate) kplain.load(krows, a.k_stride, ct);
+    if (warp == 0) {
+        if (RULE == RC_RETENTION) {
+            decay_powers(pw, a.p0[h]);
+            __syncwarp();
+            weight[lane] = lane < ct ? pw[ct - 1 - lane] : 0.f;
+            weight[lane + 32] = lane + 32 < ct ? pw[ct - 1 - (lane + 32)] : 0.f;
+        } else {
+            const Gates g = chunk_gates(a, h, row0, ct);
+            const double top = __shfl_sync(0xffffffffu, g.m1, 31), sum = __shfl_sync(0xffffffffu, g.f1, 31);
+            weight[lane] = lane < ct ? (float)exp(g.g0 - top) : 0.f;
+            weight[lane + 32] = lane + 32 < ct ? (float)exp(g.g1 - top) : 0.f;
+            if (lane == 0) a.chunk_gate[at] = make_double2(sum, top);
+        }
+    }
+    vrows.store(vs, VS);
+    __syncthreads();
+    if (rotate) stage_rotated(kw, a, krows, a.k_stride, row0, ct, a.k_scale, weight);
+    else stage_plain(kw, kplain, a.k_scale, weight);
+    __syncthreads();
+    const int mt = warp % MT, p0 = (warp / MT) * PAIRS;
+    float acc[2 * PAIRS][4];
+#pragma unroll
+    for (int j = 0; j < 2 * PAIRS; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+#pragma unroll
+    for (int term = 2; term >= 0; --term) {
+#pragma unroll
+        for (int k = 0; k < L / 16; ++k) {
+            uint32_t A[4], B[4];
+            ldmatrix_x4_trans(A, vs + (k * 16 + (lane & 7) + ((lane >> 4) << 3)) * VS + mt * 16 + ((lane >> 3) & 1) * 8);
+            const bf16* base = kw + (term * L + k * 16 + (lane & 15)) * RS + (lane >> 4) * 8;
+#pragma unroll
+            for (int p = 0; p < PAIRS; ++p) {
+                ldmatrix_x4_trans(B, base + (p0 + p) * 16);
+                if (term == 0) {
+                    mma_top(acc[2 * p], A, B[0], B[1]);
+                    mma_top(acc[2 * p + 1], A, B[2], B[3]);
+                } else {
+                    mma_bf16(acc[2 * p], A, B[0], B[1]);
+                    mma_bf16(acc[2 * p + 1], A, B[2], B[3]);
+                }
+            }
+        }
+    }
+    const size_t per_chunk = (size_t)DK * DV + (RULE == RC_MLSTM ? DK : 0);
+    float4* dst = reinterpret_cast<float4*>(a.chunk_state + at * per_chunk);
+#pragma unroll
+    for (int p = 0; p < PAIRS; ++p) {
+        dst[((2 * mt) * KT + p0 + p) * 32 + lane] = make_float4(acc[2 * p][0], acc[2 * p][1], acc[2 * p + 1][0], acc[2 * p + 1][1]);
+        dst[((2 * mt + 1) * KT + p0 + p) * 32 + lane] = make_float4(acc[2 * p][2], acc[2 * p][3], acc[2 * p + 1][2], acc[2 * p + 1][3]);
+    }
+    if (RULE == RC_MLSTM && threadIdx.x < DK) {             // the keys' own sum
+        const int i = threadIdx.x;
+        float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int t = 0; t < L; ++t)
+            part[t & 3] += (__bfloat162float(kw[t * RS + i]) + __bfloat162float(kw[(L + t) * RS + i])) + __bfloat162float(kw[(2 * L + t) * RS + i]);
+        a.chunk_state[at * per_chunk + (size_t)DK * DV + i] = (part[0] + part[1]) + (part[2] + part[3]);
+    }
+}
+
+// ---- (2) the walk over the chunks: a thread owns four elements of a head's state (two pairs of key channels of one value).
+template <int RULE, int DV>
+__global__ void __launch_bounds__(THREADS) chunk_walk_kernel(RcArgs a) {
+    constexpr int GROUPS = DK * DV / 4, COLS = RULE == RC_MLSTM ? DV + 1 : DV, NG = RULE == RC_MLSTM ? DK / 4 : 0;
+    constexpr size_t per_chunk = (size_t)DK * DV + (RULE == RC_MLSTM ? DK : 0);
+    constexpr int AHEAD = 16, BATCH = 128;
+    __shared__ double2 gates[RULE == RC_MLSTM ? BATCH : 1];
+    __shared__ float tops[RULE == RC_MLSTM ? BATCH + 1 : 1], by[RULE == RC_MLSTM ? BATCH : 1], of[RULE == RC_MLSTM ? BATCH : 1];
+    tw_grid_wait();
+    tw_grid_launch_dependents();
+    const int h = blockIdx.y, s = blockIdx.z;
+    const int len = a.seq_q_len[s];
+    if (len < a.min_len) return;
+    const int chunks = (len + L - 1) / L;
+    const size_t at0 = (size_t)first_chunk(a.seq_q_len, s, a.min_len) * a.H + h;
+    const int own = blockIdx.x * THREADS + threadIdx.x;
+    const bool live = own < GROUPS + NG;                    // (the others read what the last one reads and write nothing)
+    const int g = live ? own : GROUPS + NG - 1;
+    float* slot = a.state + (size_t)a.seq_slot[s] * a.state_stride + (size_t)h * ((size_t)DK * COLS + (RULE == RC_MLSTM ? 1 : 0));
+    // where the four elements lie in the slot
+    int dk, dv, step;               // elements (dk, dv), (dk + 1, dv), (dk + step, dv), (dk + step + 1, dv)
+    if (g < GROUPS) {
+        const int lane = g & 31, tile = g >> 5;
+        dv = (tile / KT) * 8 + (lane >> 2);
+        dk = (tile % KT) * 16 + 2 * (lane & 3);
+        step = 8;
+    } else {
+        dk = 4 * (g - GROUPS); dv = DV; step = 2;
+    }
+    float* e0 = slot + (size_t)dk * COLS + dv;
+    float4 S = make_float4(e0[0], e0[COLS], e0[(size_t)step * COLS], e0[(size_t)(step + 1) * COLS]);
+    float m = RULE == RC_MLSTM ? slot[(size_t)DK * COLS] : 0.f;
+    float keep_full = 0.f, keep_last = 0.f;
+    if (RULE == RC_RETENTION) {
+        auto power = [&](int n) {
+            double p = 1.0, b = a.p0[h];
+            for (; n; n >>= 1) { if (n & 1) p *= b; b *= b; }
+            return (float)p;
+        };
+        keep_full = power(L);
+        keep_last = power(len - (chunks - 1) * L);
+    }
+    float4* mine = reinterpret_cast<float4*>(a.chunk_state + at0 * per_chunk) + g;
+    const size_t stride = per_chunk / 4 * a.H;
+    for (int b0 = 0; b0 < chunks; b0 += BATCH) {
+        const int nb = min(BATCH, chunks - b0);
+        if (RULE == RC_MLSTM) {
+            // the running maxima, one after the other; then what each chunk keeps and adds, a thread per chunk
+            __syncthreads();
+            for (int c = threadIdx.x; c < nb; c += THREADS) gates[c] = a.chunk_gate[at0 + (size_t)(b0 + c) * a.H];
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (int c = 0; c < nb; ++c) {
+                    tops[c] = m;
+                    m = (float)(gates[c].x + fmax((double)m, gates[c].y));
+                }
+                tops[nb] = m;
+            }
+            __syncthreads();
+            m = tops[nb];
+            for (int c = threadIdx.x; c < nb; c += THREADS) {
+                by[c] = (float)exp(gates[c].x + (double)tops[c] - (double)tops[c + 1]);
+                of[c] = (float)exp(gates[c].x + gates[c].y - (double)tops[c + 1]);
+                if (blockIdx.x == 0) a.chunk_max[at0 + (size_t)(b0 + c) * a.H] = tops[c];
+            }
+            __syncthreads();
+        }
+        for (int c0 = 0; c0 < nb; c0 += AHEAD) {
+            float4 u[AHEAD];
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j)
+                if (c0 + j < nb) u[j] = mine[(size_t)(b0 + c0 + j) * stride];
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j) {
+                if (c0 + j < nb) {
+                    const int c = b0 + c0 + j;
+                    if (live) mine[(size_t)c * stride] = S;
+                    const float keep = RULE == RC_MLSTM ? by[c0 + j] : (c + 1 < chunks ? keep_full : keep_last);
+                    const float add = RULE == RC_MLSTM ? of[c0 + j] : 1.f;
+                    S.x = keep * S.x + add * u[j].x; S.y = keep * S.y + add * u[j].y;
+                    S.z = keep * S.z + add * u[j].z; S.w = keep * S.w + add * u[j].w;
+                }
+            }
+        }
+    }
+    if (!a.write_state || !live) return;
+    // (the running maximum behind the state, which every block of the head reads, is moved on by the next launch)
+    e0[0] = S.x; e0[COLS] = S.y; e0[(size_t)step * COLS] = S.z; e0[(size_t)(step + 1) * COLS] = S.w;
+}
+
+// ---- (3) a chunk's outputs.  The 64 x 64 products q . k are shared out over the warps (a tile of 16 rows and every other
+// tile of 16 columns at or before the diagonal), get their coefficients and lie in shared memory as three bf16 terms; then
+// a warp owns DV / 8 values for all 64 tokens, so that the state is read, and split into its terms, once.
+template <int RULE, int DV>
+__global__ void __launch_bounds__(THREADS, 2) chunk_outputs_kernel(RcArgs a) {
+    constexpr int VS = DV + 8, NTW = DV / 64, NQ = RULE == RC_RETENTION ? 3 : 1;
+    static_assert(NTW == 1 || NTW == 2, "value sizes");
+    extern __shared__ __align__(16) unsigned char rc_smem[];
+    bf16* qs = reinterpret_cast<bf16*>(rc_smem);            // [NQ][L][RS]
+    bf16* ks = qs + NQ * L * RS;                            // [NQ][L][RS]; later, in its place:
+    bf16* ms = ks;                                          // [3][L][MS] the coefficients times q . k
+    bf16* vs = ms + 3 * L * MS;                             // [L][VS]
+    __shared__ float pw[L + 1];
+    __shared__ float in[L], floor_[L], row_sum[2][L];
+    __shared__ float2 gs[L], rs[L];                         // mlstm: G_s and R_t as a float and what it leaves
+    tw_grid_wait();
+    tw_grid_launch_dependents();
+    const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
+    const int len = a.seq_q_len[s];
+    if (len < a.min_len || c * L >= len) return;
+    const int ct = min(L, len - c * L);
+    const size_t row0 = (size_t)a.seq_q_start[s] + c * L;
+    const size_t at = (size_t)(first_chunk(a.seq_q_len, s, a.min_len) + c) * a.H + h;
+    constexpr size_t per_chunk = (size_t)DK * DV + (RULE == RC_MLSTM ? DK : 0);
+    const float4* state = reinterpret_cast<const float4*>(a.chunk_state + at * per_chunk);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const bf16* qrows = a.q + row0 * a.q_stride + (size_t)h * DK;
+    const bf16* krows = a.k + row0 * a.k_stride + (size_t)h * DK;
+    Rows<DV> vrows;
+    vrows.load(a.v + row0 * a.v_stride + (size_t)h * DV, a.v_stride, ct);
+    if (RULE == RC_RETENTION && a.rot_dims > 0) {
+        stage_rotated(qs, a, qrows, a.q_stride, row0, ct, a.q_scale, nullptr);
+        stage_rotated(ks, a, krows, a.k_stride, row0, ct, a.k_scale, nullptr);
+    } else {
+        Rows<DK> qr, kr;
+        qr.load(qrows, a.q_stride, ct);
+        kr.load(krows, a.k_stride, ct);
+        if (RULE == RC_RETENTION) {
+            stage_plain(qs, qr, a.q_scale, nullptr);
+            stage_plain(ks, kr, a.k_scale, nullptr);
+        } else {
+            qr.store(qs, RS);
+            kr.store(ks, RS);
+        }
+    }
+    // (a value that is not finite must not reach the tokens before its own: they share a tile of the product with it)
+    const bool found = vrows.keep_finite();
+    // what the q and k in shared memory still lack
+    const float qk = RULE == RC_RETENTION ? 1.f : a.q_scale * a.k_scale;
+    if (warp == 0) {
+        if (RULE == RC_RETENTION) {
+            decay_powers(pw, a.p0[h]);
+            __syncwarp();
+            in[lane] = pw[lane + 1]; in[lane + 32] = pw[lane + 33];
+        } else {
+            const Gates gt = chunk_gates(a, h, row0, ct);
+            const float m = a.chunk_max[at];
+            auto put = [&](int t, double F, double G, double top) {
+                const double R = fmax((double)m, top);
+                const float gh = (float)G, rh = (float)R;
+                gs[t] = make_float2(gh, t < ct ? (float)(G - (double)gh) : 0.f);
+                rs[t] = make_float2(rh, (float)(R - (double)rh));
+                in[t] = expf((float)((double)m - R)) * a.q_scale;
+                floor_[t] = expf(-(float)(F + R));
+                if (t == ct - 1 && a.write_state && c * L + ct == len)
+                    a.state[(size_t)a.seq_slot[s] * a.state_stride + (size_t)h * ((size_t)DK * (DV + 1) + 1) + (size_t)DK * (DV + 1)] = (float)(F + R);
+            };
+            put(lane, gt.f0, gt.g0, gt.m0);
+            put(lane + 32, gt.f1, gt.g1, gt.m1);
+        }
+    }
+    const bool loud = __syncthreads_or(found);
+    // ---- q . k
+    const int half = warp >> 2, rt = half ? 3 - (warp & 3) : (warp & 3);       // (opposite orders: the schedulers get equal shares)
+    float G[2][2][4], Gl[2][2][4];                          // the tiles half, half + 2 at or before the diagonal
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            G[x][y][0] = G[x][y][1] = G[x][y][2] = G[x][y][3] = 0.f;
+            Gl[x][y][0] = Gl[x][y][1] = Gl[x][y][2] = Gl[x][y][3] = 0.f;
+        }
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        uint32_t A[NQ][4];
+#pragma unroll
+        for (int t = 0; t < NQ; ++t) ldmatrix_x4(A[t], qs + (t * L + rt * 16 + (lane & 15)) * RS + k * 16 + (lane >> 4) * 8);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int j = half + 2 * x;
+            if (j > rt) continue;
+#pragma unroll
+            for (int u = NQ - 1; u >= 0; --u) {             // term u of k with the terms of q that matter beside it
+                uint32_t B[4];
+                ldmatrix_x4(B, ks + (u * L + j * 16 + (lane & 7) + ((lane >> 4) << 3)) * RS + k * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+                for (int t = NQ - 1 - u; t >= 0; --t) {
+                    if (t + u == 0) {
+                        mma_top(G[x][0], A[t], B[0], B[1]);
+                        mma_top(G[x][1], A[t], B[2], B[3]);
+                    } else {
+                        mma_bf16(Gl[x][0], A[t], B[0], B[1]);
+                        mma_bf16(Gl[x][1], A[t], B[2], B[3]);
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();                                        // nobody reads k any more: its place is the coefficients' and the values'
+    vrows.store(vs, VS);
+    {
+        const int ta = rt * 16 + g, tb = ta + 8;
+        float sum_a = 0.f, sum_b = 0.f;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int j = half + 2 * x;
+            if (j > rt) continue;
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                const int s0 = j * 16 + y * 8 + 2 * tq;
+                float m[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = e < 2 ? ta : tb, src = s0 + (e & 1);
+                    float co = 0.f;
+                    if (src <= t) {
+                        if (RULE == RC_RETENTION) co = pw[t - src];
+                        else co = expf((gs[src].x - rs[t].x) + (gs[src].y - rs[t].y));
+                    }
+                    m[e] = src <= t ? (G[x][y][e] + Gl[x][y][e]) * (co * qk) : 0.f;
+                }
+                sum_a += m[0] + m[1]; sum_b += m[2] + m[3];
+                uint32_t hi, mid, lo;
+                split3(m[0], m[1], hi, mid, lo);
+                *reinterpret_cast<uint32_t*>(ms + ta * MS + s0) = hi;
+                *reinterpret_cast<uint32_t*>(ms + (L + ta) * MS + s0) = mid;
+                *reinterpret_cast<uint32_t*>(ms + (2 * L + ta) * MS + s0) = lo;
+                split3(m[2], m[3], hi, mid, lo);
+                *reinterpret_cast<uint32_t*>(ms + tb * MS + s0) = hi;
+                *reinterpret_cast<uint32_t*>(ms + (L + tb) * MS + s0) = mid;
+                *reinterpret_cast<uint32_t*>(ms + (2 * L + tb) * MS + s0) = lo;
+            }
+        }
+        if (RULE == RC_MLSTM) {
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                sum_a += __shfl_xor_sync(0xffffffffu, sum_a, o);
+                sum_b += __shfl_xor_sync(0xffffffffu, sum_b, o);
+            }
+            if (tq == 0) { row_sum[half][ta] = sum_a; row_sum[half][tb] = sum_b; }
+        }
+    }
+    // ---- q times the state before the chunk: this warp's values for all tokens
+    float acc[L / 16][NTW][4], low[L / 16][NTW][4];
+#pragma unroll
+    for (int r = 0; r < L / 16; ++r)
+#pragma unroll
+        for (int n = 0; n < NTW; ++n) {
+            acc[r][n][0] = acc[r][n][1] = acc[r][n][2] = acc[r][n][3] = 0.f;
+            low[r][n][0] = low[r][n][1] = low[r][n][2] = low[r][n][3] = 0.f;
+        }
+    float4 next[NTW];
+#pragma unroll
+    for (int n = 0; n < NTW; ++n) next[n] = state[((warp * NTW + n) * KT) * 32 + lane];
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        uint32_t B[NTW][3][2];
+#pragma unroll
+        for (int n = 0; n < NTW; ++n) {
+            const float4 v = next[n];
+            if (k + 1 < KT) next[n] = state[((warp * NTW + n) * KT + k + 1) * 32 + lane];
+            split3(v.x, v.y, B[n][0][0], B[n][1][0], B[n][2][0]);
+            split3(v.z, v.w, B[n][0][1], B[n][1][1], B[n][2][1]);
+        }
+#pragma unroll
+        for (int r = 0; r < L / 16; ++r) {
+#pragma unroll
+            for (int t = NQ - 1; t >= 0; --t) {
+                uint32_t A[4];
+                ldmatrix_x4(A, qs + (t * L + r * 16 + (lane & 15)) * RS + k * 16 + (lane >> 4) * 8);
+#pragma unroll
+                for (int n = 0; n < NTW; ++n)
+#pragma unroll
+                    for (int u = 2 - t; u >= 0; --u) {
+                        if (t + u == 0) mma_top(acc[r][n], A, B[n][u][0], B[n][u][1]);
+                        else mma_bf16(low[r][n], A, B[n][u][0], B[n][u][1]);
+                    }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < L / 16; ++r) {
+        const float ia = in[r * 16 + g], ib = in[r * 16 + g + 8];
+#pragma unroll
+        for (int n = 0; n < NTW; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[r][n][e] = (acc[r][n][e] + low[r][n][e]) * (e < 2 ? ia : ib);
+                low[r][n][e] = 0.f;
+            }
+    }
+    __syncthreads();                                        // the coefficients are there
+    // ---- plus the chunk's own tokens
+#pragma unroll
+    for (int j = 0; j < L / 16; ++j) {
+        uint32_t B[4];
+        const bf16* base = vs + (j * 16 + (lane & 15)) * VS + warp * NTW * 8;
+        if constexpr (NTW == 2) {
+            ldmatrix_x4_trans(B, base + (lane >> 4) * 8);
+        } else {
+            asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+                         : "=r"(B[0]), "=r"(B[1]) : "r"((uint32_t)__cvta_generic_to_shared(base)));
+        }
+#pragma unroll
+        for (int r = j; r < L / 16; ++r) {
+#pragma unroll
+            for (int t = 2; t >= 0; --t) {
+                uint32_t A[4];
+                ldmatrix_x4(A, ms + (t * L + r * 16 + (lane & 15)) * MS + j * 16 + (lane >> 4) * 8);
+                if (t == 0) {
+                    mma_top(acc[r][0], A, B[0], B[1]);
+                    if constexpr (NTW == 2) mma_top(acc[r][1], A, B[2], B[3]);
+                } else {
+                    mma_bf16(low[r][0], A, B[0], B[1]);
+                    if constexpr (NTW == 2) mma_bf16(low[r][1], A, B[2], B[3]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < L / 16; ++r)
+#pragma unroll
+        for (int n = 0; n < NTW; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[r][n][e] += low[r][n][e];
+    if (loud) {                                             // what the product left out, token by token
+        for (int src = 0; src < ct; ++src) {
+            const bf16* row = a.v + (row0 + src) * a.v_stride + (size_t)h * DV;
+#pragma unroll
+            for (int n = 0; n < NTW; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float v = __bfloat162float(row[(warp * NTW + n) * 8 + 2 * tq + e]);
+                    if (isfinite(v)) continue;
+#pragma unroll
+                    for (int r = 0; r < L / 16; ++r)
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            const int t = r * 16 + g + 8 * x;
+                            if (t >= src)
+                                acc[r][n][2 * x + e] += v * ((__bfloat162float(ms[t * MS + src]) + __bfloat162float(ms[(L + t) * MS + src]))
+                                                             + __bfloat162float(ms[(2 * L + t) * MS + src]));
+                        }
+                }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < L / 16; ++r)
+#pragma unroll
+        for (int n = 0; n < NTW; ++n) {
+            const int ta = r * 16 + g, tb = ta + 8;
+            float* dst = a.out + (row0 + ta) * ((size_t)a.H * DV) + (size_t)h * DV + (warp * NTW + n) * 8 + 2 * tq;
+            if (ta < ct) *reinterpret_cast<float2*>(dst) = make_float2(acc[r][n][0], acc[r][n][1]);
+            if (tb < ct) *reinterpret_cast<float2*>(dst + (size_t)8 * a.H * DV) = make_float2(acc[r][n][2], acc[r][n][3]);
+        }
+    if constexpr (RULE == RC_MLSTM) {
+        // the denominators: n . q of the carried and the own keys; a warp takes eight tokens, one after the other
+        const float* n_prev = a.chunk_state + at * per_chunk + (size_t)DK * DV;
+        float nv[DK / 32];
+#pragma unroll
+        for (int e = 0; e < DK / 32; ++e) nv[e] = n_prev[lane + 32 * e];
+        for (int x = 0; x < 8; ++x) {
+            const int t = warp * 8 + x;
+            float d = 0.f;
+#pragma unroll
+            for (int e = 0; e < DK / 32; ++e) d += nv[e] * __bfloat162float(qs[t * RS + lane + 32 * e]);
+            d = tw_warp_sum(d);
+            if (lane == 0 && t < ct) {
+                // (the halves' tiles: half 0 has the tiles 0 and 2, half 1 has 1 and 3; rows of the first tile have none of the latter)
+                const float own = row_sum[0][t] + (t >= 16 ? row_sum[1][t] : 0.f);
+                a.den[(row0 + t) * a.H + h] = fmaxf(fabsf(in[t] * d + own), floor_[t]) + 1e-6f;
+            }
+        }
+    }
+}
+
+template <int RULE, int DV>
+int launch_chunks(const RcArgs& a, int max_q_len, cudaStream_t stream) {
+    constexpr int NQ = RULE == RC_RETENTION ? 3 : 1, VS = DV + 8;
+    constexpr size_t smem1 = (size_t)(3 * L * RS + L * VS) * 2;
+    constexpr size_t tail = NQ * L * RS > 3 * L * MS + L * VS ? NQ * L * RS : 3 * L * MS + L * VS;
+    constexpr size_t smem3 = (size_t)(NQ * L * RS + tail) * 2;
+    static_assert(smem1 <= 220 * 1024 && smem3 <= 112 * 1024, "shared memory");
+    cudaError_t e = cudaFuncSetAttribute(chunk_sums_kernel<RULE, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    if (e != cudaSuccess) return (int)e;
+    e = cudaFuncSetAttribute(chunk_outputs_kernel<RULE, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
+    if (e != cudaSuccess) return (int)e;
+    const dim3 grid((max_q_len + L - 1) / L, a.H, a.n_seqs);
+    constexpr int walkers = DK * DV / 4 + (RULE == RC_MLSTM ? DK / 4 : 0);
+    int code = tw_launch(chunk_sums_kernel<RULE, DV>, grid, dim3(THREADS), smem1, stream, 1, a);
+    if (code) return code;
+    code = tw_launch(chunk_walk_kernel<RULE, DV>, dim3((walkers + THREADS - 1) / THREADS, a.H, a.n_seqs), dim3(THREADS), 0, stream, 1, a);
+    if (code) return code;
+    return tw_launch(chunk_outputs_kernel<RULE, DV>, grid, dim3(THREADS), smem3, stream, 1, a);
+}
+
+}  // namespace
+
+// Requests with at least `min_len` rows (the others are left to tw_linear_recurrence).  rule: 0 retention, 2 mlstm, with the
+// operands tw_linear_recurrence has.  q, k, v: bf16 rows on 16-byte boundaries; Dk as compiled, Dv 64 or 128.
+// chunk_state: fp32 [chunks * H * (Dk * Dv + Dk)], chunk_gate: 64-bit [chunks * H * 2], chunk_max: fp32 [chunks * H], where
+// chunks >= the sum of ceil(rows / 64) over those requests.
+TW_EXPORT int tw_recurrence_chunks(int rule, float* out, float* den, const void* q, int q_stride, const void* k, int k_stride, const void* v,
+                                   int v_stride, const float* pre, int pre_stride, const float* p0, const float* inv_freq, int rot_dims,
+                                   float q_scale, float k_scale, float cap, float* state, long long state_stride, const int* positions,
+                                   const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_seqs, int H, int Dk, int Dv,
+                                   int min_len, int max_q_len, int write_state, float* chunk_state, double* chunk_gate, float* chunk_max,
+                                   cudaStream_t stream) {
+    if (n_seqs <= 0 || H <= 0 || max_q_len <= 0) return 0;
+    auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    if (Dk != DK || (Dv != 64 && Dv != 128) || min_len < 1 || (q_stride & 7) || (k_stride & 7) || (v_stride & 7) || !a16(q) || !a16(k)
+        || !a16(v) || !a16(chunk_state) || !a16(chunk_gate) || (reinterpret_cast<uintptr_t>(out) & 7) || n_seqs > 65535 || H > 65535
+        || rot_dims < 0 || rot_dims > DK || (inv_freq && (rot_dims & 3)))
+        return (int)cudaErrorInvalidValue;
+    RcArgs a;
+    a.out = out; a.den = den; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v;
+    a.q_stride = q_stride; a.k_stride = k_stride; a.v_stride = v_stride; a.pre = pre; a.pre_stride = pre_stride; a.p0 = p0;
+    a.inv_freq = inv_freq; a.rot_dims = inv_freq ? rot_dims : 0; a.q_scale = q_scale; a.k_scale = k_scale; a.cap = cap;
+    a.state = state; a.state_stride = state_stride; a.positions = positions; a.seq_slot = seq_slot; a.seq_q_start = seq_q_start;
+    a.seq_q_len = seq_q_len; a.n_seqs = n_seqs; a.H = H; a.min_len = min_len; a.write_state = write_state;
+    a.chunk_state = chunk_state; a.chunk_gate = (double2*)chunk_gate; a.chunk_max = chunk_max;
+    if (rule == 0)
+        return Dv == 128 ? launch_chunks<RC_RETENTION, 128>(a, max_q_len, stream) : launch_chunks<RC_RETENTION, 64>(a, max_q_len, stream);
+    if (rule == 2) {
+        if (!pre || !den) return (int)cudaErrorInvalidValue;
+        return Dv == 128 ? launch_chunks<RC_MLSTM, 128>(a, max_q_len, stream) : launch_chunks<RC_MLSTM, 64>(a, max_q_len, stream);
+    }
+    return (int)cudaErrorInvalidValue;
+}

@@ -99,9 +99,25 @@ class MatrixStateMixer(Mixer):
         n, ws = ctx.n_tokens, ctx.workspace
         raw = ws.get("recurrence.raw", (n, self.v_size), torch.float32)
         den = ws.get("recurrence.den", (n, self.n_heads), torch.float32) if self.rule == ops.RECURRENCE_MLSTM else None
-        ops.linear_recurrence(self.rule, raw, den, q, k, v, cache.state, ctx.positions, ctx.seq_slot, ctx.seq_q_start,
-                              ctx.seq_q_len, ctx.n_seqs, self.n_heads, self.key_dim, self.value_dim, write_state,
-                              max_q_len=ctx.max_q_len, **rule_args)
+        common = (cache.state, ctx.positions, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.n_seqs, self.n_heads, self.key_dim,
+                  self.value_dim)
+        below, longest = 0, ctx.max_q_len
+        if ops.recurrence_chunks_supported(self.rule, q.dtype, self.key_dim, self.value_dim, rule_args.get("rot_dims", 0)):
+            # long portions in chunks, the others token by token.  The chunks' scratch is asked for in captured steps too, so
+            # that the workspace has its final size after the largest one
+            least = ops.RECURRENCE_CHUNK_MIN_TOKENS
+            chunks = ops.recurrence_chunk_count(n, ctx.n_seqs)
+            if chunks > 0:
+                scratch = (ws.get("recurrence.chunk_state", (chunks, self.n_heads * self.key_dim * (self.value_dim + 1)), torch.float32),
+                           ws.get("recurrence.chunk_gate", (chunks, self.n_heads, 2), torch.float64),
+                           ws.get("recurrence.chunk_max", (chunks, self.n_heads), torch.float32))
+            longest_known = 0 if ctx.fixed_shape else max(ctx.host_q_len, default=0)     # (a captured step knows no row counts)
+            if longest_known >= least:
+                ops.recurrence_chunks(self.rule, raw, den, q, k, v, *common, longest_known, *scratch, write_state, **rule_args)
+                below = least
+                longest = max((m for m in ctx.host_q_len if m < least), default=0)
+        if longest > 0:
+            ops.linear_recurrence(self.rule, raw, den, q, k, v, *common, write_state, max_q_len=longest, below=below, **rule_args)
         return raw, den
 
     def _finish(self, ctx: StepContext, raw, den, weight, gate):
