@@ -3,13 +3,13 @@
 //
 // A block serves one (request, key/value head, slice of the request's keys) for requests that bring ONE
 // token; the up to 8 query heads of the group are the columns of one MMA tile, so keys and values are read
-// once for the whole group.  One warp is the producer: for every tile of 64 keys it issues one
-// cp.async.bulk.tensor.2d per cache page and 64 columns of d (no multicast) into a ring of stages in shared
+// once for the whole group.  Two warps are producers, one for keys and one for values: for every tile of 64 keys it issues
+// one cp.async.bulk.tensor.3d per cache page (no multicast) into a ring of stages in shared
 // memory, in the 128-byte swizzle, and never touches the data.  Four consumer warps each own 16 keys of a
 // tile: S^T = K Q^T and O^T += V^T P^T on mma.sync with fragments read by ldmatrix (conflict-free under the
 // swizzle), online softmax in fp32.  How many bytes a block keeps in flight is the depth of the ring (up to
-// 200 KB per SM), not a matter of registers, and the producer starts before the kernel ahead of this one has
-// finished wherever the cache it reads was written by earlier steps.  When its last copy has landed the
+// 200 KB per SM), not a matter of registers, and the producers start before the kernel ahead of this one has
+// finished wherever the cache it reads was written by earlier steps.  When the last copy has landed one
 // producer asks for weights of a later kernel to be brought into L2 (`fq.next_weights`) and leaves; the merges
 // below are the consumer warps' alone.
 //
@@ -27,7 +27,7 @@
 // Reference: flow_engine/model.py:193-200 and flow_engine/kernels/paged_decode.py:13-43.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets TW_ERR_WAIT in the status word, every role
-// stops, the producer waits (bounded) for its copies in flight, and the block writes zeros and returns.
+// stops, the producers wait (bounded) for their copies in flight, and the block writes zeros and returns.
 #include "tcgen05.cuh"
 #include "attention_common.cuh"
 #include <cooperative_groups.h>
@@ -49,7 +49,7 @@ using tc5::mbar_expect_tx;
 using tc5::mbar_fence_init;
 using tc5::mbar_init;
 using tc5::mbar_wait;
-using tc5::tma_load_2d;
+using tc5::tma_load_3d;
 using tw_attn::FusedQkv;
 using tw_attn::ldmatrix_x4;
 using tw_attn::ldmatrix_x4_trans;
@@ -68,7 +68,8 @@ constexpr int VB = DV / 64;                        // 64-column blocks of a row 
 constexpr int TILE = 64;                           // keys per stage
 constexpr int CWARPS = 4;                          // consumer warps: warp w owns keys 16 w .. 16 w + 15 of a tile
 constexpr int CTHREADS = CWARPS * 32;
-constexpr int THREADS = CTHREADS + 32;             // plus the producer warp
+constexpr int PWARPS = 2;                          // producer warps: one for the keys, one for the values
+constexpr int THREADS = CTHREADS + PWARPS * 32;
 constexpr int HEADS = 8;                           // query heads per block (columns of the MMA)
 constexpr int BLKB = TILE * 128;                   // bytes of a [64 keys][64 values of d] swizzled block
 constexpr int STAGE_BYTES = (KB + VB) * BLKB;      // K, then V
@@ -103,9 +104,12 @@ constexpr float NEG_INF = -INFINITY;
 constexpr int MERGE_BYTES = CWARPS * HEADS * (DV + 2) * 4;
 constexpr int MIN_STAGES = (MERGE_BYTES + STAGE_BYTES - 1) / STAGE_BYTES < 2 ? 2 : (MERGE_BYTES + STAGE_BYTES - 1) / STAGE_BYTES;
 
-// byte offset of (key row, 16-byte chunk of d) inside a K or V tile of a stage
-__device__ __forceinline__ int tile_offset(int row, int chunk) {
-    return (chunk >> 3) * BLKB + row * 128 + (((chunk & 7) ^ (row & 7)) << 4);
+// A K or V tile of a stage is what one copy per cache page leaves: pages (of 1 << shift keys, at most 64) one behind the other,
+// a page as blocks of 64 columns of d.  Byte offset of (key row, 16-byte chunk of d) in it, NB the blocks of a row:
+template <int NB>
+__device__ __forceinline__ int tile_offset(int row, int chunk, int shift) {
+    const int line = ((((row >> shift) * NB + (chunk >> 3)) << shift) | (row & ((1 << shift) - 1)));      // of 128 bytes
+    return line * 128 + (((chunk & 7) ^ (line & 7)) << 4);
 }
 
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CTHREADS) : "memory"); }
@@ -162,7 +166,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
     const int first_blk = k_begin / page_size;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < nstages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], CWARPS); }
+        for (int i = 0; i < nstages; ++i) { mbar_init(&full[i], PWARPS); mbar_init(&empty[i], CWARPS); }
         s_aborted = 0;
         mbar_fence_init();
     }
@@ -181,18 +185,25 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     float m0 = NEG_INF, m1 = NEG_INF, l0 = 0.f, l1 = 0.f;           // heads 2c and 2c + 1 of the tile
     const int g = lane >> 2, c = lane & 3;
 
-    if (warp == CWARPS) {
-        // ---- producer.  Where this kernel itself writes the step's new key and value, everything else in the
-        // cache is from earlier steps and may be fetched at once; otherwise the kernel before this one (or
-        // one before that) wrote the newest position, and the copies wait for it.
+    const int box_rows = min(page_size, TILE);
+    const int shift = 31 - __clz(box_rows);                          // (a power of two: pages are fractions or multiples of 64 keys)
+    if (warp >= CWARPS) {
+        // ---- producers: one warp copies keys, one values, a page per lane and copy.  (A warp issues the copies of its lanes one
+        // after the other, some 54 cycles each.  With one warp for both and a copy per page and 64 columns of d a tile of
+        // four pages took a block 1.13 us, however deep its ring and however idle the GPU; now 0.65 us, the consumers' share.
+        // 64 requests of 300 to 8,000 keys, 4 key/value heads: 143 us, now 101; 40 requests of 4,096: 80 us, now 55.)
+        // Where this kernel itself writes the step's new key and value, everything else in the cache is from earlier
+        // steps and may be fetched at once; otherwise the kernel before this one (or one before that) wrote the newest
+        // position, and the copies wait for it.
+        const bool values = warp > CWARPS;
         if (!(FUSED && fq.k_cache)) tw_grid_wait();
         TW_TTRACE(9);
-        const int box_rows = min(page_size, TILE);
-        const int boxes = TILE / box_rows;
-        int issued = 0;
+        const CUtensorMap* map = values ? &map_v : &map_k;
+        const int boxes = TILE / box_rows, box_bytes = (values ? VB : KB) * box_rows * 128;
+        unsigned char* place = ring + (values ? KB * BLKB : 0) + lane * box_bytes;
+        int issued = 0, st = 0;
+        uint32_t parity = 0;
         for (int i = 0; i < ntiles; ++i) {
-            const int st = i % nstages;
-            const uint32_t parity = (i / nstages) & 1;
             int row_coord = -1;
             if (lane < boxes) {
                 const int key0 = k_begin + i * TILE + lane * box_rows;
@@ -204,7 +215,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                     else row_coord = (page * Hkv + kvh) * page_size + (key0 - blk * page_size);
                 }
             }
-            const uint32_t bytes = (uint32_t)__popc(__ballot_sync(0xffffffffu, row_coord >= 0)) * ((KB + VB) * box_rows * 128);
+            const uint32_t bytes = (uint32_t)__popc(__ballot_sync(0xffffffffu, row_coord >= 0)) * box_bytes;
             int ok = 1;
             if (lane == 0) {
                 ok = (!*aborted && mbar_wait(&empty[st], parity ^ 1, status)) ? 1 : 0;
@@ -212,24 +223,19 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             }
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) break;
-            if (row_coord >= 0) {
-                unsigned char* dst = ring + st * STAGE_BYTES + lane * box_rows * 128;
-#pragma unroll
-                for (int kb = 0; kb < KB; ++kb) tma_load_2d(dst + kb * BLKB, &map_k, &full[st], kb * 64, row_coord);
-#pragma unroll
-                for (int vb = 0; vb < VB; ++vb) tma_load_2d(dst + (KB + vb) * BLKB, &map_v, &full[st], vb * 64, row_coord);
-            }
+            if (row_coord >= 0) tma_load_3d(place + st * STAGE_BYTES, map, &full[st], 0, row_coord, 0);
             issued = i + 1;
+            if (++st == nstages) { st = 0; parity ^= 1; }
         }
         TW_TTRACE(10);
-        // The producer takes no part in the merges.  It arrives at the cluster's one barrier now (it has nothing to
-        // publish) and leaves when its own work is done; the barrier counts the threads that have not exited.
+        // The producers take no part in the merges.  They arrive at the cluster's one barrier now (they have nothing to
+        // publish) and leave when their own work is done; the barrier counts the threads that have not exited.
         if (CLUSTER && nsplit > 1) cg::this_cluster().barrier_arrive();
         if (lane == 0) {
             if (*aborted) {
                 // wait (bounded) for the copies already in flight, so that none lands after the block has gone
                 for (int i = max(0, issued - nstages); i < issued; ++i) mbar_wait(&full[i % nstages], (i / nstages) & 1, status);
-            } else if (FUSED && fq.next_weights) {
+            } else if (FUSED && fq.next_weights && !values) {
                 // The last keys and values are on their way.  Once they are in, the memory system has little to do
                 // while the slices merge: it may fetch weights of the kernels that follow.  Asked for from here,
                 // not by a consumer: the requests take a thread one or two microseconds to issue.
@@ -321,10 +327,19 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             qb[ks][0] = *reinterpret_cast<const uint32_t*>(s_q + g * D + 16 * ks + 2 * c);
             qb[ks][1] = *reinterpret_cast<const uint32_t*>(s_q + g * D + 16 * ks + 2 * c + 8);
         }
+        // where this lane's rows of the fragments lie in a tile: keys krow, values vrow (read transposed)
+        const int krow = warp * 16 + (lane & 15);
+        const int mj = lane >> 3, vrow = warp * 16 + (mj >> 1) * 8 + (lane & 7);
+        int k_at[KSTEPS], v_at[MT_O];
+#pragma unroll
+        for (int ks = 0; ks < KSTEPS; ++ks) k_at[ks] = tile_offset<KB>(krow, 2 * ks + (lane >> 4), shift);
+#pragma unroll
+        for (int mt = 0; mt < MT_O; ++mt) v_at[mt] = tile_offset<VB>(vrow, 2 * mt + (mj & 1), shift);
         bool ok = true;
+        int st = 0;
+        uint32_t parity = 0;
         for (int i = 0; i < ntiles && ok; ++i) {
-            const int st = i % nstages;
-            ok = !*aborted && mbar_wait(&full[st], (i / nstages) & 1, status);
+            ok = !*aborted && mbar_wait(&full[st], parity, status);
             if (!ok) { *aborted = 1; break; }
             if (warp == 0 && i == 0) TW_TTRACE(3);
             const int key0 = k_begin + i * TILE + warp * 16;
@@ -337,7 +352,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                     for (int idx = lane; idx < 16 * (DV / 8); idx += 32) {
                         const int r = idx / (DV / 8), ch = idx - r * (DV / 8);
                         if (key0 + r < first_key || key0 + r >= k_end)
-                            *reinterpret_cast<uint4*>(vs_ + tile_offset(warp * 16 + r, ch)) = make_uint4(0u, 0u, 0u, 0u);
+                            *reinterpret_cast<uint4*>(vs_ + tile_offset<VB>(warp * 16 + r, ch, shift)) = make_uint4(0u, 0u, 0u, 0u);
                     }
                     tc5::fence_proxy_async();      // these stores stay ahead of the copy that fills the stage next
                 }
@@ -347,22 +362,27 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                         const int r = warp * 16 + (pos - key0);
                         for (int idx = lane; idx < 2 * (D / 8); idx += 32) {
                             const int which = idx / (D / 8), ch = idx - which * (D / 8);
-                            *reinterpret_cast<uint4*>((which ? vs_ : ks_) + tile_offset(r, ch)) =
+                            *reinterpret_cast<uint4*>((which ? vs_ : ks_) + tile_offset<KB>(r, ch, shift)) =
                                 *reinterpret_cast<const uint4*>(s_fresh + which * D + ch * 8);
                         }
                         tc5::fence_proxy_async();
                     }
                 }
                 __syncwarp();
-                // S^T = K Q^T: rows = keys g, g + 8; columns = heads 2c, 2c + 1
-                float sacc[4] = {0.f, 0.f, 0.f, 0.f};
-                const int krow = warp * 16 + (lane & 15);
+                // S^T = K Q^T: rows = keys g, g + 8; columns = heads 2c, 2c + 1.  Four sums over the steps ks mod 4, so that
+                // the chain of dependent products is a quarter as long
+                float sp[4][4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) { sp[x][0] = sp[x][1] = sp[x][2] = sp[x][3] = 0.f; }
 #pragma unroll
                 for (int ks = 0; ks < KSTEPS; ++ks) {
                     uint32_t a[4];
-                    ldmatrix_x4(a, ks_ + tile_offset(krow, 2 * ks + (lane >> 4)));
-                    mma_bf16_regs(sacc, a[0], a[1], a[2], a[3], qb[ks][0], qb[ks][1]);
+                    ldmatrix_x4(a, ks_ + k_at[ks]);
+                    mma_bf16_regs(sp[ks & 3], a[0], a[1], a[2], a[3], qb[ks][0], qb[ks][1]);
                 }
+                float sacc[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) sacc[x] = (sp[0][x] + sp[1][x]) + (sp[2][x] + sp[3][x]);
                 const bool oka = key0 + g >= first_key && key0 + g < k_end;
                 const bool okb = key0 + g + 8 >= first_key && key0 + g + 8 < k_end;
                 sacc[0] = oka ? sacc[0] * scale_log2e : NEG_INF;
@@ -395,17 +415,16 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                     }
                 }
                 // O^T += V^T P^T: V read transposed, 8 keys x 8 values of d per matrix
-                const int j = lane >> 3, r = lane & 7;
-                const int vrow = warp * 16 + (j >> 1) * 8 + r;
 #pragma unroll
                 for (int mt = 0; mt < MT_O; ++mt) {
                     uint32_t a[4];
-                    ldmatrix_x4_trans(a, vs_ + tile_offset(vrow, 2 * mt + (j & 1)));
+                    ldmatrix_x4_trans(a, vs_ + v_at[mt]);
                     mma_bf16_regs(oacc[mt], a[0], a[1], a[2], a[3], pb0, pb1);
                 }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[st]);
+            if (++st == nstages) { st = 0; parity ^= 1; }
         }
         if (warp == 0) TW_TTRACE(4);
         // sums over the keys of the other threads with the same heads
@@ -418,7 +437,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
     // ---- merge the warps (the ring is free: every copy that was issued has been waited for).  The warps exchange
     // their maxima, each scales its sums to the block's maximum in registers, and the four are added in warp order.
-    // Only the consumer warps are here: the producer has left (see above), so every barrier below is theirs.
+    // Only the consumer warps are here: the producers have left or are leaving (see above), so every barrier below is theirs.
     consumer_sync();
     const bool failed = *aborted != 0;
     float* mo = reinterpret_cast<float*>(ring);                  // [warps][heads][DV]
@@ -519,11 +538,11 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             for (int i = 0; i < nsplit; ++i) {
                 const float2 ml = s_recv_ml[i][row];
                 const float f = (ml.x == NEG_INF || M == NEG_INF) ? 0.f : exp2f(ml.x - M);
-                L += ml.y * f;
-                o += mine[(i * own4 + jj) * 4] * f;
+                L = __fadd_rn(L, __fmul_rn(ml.y, f));      // (rounded as the merge through scratch memory rounds it)
+                o = fmaf(mine[(i * own4 + jj) * 4], f, o);
             }
-            out[(size_t)n * out_stride + (size_t)(kvh * G + h0 + row) * DV + d] =
-                __float2bfloat16_rn(L > 0.f ? o / L * tw_attn::head_gate(gate, n, Hq, kvh * G + h0 + row) : 0.f);
+            const float inv = L > 0.f ? tw_attn::head_gate(gate, n, Hq, kvh * G + h0 + row) / L : 0.f;
+            out[(size_t)n * out_stride + (size_t)(kvh * G + h0 + row) * DV + d] = __float2bfloat16_rn(o * inv);
         }
         if (warp == 0) TW_TTRACE(7);
         return;
@@ -703,8 +722,8 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
     if (rows >= (1ll << 31)) return (int)cudaErrorInvalidValue;
     const int box_rows = page_size < TILE ? page_size : TILE;
     CUtensorMap mk, mv;
-    if (int e = tc5::get_map(k_cache, rows, D, box_rows, &mk)) return e;
-    if (int e = tc5::get_map(v_cache, rows, DV, box_rows, &mv)) return e;
+    if (int e = tc5::get_map_rows(k_cache, rows, D, box_rows, &mk)) return e;
+    if (int e = tc5::get_map_rows(v_cache, rows, DV, box_rows, &mv)) return e;
     float* partial_o = scratch;
     float* partial_ml = scratch ? scratch + (size_t)n_seqs * Hq * nsplit * DV : nullptr;
     FusedQkv fq = {};
