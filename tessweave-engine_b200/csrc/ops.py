@@ -1659,6 +1659,9 @@ RECURRENCE_CHUNK = 64                   # tokens of a chunk (csrc/recurrence_chu
 # Where a portion goes through the chunks' three launches.  14 heads of 128 x 128, mLSTM / retention: 26 / 33 us for up to 256
 # tokens (one wave of blocks), token by token 30 / 28 us for 96, 38 / 37 for 128, 71 for 256 (6 heads of 64: 18 and 36 for 128).
 RECURRENCE_CHUNK_MIN_TOKENS = 128
+# Beside such a portion, how many rows a request needs to go with it (a chunk more hardly counts; token by token it would be a
+# launch of its own, 0.25 us a token: the delta rule over portions of 777, 1,024 and 201, 195 + 67 us with the last by tokens).
+RECURRENCE_CHUNK_MIN_ROWS = 32
 
 
 def recurrence_chunks_supported(mode: int, dtype: torch.dtype, key_dim: int, value_dim: int, rot_dims: int = 0) -> bool:
@@ -1668,8 +1671,8 @@ def recurrence_chunks_supported(mode: int, dtype: torch.dtype, key_dim: int, val
 
 
 def recurrence_chunk_count(rows: int, n_seqs: int) -> int:
-    """The most chunks that portions of at least ``RECURRENCE_CHUNK_MIN_TOKENS`` rows, ``rows`` in all, are cut into."""
-    return rows // RECURRENCE_CHUNK + min(n_seqs, rows // RECURRENCE_CHUNK_MIN_TOKENS)
+    """The most chunks that portions of at least ``RECURRENCE_CHUNK_MIN_ROWS`` rows, ``rows`` in all, are cut into."""
+    return rows // RECURRENCE_CHUNK + min(n_seqs, rows // RECURRENCE_CHUNK_MIN_ROWS)
 
 
 def recurrence_chunks(mode: int, out: torch.Tensor, den: torch.Tensor | None, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
@@ -1678,7 +1681,7 @@ def recurrence_chunks(mode: int, out: torch.Tensor, den: torch.Tensor | None, q:
                       chunk_state: torch.Tensor, chunk_gate: torch.Tensor, chunk_max: torch.Tensor, write_state: bool = True,
                       pre: torch.Tensor | None = None, p0: torch.Tensor | None = None, inv_freq: torch.Tensor | None = None,
                       rot_dims: int = 0, q_scale: float = 1.0, k_scale: float = 1.0, cap: float = 1.0) -> None:
-    """``linear_recurrence`` of the requests that bring ``RECURRENCE_CHUNK_MIN_TOKENS`` rows or more, in chunks on the tensor
+    """``linear_recurrence`` of the requests that bring ``RECURRENCE_CHUNK_MIN_ROWS`` rows or more, in chunks on the tensor
     cores (csrc/recurrence_chunks.cu): same operands and state, bfloat16 q, k, v.  The other requests are left alone.
     ``chunk_state`` fp32 [chunks, heads * (key_dim * value_dim + key_dim)], ``chunk_gate`` fp64 [chunks, heads, 2] and
     ``chunk_max`` fp32 [chunks, heads] are scratch for ``recurrence_chunk_count`` chunks."""
@@ -1700,9 +1703,52 @@ def recurrence_chunks(mode: int, out: torch.Tensor, den: torch.Tensor | None, q:
         _ptr(pre), c_int(0 if pre is None else pre.stride(0)), _ptr(p0), _ptr(inv_freq), c_int(rot_dims), c_float(q_scale),
         c_float(k_scale), c_float(cap), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(positions), _ptr(seq_slot),
         _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(key_dim), c_int(value_dim),
-        c_int(RECURRENCE_CHUNK_MIN_TOKENS), c_int(max_q_len), c_int(1 if write_state else 0), _ptr(chunk_state), _ptr(chunk_gate),
+        c_int(RECURRENCE_CHUNK_MIN_ROWS), c_int(max_q_len), c_int(1 if write_state else 0), _ptr(chunk_state), _ptr(chunk_gate),
         _ptr(chunk_max), _stream())
     _check(code, "recurrence_chunks")
+
+
+# The delta rule's three launches take 45 us for 128 tokens, 51 for 256 (14 heads of 128 x 128); token by token 36 and 67.
+DELTA_CHUNK_MIN_TOKENS = 256
+
+
+def delta_chunks_supported(q: torch.Tensor, k: torch.Tensor, key_dim: int, value_dim: int, channel_decay: bool) -> bool:
+    """Whether csrc/delta_chunks.cu can take the long portions of a step: one decay per head, fp32 rows on 16-byte boundaries."""
+    return (not channel_decay and key_dim in (64, 128) and value_dim in (64, 128)
+            and all(t.dtype == torch.float32 and t.stride(1) == 1 and t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (q, k)))
+
+
+def delta_chunk_floats(heads: int, qk_group: int, key_dim: int, value_dim: int) -> int:
+    """Floats of scratch memory a chunk of the delta rule takes (csrc/delta_chunks.cu: tw_delta_chunks)."""
+    terms = 3 * RECURRENCE_CHUNK * key_dim // 2
+    return heads * (key_dim * value_dim + RECURRENCE_CHUNK * (value_dim + 2) + terms) + heads // qk_group * terms
+
+
+def delta_chunks(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, seq_slot: torch.Tensor,
+                 seq_q_start: torch.Tensor, seq_q_len: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int,
+                 max_q_len: int, scratch: torch.Tensor, write_state: bool, pre: torch.Tensor, p0: torch.Tensor, p1: torch.Tensor,
+                 write_pre: torch.Tensor, qk_group: int = 1, q_scale: float = 1.0, k_scale: float = 1.0) -> None:
+    """``linear_recurrence`` with the delta rule (a decay per head) of the requests that bring ``RECURRENCE_CHUNK_MIN_ROWS``
+    rows or more, in chunks (csrc/delta_chunks.cu): same operands and state.  The other requests are left alone.  ``scratch``:
+    ``delta_chunk_floats`` fp32 numbers for each of ``recurrence_chunk_count`` chunks."""
+    _cuda(out, q, k, v, state, seq_slot, seq_q_start, seq_q_len, pre, p0, p1, write_pre, scratch)
+    _need(delta_chunks_supported(q, k, key_dim, value_dim, False), "recurrence: the delta rule's chunk kernels do not take these sizes or rows")
+    _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == heads * value_dim, "recurrence: out must be fp32 [rows, H * Dv]")
+    _need(v.dtype == torch.float32 and v.stride(1) == 1 and qk_group >= 1 and heads % qk_group == 0, "recurrence: the delta rule takes fp32 rows")
+    _need(state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1, "recurrence: state must be fp32 [slots, numel]")
+    _need(all(t.dtype == torch.float32 and t.stride(1) == 1 and t.shape[1] >= heads for t in (pre, write_pre))
+          and all(t.dtype == torch.float32 and t.numel() == heads and t.is_contiguous() for t in (p0, p1)),
+          "recurrence: the delta rule needs a projected decay with its rate and bias, and a write strength, per head")
+    chunks = recurrence_chunk_count(out.shape[0], n_seqs)
+    _need(scratch.dtype == torch.float32 and scratch.data_ptr() % 16 == 0
+          and scratch.numel() >= chunks * delta_chunk_floats(heads, qk_group, key_dim, value_dim), "recurrence: the chunks' scratch is too small")
+    code = _fn("delta_chunks", "tw_delta_chunks", {"TW_DK": key_dim})(
+        _ptr(out), _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), _ptr(v), c_int(v.stride(0)), _ptr(pre), c_int(pre.stride(0)),
+        _ptr(write_pre), c_int(write_pre.stride(0)), _ptr(p0), _ptr(p1), c_float(q_scale), c_float(k_scale), _ptr(state),
+        ctypes.c_longlong(state.stride(0)), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(key_dim),
+        c_int(value_dim), c_int(qk_group), c_int(RECURRENCE_CHUNK_MIN_ROWS), c_int(max_q_len), c_int(1 if write_state else 0),
+        _ptr(scratch), c_int(chunks), _stream())
+    _check(code, "delta_chunks")
 
 
 STATE_SPACE_CHUNK_STATES = (16, 32, 64, 128, 256)

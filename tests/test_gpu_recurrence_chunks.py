@@ -5,7 +5,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-LENS = [193, 1, 128, 256, 127, 191]             # below 128 rows a request is left to the token kernel
+LENS = [193, 1, 32, 256, 31, 127]               # below 32 rows a request is left to the token kernel
 SLOTS = [3, 0, 6, 1, 5, 2]
 
 
@@ -19,6 +19,11 @@ def operands(rule, heads, dk, dv, rot, lens, seed=0, decay=None):
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")          # noqa: E731
     o["positions"] = i32([h + t for m, h in zip(lens, held) for t in range(m)])
     o["start"], o["len"], o["slot"] = i32([sum(lens[:i]) for i in range(len(lens))]), i32(lens), i32(SLOTS[:len(lens)])
+    if rule == "delta":                         # prepared rows: fp32, q and k of unit length, two value heads to a q/k head
+        unit = lambda m: torch.nn.functional.normalize(torch.randn(n, m, dk, generator=g), dim=-1).view(n, -1)       # noqa: E731
+        half = heads // 2
+        rows = torch.cat((unit(half) * dk ** -0.5, unit(half), torch.randn(n, heads * dv, generator=g)), 1).cuda()
+        o["q"], o["k"], o["v"] = rows[:, :half * dk], rows[:, half * dk:heads * dk], rows[:, heads * dk:]
     cols = dv + (1 if rule == "mlstm" else 0)
     state = torch.randn(7, heads * (dk * cols + (1 if rule == "mlstm" else 0)) + 5, generator=g)
     if rule == "mlstm":
@@ -27,6 +32,11 @@ def operands(rule, heads, dk, dv, rot, lens, seed=0, decay=None):
         pre = torch.randn(n, 2 * heads, generator=g) * torch.linspace(1, 12, heads).repeat(2)
         o["args"] = {"pre": pre.cuda(), "p0": torch.cat([torch.zeros(heads), torch.full((heads,), 2.0)]).cuda(), "q_scale": dk ** -0.5,
                      "cap": 15.0}
+    elif rule == "delta":
+        # decays from none worth mentioning to memories that are gone within a token, write strengths on both sides of a half
+        pre = torch.randn(n, 2 * heads, generator=g) * torch.linspace(1, 6, heads).repeat(2)
+        o["args"] = {"pre": pre[:, heads:].contiguous().cuda(), "write_pre": pre.cuda(), "p0": torch.linspace(-5, 1, heads).cuda(),
+                     "p1": torch.randn(heads, generator=g).cuda(), "qk_group": 2}
     else:
         decay = decay if decay is not None else [1.0 - 2.0 ** -(h + 1) for h in range(heads)]
         o["args"] = {"p0": torch.tensor(decay, dtype=torch.float32).cuda(), "k_scale": dk ** -0.5}
@@ -38,9 +48,21 @@ def operands(rule, heads, dk, dv, rot, lens, seed=0, decay=None):
 
 def token_by_token(rule, o, heads, dk, dv, rot, a, m, slot):
     """(outputs, denominators, state) of rows a .. a + m - 1 in 64 bits."""
-    q, k, v = (o[x][a:a + m].double().cpu().view(m, heads, -1) for x in "qkv")
+    q, k = (o[x][a:a + m].double().cpu().view(m, -1, dk) for x in "qk")
+    v = o["v"][a:a + m].double().cpu().view(m, heads, dv)
     st = o["state"][slot, :-5].double().cpu().view(heads, -1)
     out, den = torch.zeros(m, heads, dv, dtype=torch.float64), torch.zeros(m, heads, dtype=torch.float64)
+    if rule == "delta":
+        S, A = st.view(heads, dk, dv).clone(), {x: t.double().cpu() for x, t in o["args"].items() if x != "qk_group"}
+        q, k = q.repeat_interleave(2, 1), k.repeat_interleave(2, 1)
+        keep = torch.exp(-torch.exp(A["p0"]) * torch.nn.functional.softplus(A["pre"][a:a + m, :heads] + A["p1"], threshold=700.0))
+        beta = torch.sigmoid(A["write_pre"][a:a + m, :heads])
+        for t in range(m):
+            S = keep[t][:, None, None] * S
+            u = beta[t][:, None] * (v[t] - torch.einsum("hij,hi->hj", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None]
+            out[t] = torch.einsum("hij,hi->hj", S, q[t])
+        return out, den, S.reshape(-1)
     if rule == "retention":
         S = st.view(heads, dk, dv).clone()
         if rot:
@@ -73,13 +95,17 @@ def token_by_token(rule, o, heads, dk, dv, rot, a, m, slot):
 
 def run(rule, o, heads, dk, dv, chunks, write=True, lens=LENS):
     from tessweave_engine_b200.csrc import ops
-    mode = ops.RECURRENCE_MLSTM if rule == "mlstm" else ops.RECURRENCE_RETENTION
+    mode = {"mlstm": ops.RECURRENCE_MLSTM, "retention": ops.RECURRENCE_RETENTION, "delta": ops.RECURRENCE_DELTA}[rule]
     n = o["q"].shape[0]
     out, den = torch.full((n, heads * dv), -7.0, device="cuda"), torch.full((n, heads), -7.0, device="cuda")
     state = o["state"].clone()
     common = (out, den if rule == "mlstm" else None, o["q"], o["k"], o["v"], state, o["positions"], o["slot"], o["start"], o["len"], len(lens),
               heads, dk, dv)
-    if chunks:
+    if chunks and rule == "delta":
+        count = ops.recurrence_chunk_count(n, len(lens)) * ops.delta_chunk_floats(heads, 2, dk, dv)
+        ops.delta_chunks(out, o["q"], o["k"], o["v"], state, *common[7:], max(lens), torch.full((count,), float("nan"), device="cuda"), write,
+                         **o["args"])
+    elif chunks:
         count = ops.recurrence_chunk_count(n, len(lens))
         nan = lambda k, dt=torch.float32: torch.full((k,), float("nan"), device="cuda", dtype=dt)         # noqa: E731
         ops.recurrence_chunks(mode, *common, max(lens), nan(count * heads * dk * (dv + 1)), nan(count * heads * 2, torch.float64),
@@ -95,7 +121,9 @@ def distance(got, want):
 
 @pytest.mark.parametrize("rule,heads,dk,dv,rot", [("mlstm", 3, 128, 128, 0), ("mlstm", 2, 64, 128, 0), ("mlstm", 5, 64, 64, 0),
                                                   ("mlstm", 2, 32, 64, 0), ("retention", 3, 128, 128, 128), ("retention", 2, 64, 64, 0),
-                                                  ("retention", 4, 128, 64, 64), ("retention", 2, 32, 128, 32)])
+                                                  ("retention", 4, 128, 64, 64), ("retention", 2, 32, 128, 32),
+                                                  ("delta", 4, 128, 128, 0), ("delta", 6, 64, 64, 0), ("delta", 2, 64, 128, 0),
+                                                  ("delta", 2, 128, 64, 0)])
 def test_chunks_against_tokens(rule, heads, dk, dv, rot):
     """The chunks' error against 64 bits is that of the token kernel or below it.  A quarter more is allowed for chance, and the
     least that 32 bits leave: 1e-7 in sums; with mLSTM's gates, numbers of up to 15 evaluated in 32 bits (an error of up to
@@ -106,7 +134,7 @@ def test_chunks_against_tokens(rule, heads, dk, dv, rot):
     got, token = run(rule, o, heads, dk, dv, True), run(rule, o, heads, dk, dv, False)
     a = 0
     for m, slot in zip(LENS, SLOTS):
-        if m < 128:
+        if m < 32:
             assert torch.all(got[0][a:a + m] == -7.0) and torch.equal(got[2][slot], o["state"][slot].cpu())
         else:
             want = token_by_token(rule, o, heads, dk, dv, rot, a, m, slot)
@@ -143,14 +171,15 @@ def test_decays_at_the_edges(decay):
             assert distance(got[2][slot, :-5].double().view(2, -1)[h], want[2].view(2, -1)[h]) < 5e-7
 
 
-@pytest.mark.parametrize("rule", ["mlstm", "retention"])
+@pytest.mark.parametrize("rule", ["mlstm", "retention", "delta"])
 def test_a_token_does_not_reach_those_before_it(rule):
     """A value that is infinite or not a number spoils its own token's column and later ones, nothing earlier."""
-    o = operands(rule, 2, 64, 64, 0, LENS)
-    clean = run(rule, o, 2, 64, 64, True)
+    lens = [321, 1, 128, 256]
+    o = operands(rule, 2, 64, 64, 0, lens)
+    clean = run(rule, o, 2, 64, 64, True, lens=lens)
     o["v"][70, 5], o["v"][72, 64 + 9] = float("inf"), float("nan")              # heads 0 and 1 of the first request
-    got = run(rule, o, 2, 64, 64, True)
+    got = run(rule, o, 2, 64, 64, True, lens=lens)
     same = torch.ones(clean[0].shape, dtype=torch.bool)
-    same[70:193, 0, 5] = same[72:193, 1, 9] = False
+    same[70:321, 0, 5] = same[72:321, 1, 9] = False
     assert torch.equal(got[0][same], clean[0][same])
-    assert not torch.isfinite(got[0][70:193, 0, 5]).any() and torch.isnan(got[0][72:193, 1, 9]).all()
+    assert not torch.isfinite(got[0][70:321, 0, 5]).any() and torch.isnan(got[0][72:321, 1, 9]).all()
