@@ -964,19 +964,17 @@ __global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ gate_
 
 // bf16 with the intermediate size a multiple of 8: a thread handles 8 outputs with 16-byte accesses.
 __global__ void silu_mul_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ gate_up,
-                                       int inter, long total8, int interleaved, int act,
+                                       int inter, int chunk, int interleaved, int act,
                                        const __nv_bfloat16* __restrict__ bias) {
     TW_TIMELINE_SCOPE(TW_K_SILU_MUL);
     tw_grid_wait();
     TW_TIMELINE_MARK();
     tw_grid_launch_dependents();
-    long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long step = (long)gridDim.x * blockDim.x;
-    const int groups = inter >> 3;
-    for (; idx < total8; idx += step) {
-        const long n = idx / groups;
-        const int j = (int)(idx - n * groups);
-        const __nv_bfloat16* row = gate_up + n * 2 * (long)inter;
+    // a block per row and `chunk` groups of eight, so that no thread divides (a running index over all rows: 33 us for 4,096
+    // rows of 4,736, now 31)
+    const int groups = inter >> 3, n = blockIdx.x, end = min(groups, ((int)blockIdx.y + 1) * chunk);
+    const __nv_bfloat16* row = gate_up + n * 2 * (long)inter;
+    for (int j = blockIdx.y * chunk + threadIdx.x; j < end; j += blockDim.x) {
         const uint4 gv = *reinterpret_cast<const uint4*>(row + (interleaved ? j * 16 : j * 8));
         const uint4 uv = *reinterpret_cast<const uint4*>(row + (interleaved ? j * 16 + 8 : inter + j * 8));
         const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gv);
@@ -1072,11 +1070,10 @@ TW_EXPORT int tw_silu_mul(void* out, const void* gate_up, int n_rows, int inter,
     long blocks = (total + 255) / 256;
     if (blocks > 148L * 16) blocks = 148L * 16;
     if (dtype == TW_BF16 && (inter & 7) == 0 && ((uintptr_t)bias & 3) == 0) {
-        const long total8 = total >> 3;
-        long b8 = (total8 + 255) / 256;
-        if (b8 > 148L * 16) b8 = 148L * 16;
-        tw_launch(silu_mul_bf16x8_kernel, dim3((int)b8), dim3(256), 0, stream, 1, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate_up, inter,
-                                                            total8, interleaved, act, (const __nv_bfloat16*)bias);
+        const int groups = inter >> 3, rows = (int)(total / inter);
+        const int chunk = rows >= 512 ? 1024 : 256;         // few rows: a group per thread, more blocks
+        tw_launch(silu_mul_bf16x8_kernel, dim3(rows, (groups + chunk - 1) / chunk), dim3(256), 0, stream, 1, (__nv_bfloat16*)out,
+                  (const __nv_bfloat16*)gate_up, inter, chunk, interleaved, act, (const __nv_bfloat16*)bias);
         return TW_LAUNCH_CHECK();
     }
     if (dtype == TW_F32)
