@@ -2067,6 +2067,47 @@ def moe_gather(xs: torch.Tensor, h: torch.Tensor, order: torch.Tensor, pairs: in
     _check(code, "moe_gather")
 
 
+# The largest step (rows) that runs its experts' products through csrc/moe_smallm.cu.  A layer of 8 experts of 4,736 (2 chosen, a
+# shared one), against the library's grouped product: 2 rows 122 and 161 us, 8 rows 158 and 238, 16 rows 177 and 238; 24 rows,
+# where the fragments of four tiles of rows leave too few loads under way, 286 and 257.
+MOE_ROWS_MOST = 16
+
+
+def moe_rows_supported(dtype: torch.dtype, rows: int, hidden: int, intermediate: int) -> bool:
+    """Whether csrc/moe_smallm.cu takes the experts' products of a step of ``rows`` rows: bfloat16, few rows, matrices whose rows
+    start on 16-byte boundaries."""
+    return dtype == torch.bfloat16 and 0 < rows <= MOE_ROWS_MOST and hidden % 8 == 0 and intermediate % 8 == 0
+
+
+def moe_rows_in(act: torch.Tensor, h: torch.Tensor, w: torch.Tensor, order: torch.Tensor, ends: torch.Tensor, n_rows: int, top: int,
+                how: int, limit: float = 0.0, alpha: float = 1.0) -> None:
+    """act[place] = glu(Wg_e x, Wu_e x) for the pairs sorted by expert (``moe_sort``), x the pair's row of ``h``; ``w``
+    [experts, 2, ff, width] with ``how`` one of the glus, or [experts, ff, width] with ``how`` one of ``ACTIVATIONS``."""
+    _cuda(act, h, w, order, ends)
+    gated = w.dim() == 4
+    experts, ff, width = w.shape[0], w.shape[-2], w.shape[-1]
+    _need(moe_rows_supported(h.dtype, n_rows, width, ff) and w.is_contiguous() and act.is_contiguous() and act.dtype == w.dtype == h.dtype
+          and act.shape[1] == ff and act.shape[0] >= n_rows * top and h.stride(1) == 1 and h.shape[1] == width and h.stride(0) % 8 == 0
+          and h.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and (not gated or w.shape[1] == 2), "moe_rows_in: bad operands")
+    _need(order.dtype == ends.dtype == torch.int32 and order.numel() >= n_rows * top and ends.numel() >= experts, "moe_rows_in: bad order")
+    code = _fn("moe_smallm", "tw_moe_rows_in")(_ptr(act), _ptr(h), c_int(h.stride(0)), _ptr(w), _ptr(order), _ptr(ends), c_int(ff),
+                                               c_int(width), c_int(experts), c_int(top), c_int(n_rows), c_int(1 if gated else 0), c_int(how),
+                                               c_float(limit), c_float(alpha), _stream())
+    _check(code, "moe_rows_in")
+
+
+def moe_rows_out(ys: torch.Tensor, act: torch.Tensor, w: torch.Tensor, ends: torch.Tensor, n_rows: int) -> None:
+    """ys[place] = Wd_e act[place] for the pairs sorted by expert; ``w`` [experts, width, ff]."""
+    _cuda(ys, act, w, ends)
+    experts, width, ff = w.shape
+    _need(moe_rows_supported(act.dtype, n_rows, width, ff) and w.is_contiguous() and act.is_contiguous() and ys.is_contiguous()
+          and act.dtype == w.dtype == ys.dtype and act.shape[1] == ff and ys.shape[1] == width and act.data_ptr() % 16 == 0
+          and w.data_ptr() % 16 == 0 and ends.dtype == torch.int32 and ends.numel() >= experts, "moe_rows_out: bad operands")
+    code = _fn("moe_smallm", "tw_moe_rows_out")(_ptr(ys), _ptr(act), _ptr(w), _ptr(ends), c_int(width), c_int(ff), c_int(experts),
+                                                c_int(n_rows), _stream())
+    _check(code, "moe_rows_out")
+
+
 def moe_combine(out: torch.Tensor, ys: torch.Tensor, place: torch.Tensor, weight: torch.Tensor, shared: torch.Tensor | None,
                 shared_gate: torch.Tensor | None, n_rows: int, chosen: torch.Tensor | None = None, h: torch.Tensor | None = None,
                 experts: int = 0, identity: int = 0) -> None:

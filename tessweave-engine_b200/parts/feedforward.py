@@ -310,6 +310,15 @@ class RoutedExperts(FeedForward):
         pairs = n * self.top
         order, place, ends, xs, act = buffers
         ops.moe_sort(order, place, ends, chosen, n)
+        if ops.moe_rows_supported(self.runtime.dtype, n, self.hidden, self.intermediate) and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0:
+            # few rows: kernels that stream every chosen expert's matrices once (the results take the sorted rows' place)
+            if self.gated:
+                ops.moe_rows_in(act, h, self.w_gate_up, order, ends, n, self.top, self.glu, self.glu_limit, self.glu_alpha)
+            else:
+                ops.moe_rows_in(act, h, self.w_up, order, ends, n, self.top, self.plain_act)
+            ops.moe_rows_out(xs, act, self.w_down, ends, n)
+            self._combine(out, xs, place, weight, shared, gate, n, chosen, h)
+            return
         ops.moe_gather(xs, h, order, pairs, self.top)
         if not self.gated:
             act = grouped_matmul_nt(xs, self.w_up, ends)
@@ -321,6 +330,9 @@ class RoutedExperts(FeedForward):
             else:
                 ops.glu_rows(act, gate_up, pairs, self.glu, self.glu_limit, self.glu_alpha)
         ys = grouped_matmul_nt(act, self.w_down, ends)
+        self._combine(out, ys, place, weight, shared, gate, n, chosen, h)
+
+    def _combine(self, out, ys, place, weight, shared, gate, n, chosen, h) -> None:
         if self.identity:
             ops.moe_combine(out, ys, place, weight, shared, gate, n, chosen=chosen, h=h, experts=self.experts, identity=self.identity)
         else:

@@ -14,6 +14,51 @@ def sorted_pairs(ops, chosen, experts):
     return order, place, ends
 
 
+@pytest.mark.parametrize("rows,experts,top,hidden,ff", [(1, 3, 1, 64, 24), (2, 4, 2, 200, 56), (8, 8, 2, 256, 136), (9, 2, 2, 72, 8),
+                                                       (13, 5, 3, 520, 64), (16, 6, 2, 1032, 328)])
+@pytest.mark.parametrize("kind", ["silu", "clamped", "plain"])
+def test_rows_through_their_experts(rows, experts, top, hidden, ff, kind):
+    """One expert that everybody chose, one that nobody did, a pair without an expert, sizes that fill no tile, rows inside
+    wider ones; against 64 bits."""
+    from tessweave_engine_b200.csrc import ops
+    g = torch.Generator().manual_seed(rows + hidden)
+    wide = torch.randn(rows, hidden + 16, generator=g).to(BF).cuda()
+    h = wide[:, 8:8 + hidden]
+    gated = kind != "plain"
+    w_in = (torch.randn(*((experts, 2, ff, hidden) if gated else (experts, ff, hidden)), generator=g) * hidden ** -0.5).to(BF).cuda()
+    w_out = (torch.randn(experts, hidden, ff, generator=g) * ff ** -0.5).to(BF).cuda()
+    pick = torch.stack([torch.randperm(max(1, experts - 1), generator=g)[:top] for _ in range(rows)]) if experts - 1 >= top else \
+        torch.arange(top).repeat(rows, 1)
+    pick[:, 0] = torch.where((pick[:, 1:] == 0).any(1), pick[:, 0], 0)
+    if rows > 4:
+        pick[3, top - 1] = experts                                                # an expert without matrices
+    chosen = pick.to(torch.int32).cuda()
+    order, place, ends = sorted_pairs(ops, chosen, experts)
+    nan = lambda *s: torch.full(s, float("nan"), device="cuda", dtype=BF)          # noqa: E731
+    act, ys = nan(rows * top, ff), nan(rows * top, hidden)
+    how = {"silu": ops.GLU_SILU, "clamped": ops.GLU_CLAMPED, "plain": ops.ACTIVATIONS["relu_squared"]}[kind]
+    ops.moe_rows_in(act, h, w_in, order, ends, rows, top, how, 1.5, 1.7)
+    ops.moe_rows_out(ys, act, w_out, ends, rows)
+    for r in range(rows):
+        for j in range(top):
+            e, at = int(pick[r, j]), int(place[r * top + j])
+            if e >= experts:
+                assert at == -1
+                continue
+            x, w = h[r].double(), w_in[e].double()
+            if gated:
+                a, b = w[0] @ x, w[1] @ x
+                want = torch.nn.functional.silu(a) * b if kind == "silu" else \
+                    (lambda a, b: a * torch.sigmoid(1.7 * a) * (b + 1))(a.clamp(max=1.5), b.clamp(-1.5, 1.5))
+            else:
+                want = torch.relu(w @ x) ** 2
+            # one rounding to bf16 (eight significant bits: 2^-8 of the value), sums of up to 1,032 products of size 1/32 in fp32
+            assert torch.allclose(act[at].double(), want, rtol=1.01 * 2 ** -8, atol=1e-5)
+            assert torch.allclose(ys[at].double(), w_out[e].double() @ act[at].double(), rtol=1.01 * 2 ** -8, atol=1e-5)
+    used = int(ends[-1])
+    assert torch.isnan(act[used:].float()).all() and torch.isnan(ys[used:].float()).all()
+
+
 @pytest.mark.parametrize("rows,width,experts,shared,how", [(128, 64, 3, False, 0), (130, 1160, 8, True, 0), (129, 3584, 20, True, 1),
                                                            (200, 776, 12, False, 2)])
 def test_router_of_many_rows(rows, width, experts, shared, how):
