@@ -23,7 +23,8 @@
 // can hold -- through scratch memory in the block that finishes last.
 //
 //   score = (q . k) * scale,  visible iff  tw_first_key(position, window) <= p <= position
-//   (`gate`: fp32 [rows][Hq] or null; head h's output is multiplied by its entry)
+//   (`gate`: fp32 [rows][Hq] or null; head h's output is multiplied by its entry.  `sink`: fp32 [Hq] or null; exp(sink[h]) joins
+//   head h's denominator)
 // Reference: flow_engine/model.py:193-200 and flow_engine/kernels/paged_decode.py:13-43.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets TW_ERR_WAIT in the status word, every role
@@ -112,6 +113,15 @@ __device__ __forceinline__ int tile_offset(int row, int chunk, int shift) {
     return line * 128 + (((chunk & 7) ^ (line & 7)) << 4);
 }
 
+// What a head's summed values are multiplied by: gate / sum, the sum with the sink's term (a term without key or value).
+// M, L: the maximum of the scores and their sum, in units of log2.
+__device__ __forceinline__ float normaliser(float M, float L, const float* sink, int head, float gate) {
+    if (!sink) return L > 0.f ? gate / L : 0.f;
+    const float s = sink[head] * 1.4426950408889634f, top = fmaxf(M, s);
+    const float f = M == -INFINITY ? 0.f : exp2f(M - top);
+    return f * gate / (L * f + exp2f(s - top));
+}
+
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CTHREADS) : "memory"); }
 
 template <bool CLUSTER, bool FUSED>
@@ -123,7 +133,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                        const int* __restrict__ block_table, int table_stride, int Hq, int Hkv, int page_size,
                        int num_pages, int window, float scale_log2e, int nsplit, int nstages,
                        float* __restrict__ partial_o, float* __restrict__ partial_ml, int* __restrict__ counters,
-                       int* status, const FusedQkv fq, const float* __restrict__ gate) {
+                       int* status, const FusedQkv fq, const float* __restrict__ gate, const float* __restrict__ sink,
+                       const int shared_kv) {
     static_assert(!FUSED || SAME_DIMS, "the fused form packs q, k and v as heads of one size");
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[MAX_STAGES];
@@ -196,10 +207,11 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // steps and may be fetched at once; otherwise the kernel before this one (or one before that) wrote the newest
         // position, and the copies wait for it.
         const bool values = warp > CWARPS;
+        const int stage_bytes = shared_kv ? KB * BLKB : STAGE_BYTES;     // (values that are the keys: the keys' copy serves as both)
         if (!(FUSED && fq.k_cache)) tw_grid_wait();
         TW_TTRACE(9);
         const CUtensorMap* map = values ? &map_v : &map_k;
-        const int boxes = TILE / box_rows, box_bytes = (values ? VB : KB) * box_rows * 128;
+        const int boxes = values && shared_kv ? 0 : TILE / box_rows, box_bytes = (values ? VB : KB) * box_rows * 128;
         unsigned char* place = ring + (values ? KB * BLKB : 0) + lane * box_bytes;
         int issued = 0, st = 0;
         uint32_t parity = 0;
@@ -223,7 +235,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             }
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) break;
-            if (row_coord >= 0) tma_load_3d(place + st * STAGE_BYTES, map, &full[st], 0, row_coord, 0);
+            if (row_coord >= 0) tma_load_3d(place + st * stage_bytes, map, &full[st], 0, row_coord, 0);
             issued = i + 1;
             if (++st == nstages) { st = 0; parity ^= 1; }
         }
@@ -330,11 +342,14 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // where this lane's rows of the fragments lie in a tile: keys krow, values vrow (read transposed)
         const int krow = warp * 16 + (lane & 15);
         const int mj = lane >> 3, vrow = warp * 16 + (mj >> 1) * 8 + (lane & 7);
-        int k_at[KSTEPS], v_at[MT_O];
+        // (the blocks of 64 columns of d lie `block` bytes apart and, but for pages of four keys, are swizzled alike)
+        const int block = box_rows * 128, toggle = box_rows < 8 ? 64 : 0;
+        int k_at[4], v_at[4];
 #pragma unroll
-        for (int ks = 0; ks < KSTEPS; ++ks) k_at[ks] = tile_offset<KB>(krow, 2 * ks + (lane >> 4), shift);
-#pragma unroll
-        for (int mt = 0; mt < MT_O; ++mt) v_at[mt] = tile_offset<VB>(vrow, 2 * mt + (mj & 1), shift);
+        for (int x = 0; x < 4; ++x) {
+            k_at[x] = tile_offset<KB>(krow, 2 * x + (lane >> 4), shift);
+            v_at[x] = tile_offset<VB>(vrow, 2 * x + (mj & 1), shift);
+        }
         bool ok = true;
         int st = 0;
         uint32_t parity = 0;
@@ -344,8 +359,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             if (warp == 0 && i == 0) TW_TTRACE(3);
             const int key0 = k_begin + i * TILE + warp * 16;
             if (key0 < k_end && key0 + 16 > first_key) {
-                unsigned char* ks_ = ring + st * STAGE_BYTES;
-                unsigned char* vs_ = ks_ + KB * BLKB;
+                unsigned char* ks_ = ring + st * (shared_kv ? KB * BLKB : STAGE_BYTES);
+                unsigned char* vs_ = shared_kv ? ks_ : ks_ + KB * BLKB;
                 // Value rows of keys this block must not see -- beyond the request's last key, before the window,
                 // or of a page that was never copied -- hold whatever was there: zero them (0 x NaN is NaN).
                 if (key0 < first_key || key0 + 16 > k_end) {
@@ -377,7 +392,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
                 for (int ks = 0; ks < KSTEPS; ++ks) {
                     uint32_t a[4];
-                    ldmatrix_x4(a, ks_ + k_at[ks]);
+                    ldmatrix_x4(a, ks_ + (ks >> 2) * block + (k_at[ks & 3] ^ ((ks >> 2) & 1 ? toggle : 0)));
                     mma_bf16_regs(sp[ks & 3], a[0], a[1], a[2], a[3], qb[ks][0], qb[ks][1]);
                 }
                 float sacc[4];
@@ -418,7 +433,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
                 for (int mt = 0; mt < MT_O; ++mt) {
                     uint32_t a[4];
-                    ldmatrix_x4_trans(a, vs_ + v_at[mt]);
+                    ldmatrix_x4_trans(a, vs_ + (mt >> 2) * block + (v_at[mt & 3] ^ ((mt >> 2) & 1 ? toggle : 0)));
                     mma_bf16_regs(oacc[mt], a[0], a[1], a[2], a[3], pb0, pb1);
                 }
             }
@@ -494,8 +509,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         }
         const int head = kvh * G + h0 + row;
         if (nsplit == 1) {
-            const float L = s_row_ml[row].y;
-            const float inv = L > 0.f ? tw_attn::head_gate(gate, n, Hq, head) / L : 0.f;
+            const float inv = normaliser(s_row_ml[row].x, s_row_ml[row].y, sink, head, tw_attn::head_gate(gate, n, Hq, head));
             uint2 packed;
             packed.x = pack_bf16(o.x * inv, o.y * inv);
             packed.y = pack_bf16(o.z * inv, o.w * inv);
@@ -541,7 +555,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 L = __fadd_rn(L, __fmul_rn(ml.y, f));      // (rounded as the merge through scratch memory rounds it)
                 o = fmaf(mine[(i * own4 + jj) * 4], f, o);
             }
-            const float inv = L > 0.f ? tw_attn::head_gate(gate, n, Hq, kvh * G + h0 + row) / L : 0.f;
+            const float inv = normaliser(M, L, sink, kvh * G + h0 + row, tw_attn::head_gate(gate, n, Hq, kvh * G + h0 + row));
             out[(size_t)n * out_stride + (size_t)(kvh * G + h0 + row) * DV + d] = __float2bfloat16_rn(o * inv);
         }
         if (warp == 0) TW_TTRACE(7);
@@ -606,7 +620,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             const float fj = f[i];
             o.x += v.x * fj; o.y += v.y * fj; o.z += v.z * fj; o.w += v.w * fj;
         }
-        const float inv = L > 0.f ? tw_attn::head_gate(gate, n, Hq, kvh * G + h0 + row) / L : 0.f;
+        const float inv = normaliser(s_row_max[row], L, sink, kvh * G + h0 + row, tw_attn::head_gate(gate, n, Hq, kvh * G + h0 + row));
         uint2 packed;
         packed.x = pack_bf16(o.x * inv, o.y * inv);
         packed.y = pack_bf16(o.z * inv, o.w * inv);
@@ -617,7 +631,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 constexpr int DEC_MAX_SPLITS = 128;
 static_assert(2 * HEADS * DEC_MAX_SPLITS * 4 <= MIN_STAGES * STAGE_BYTES, "the merge factors of the most slices must fit the ring");
 
-size_t smem_bytes(int nstages);
+size_t smem_bytes(int nstages, bool shared_kv = false);
 
 template <bool CLUSTER, bool FUSED>
 int prepare() {
@@ -634,17 +648,17 @@ int prepare() {
     return 0;
 }
 
-int g_cluster_ok[MAX_CLUSTER + 1][MAX_STAGES + 1] = {};      // 0 unknown, 1 fits, -1 does not
+int g_cluster_ok[2][MAX_CLUSTER + 1][MAX_STAGES + 1] = {};      // 0 unknown, 1 fits, -1 does not
 
-bool cluster_fits(int size, int nstages) {
+bool cluster_fits(int size, int nstages, bool shared_kv) {
     if (size < 2 || size > MAX_CLUSTER) return false;
-    int& known = g_cluster_ok[size][nstages];
+    int& known = g_cluster_ok[shared_kv][size][nstages];
     if (known == 0) {
         if (prepare<true, false>() != 0) return false;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(size);
         cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = smem_bytes(nstages);
+        cfg.dynamicSmemBytes = smem_bytes(nstages, shared_kv);
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = size;
@@ -660,7 +674,7 @@ bool cluster_fits(int size, int nstages) {
     return known > 0;
 }
 
-size_t smem_bytes(int nstages) { return (size_t)nstages * STAGE_BYTES + 1024; }
+size_t smem_bytes(int nstages, bool shared_kv) { return (size_t)nstages * (shared_kv ? KB * BLKB : STAGE_BYTES) + 1024; }
 
 int g_sm_count = 0;
 
@@ -689,7 +703,9 @@ TW_EXPORT int tw_attn_decode_tma_supported(int page_size) {
 // duty to store the new key and value.  `nstages` is the depth of the ring (0: as deep as one block per SM
 // allows while the launch has no more blocks than SMs, else half of that so that two blocks share an SM).
 // `scratch` and `counters` as for tw_attn_decode; they are used when the slices do not fit a cluster.
-// `gate` (fp32 [rows][Hq] or null): head h's output of a row is multiplied by its entry.
+// `gate` (fp32 [rows][Hq] or null): head h's output of a row is multiplied by its entry.  `sink` (fp32 [Hq] or null, with `q`
+// only): exp(sink[h]) joins head h's denominator.  v_cache may be k_cache (with `q` only): a position's value is its key, which
+// is copied once and read as both.
 TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q_stride, const float* partial, int nslices,
                                  long long slice_stride, const void* dense, int dense_stride, const float* bias,
                                  const float* inv_freq, int write_cache, const int* seq_q_start, const int* seq_q_len,
@@ -697,10 +713,12 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
                                  void* k_cache, void* v_cache, int n_seqs, int Hq, int Hkv, int page_size, int num_pages,
                                  int window, float scale, int nsplit, int nstages, int flags, float* scratch, int* counters,
                                  int* status, const void* next_weights, long long next_bytes, const float* gate,
-                                 cudaStream_t stream) {
+                                 const float* sink, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     const bool fused = partial || dense;
-    if (fused && !SAME_DIMS) return (int)cudaErrorInvalidValue;
+    const bool shared_kv = k_cache == v_cache;
+    if ((fused || shared_kv) && !SAME_DIMS) return (int)cudaErrorInvalidValue;
+    if (fused && (shared_kv || sink)) return (int)cudaErrorInvalidValue;
     if (Hkv <= 0 || Hq % Hkv || nsplit < 1 || nsplit > DEC_MAX_SPLITS || !tw_attn_decode_tma_supported(page_size) ||
         (!fused && !q) || (partial && nslices < 1) || (nsplit > 1 && (!scratch || !counters)))
         return (int)cudaErrorInvalidValue;
@@ -714,10 +732,13 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
     }
     const int G = Hq / Hkv, htiles = (G + HEADS - 1) / HEADS;
     const long long blocks = (long long)nsplit * htiles * Hkv * n_seqs;
-    const int deepest = tw_attn_decode_tma_max_stages();
-    if (nstages <= 0) nstages = blocks <= g_sm_count ? deepest : (113 * 1024 - STATIC_SMEM_ROOM) / STAGE_BYTES;
+    // (with one copy for keys and values a stage is half as large; as many stages as the barriers allow)
+    const int stage_bytes = shared_kv ? KB * BLKB : STAGE_BYTES;
+    const int deepest = shared_kv ? (MAX_STAGES < 2 * DEEPEST ? MAX_STAGES : 2 * DEEPEST) : tw_attn_decode_tma_max_stages();
+    const int least = shared_kv ? ((MERGE_BYTES + stage_bytes - 1) / stage_bytes > 2 ? (MERGE_BYTES + stage_bytes - 1) / stage_bytes : 2) : MIN_STAGES;
+    if (nstages <= 0) nstages = blocks <= g_sm_count ? deepest : (113 * 1024 - STATIC_SMEM_ROOM) / stage_bytes;
     if (nstages > deepest) nstages = deepest;
-    if (nstages < MIN_STAGES) nstages = MIN_STAGES;
+    if (nstages < least) nstages = least;
     const long long rows = (long long)num_pages * Hkv * page_size;
     if (rows >= (1ll << 31)) return (int)cudaErrorInvalidValue;
     const int box_rows = page_size < TILE ? page_size : TILE;
@@ -735,16 +756,16 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
         fq.next_weights = next_weights; fq.next_bytes = next_weights ? next_bytes : 0;
     }
     const dim3 grid(nsplit * htiles, Hkv, n_seqs);
-    const size_t smem = smem_bytes(nstages);
+    const size_t smem = smem_bytes(nstages, shared_kv);
     const float scale_log2e = scale * 1.4426950408889634f;
-    const bool cluster = nsplit > 1 && !(flags & 1) && cluster_fits(nsplit, nstages);
+    const bool cluster = nsplit > 1 && !(flags & 1) && cluster_fits(nsplit, nstages, shared_kv);
 #define TW_DECODE_TMA_LAUNCH(CL, FU)                                                                                   \
     do {                                                                                                               \
         if (int e = prepare<CL, FU>()) return e;                                                                       \
         return tw_launch(attn_decode_tma_kernel<CL, FU>, grid, dim3(THREADS), smem, stream, CL ? nsplit : 1, mk, mv,    \
                          (bf16*)out, out_stride, (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, \
                          block_table, table_stride, Hq, Hkv, page_size, num_pages, window, scale_log2e, nsplit, nstages, \
-                         partial_o, partial_ml, counters, status, fq, gate);                                              \
+                         partial_o, partial_ml, counters, status, fq, gate, sink, (int)shared_kv);                         \
     } while (0)
     if constexpr (SAME_DIMS) {
         if (cluster && fused) TW_DECODE_TMA_LAUNCH(true, SAME_DIMS);

@@ -1166,13 +1166,14 @@ def decode_attention_resident_early(blocks: int, nsplit: int) -> bool:
 def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_start, seq_q_len, seq_kv_len, seq_slot,
                          block_table, k_pages, v_pages, n_seqs, n_q_heads, n_kv_heads, head_dim, window, scale, nsplit,
                          scratch, counters, status, merge_in_scratch: bool = False, prefetch: torch.Tensor | None = None,
-                         stages: int = 0, gate: torch.Tensor | None = None) -> None:
+                         stages: int = 0, gate: torch.Tensor | None = None, sink: torch.Tensor | None = None) -> None:
     """Split-KV attention for the requests of the batch that bring one token, keys and values brought in by TMA.
     Either ``q`` (bf16 [rows, Hq D], 16-byte aligned rows) or ``source`` -- the step's untouched q/k/v product, a
     ``SplitSum`` or a bf16 [rows, (Hq + 2 Hkv) D] tensor, which the kernel biases, rotates and (``write_cache``)
     stores itself -- is given.  The other arguments are those of ``attention_decode`` / ``attention_decode_fused``;
     ``stages`` is the depth of a block's ring of 64-key tiles (0: chosen from the size of the launch).  ``window`` and
-    ``gate``: as for ``attention_decode``; with ``q`` the values may have another size than the keys."""
+    ``gate``: as for ``attention_decode``; with ``q`` the values may have another size than the keys, or be the keys (the same
+    pages), and ``sink`` (fp32 [Hq]) may join the denominator."""
     import os
     width = (n_q_heads + 2 * n_kv_heads) * head_dim
     partial = dense = None
@@ -1191,8 +1192,11 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
         _need(q is not None and q.is_cuda and q.dtype == torch.bfloat16 and q.stride(1) == 1 and q.data_ptr() % 16 == 0
               and q.stride(0) % 8 == 0, "attention_decode_tma: q must be bf16 with 16-byte aligned rows")
     _cuda(out, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table, k_pages, v_pages, scratch, counters, status,
-          bias, inv_freq, prefetch, gate)
+          bias, inv_freq, prefetch, gate, sink)
     _gate_check(gate, 0, n_q_heads)
+    _need(sink is None or (source is None and sink.dtype == torch.float32 and sink.numel() == n_q_heads and sink.is_contiguous()),
+          "attention_decode_tma: the sink must be fp32 [Hq], with q given")
+    _need(source is None or k_pages.data_ptr() != v_pages.data_ptr(), "attention_decode_tma: values that are the keys go with q given")
     v_dim = v_pages.shape[3]
     _need(decode_tma_supported(out.dtype, head_dim, k_pages.shape[2], v_dim) or os.environ.get("TESSWEAVE_DECODE_TMA") == "0",
           f"attention_decode_tma does not take head size {head_dim} with pages of {k_pages.shape[2]} keys in {out.dtype}")
@@ -1223,7 +1227,7 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
         _ptr(block_table), c_int(block_table.shape[1]), _ptr(k_pages), _ptr(v_pages), c_int(n_seqs), c_int(n_q_heads),
         c_int(n_kv_heads), c_int(k_pages.shape[2]), c_int(k_pages.shape[0]), c_int(window), c_float(scale), c_int(nsplit),
         c_int(stages), c_int(1 if merge_in_scratch else 0), _ptr(scratch), _ptr(counters), _ptr(status), _ptr(prefetch),
-        ctypes.c_longlong(prefetch.numel() * prefetch.element_size() if prefetch is not None else 0), _ptr(gate), _stream())
+        ctypes.c_longlong(prefetch.numel() * prefetch.element_size() if prefetch is not None else 0), _ptr(gate), _ptr(sink), _stream())
     _check(code, "attention_decode_tma")
 
 

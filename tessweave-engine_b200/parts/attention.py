@@ -15,8 +15,8 @@ class PagedSoftmaxMixer(Mixer):
     """What mixers that attend with a softmax over a paged cache share: the choice of the attention kernel for a
     step.  A subclass sets ``n_heads, n_kv_heads, head_dim, v_dim, same_dims, q_size, window, scale, sink, bias_rows,
     bias_by_distance, score_terms`` (``score_terms``: the softmax has a sink or a distance table, or the values are
-    the keys -- what only the exact and the mma.sync kernels know), and ``chunk`` where a token sees its own chunk of
-    positions instead of a window, and hands ``_attend`` rows whose first ``q_size`` columns are the queries, after it
+    the keys -- what only the exact and the mma.sync kernels know, and but for the table the decode kernel fed by TMA),
+    and ``chunk`` where a token sees its own chunk of positions instead of a window, and hands ``_attend`` rows whose first ``q_size`` columns are the queries, after it
     has stored the step's keys and values."""
 
     b_qkv = None
@@ -38,7 +38,9 @@ class PagedSoftmaxMixer(Mixer):
     def _decode_launch(self, ctx: StepContext, cache: PagedView) -> tuple[bool, int, int]:
         """(fed by TMA?, slices per request, blocks) of the decode attention this step will launch."""
         group = self.n_heads // self.n_kv_heads
-        tma = not self.score_terms and ops.decode_tma_supported(self.runtime.dtype, self.head_dim, cache.page_size, self.v_dim)
+        # (a table by distance is what the kernel fed by TMA does not know.  8 requests of 4,096 cached rows of 256 that are keys and
+        # values of 28 heads: 28.5 us with keys loaded through registers, 16.6 through TMA)
+        tma = self.bias_rows is None and ops.decode_tma_supported(self.runtime.dtype, self.head_dim, cache.page_size, self.v_dim)
         # (the keys a request can see: a window or a chunk bounds them, and the kernels cut those into the slices)
         seen = min(ctx.max_kv_len, self.span) if self.span else ctx.max_kv_len
         nsplit = (ops.decode_tma_splits(ctx.n_seqs, self.n_kv_heads, group, seen) if tma
@@ -87,7 +89,8 @@ class PagedSoftmaxMixer(Mixer):
             ops.attention_decode_tma(out, q, product, self.b_qkv if fused is not None else None, table, write_cache,
                                      ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.seq_slot, cache.block_table,
                                      cache.k_pages, cache.v_pages, ctx.n_seqs, self.n_heads, self.n_kv_heads, self.head_dim,
-                                     window, self.scale, nsplit, scratch, counters, ctx.status, prefetch=prefetch, gate=gate)
+                                     window, self.scale, nsplit, scratch, counters, ctx.status, prefetch=prefetch, gate=gate,
+                                     sink=self.sink if self.score_terms else None)
         elif fused is not None:
             ops.attention_decode_fused(out, product, self.b_qkv, table, write_cache, ctx.seq_q_start, ctx.seq_q_len,
                                        ctx.seq_kv_len, ctx.seq_slot, cache.block_table, cache.k_pages, cache.v_pages,

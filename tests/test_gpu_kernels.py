@@ -407,6 +407,34 @@ def run_tensor_core_attention(setup, rows_of, q, hq, hkv, d, window, nsplit=None
     return out.float().cpu().reshape(n, hq, d), qd.float().cpu().reshape(n, hq, d)
 
 
+@pytest.mark.parametrize("page", [4, 16, 64])
+@pytest.mark.parametrize("hq,hkv,d", [(28, 1, 256), (4, 2, 64), (9, 3, 128), (3, 1, 192)])
+@pytest.mark.parametrize("window,nsplit,in_scratch", [(0, 1, False), (0, 5, False), (90, 3, True)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_decode_attention_tma_sinks_and_values_that_are_keys(page, hq, hkv, d, window, nsplit, in_scratch, shared):
+    """The kernel fed by TMA with a sink per head, with pages that serve as keys and values, with pages that are fractions of a
+    tile; slices merged in one block, in a cluster and through scratch memory."""
+    o = ops()
+    lengths = [1, 300, 65, 257]
+    setup = paged_setup(lengths, page, hkv, d, torch.bfloat16, seed=d + page)
+    g = torch.Generator().manual_seed(6)
+    n = len(lengths)
+    q, sink = dev(torch.randn(n, hq * d, generator=g), torch.bfloat16), dev(torch.randn(hq, generator=g))
+    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))                               # noqa: E731
+    out = torch.full((n, hq * d), float("nan"), device="cuda", dtype=torch.bfloat16)
+    scratch = torch.full((o.decode_scratch_floats(hq, d),), float("nan"), device="cuda")
+    counters = torch.zeros(o.decode_counter_ints(n, hkv, hq // hkv), dtype=torch.int32, device="cuda")
+    st = status()
+    o.attention_decode_tma(out, q, None, None, None, False, i32(range(n)), i32([1] * n), i32(lengths), i32(setup["slots"]), setup["table"],
+                           setup["k_pages"], setup["k_pages"] if shared else setup["v_pages"], n, hq, hkv, d, window, d ** -0.5, nsplit,
+                           scratch, counters, st, merge_in_scratch=in_scratch, sink=sink)
+    assert int(st) == 0 and int(counters.abs().sum()) == 0
+    for i, m in enumerate(lengths):
+        k, v = (setup[x][i].to(torch.bfloat16).float() for x in ("k", "k" if shared else "v"))
+        want = dense_attention(q[i:i + 1].float().cpu().view(1, hq, d), k, v, [m - 1], window or None, sink=sink.cpu())
+        assert torch.allclose(out[i:i + 1].float().cpu().view(1, hq, d), want, **TOL["bfloat16"]), f"request {i}"
+
+
 @pytest.mark.parametrize("hq,hkv,d", TC_CASES)
 @pytest.mark.parametrize("window", [0, 24])
 def test_tensor_core_attention_mixed_rows(hq, hkv, d, window):
