@@ -571,6 +571,96 @@ short_conv_rows_kernel(OT* __restrict__ out, const T* __restrict__ x, int x_stri
     }
 }
 
+// The same where a unit head is 32, 64 or 128 channels, or there is none: a warp serves that many channels of four
+// rows, lane l the channels l, l + 32, ..., so a head's sum of squares is a shuffle in the order of the kernels above (the
+// same bits) and nothing goes through shared memory.  What is the same for a row (its request, how far it lies from the
+// request's start) is found once per row by one lane, and taps are looked up in the state only in warps whose rows lie that
+// near to a start.  What bounds it is latency, of the loads and of a row's chain (without the activation it still takes 21
+// us), so a warp takes four rows: eight 27.6 us, sixteen 32.4, four 23.1.  2,002 rows of 3,584 channels, 14 of 28 heads
+// unit: 45 us with short_conv_rows_kernel, 23 here.
+#define TW_CONV_HEAD_ROWS 4
+template <typename T, typename OT, int TAPS, int PER>
+__global__ void __launch_bounds__(128)
+short_conv_heads_kernel(OT* __restrict__ out, const T* __restrict__ x, int x_stride, const float* __restrict__ w, int w_c, int w_j,
+                        const float* __restrict__ bias, float* __restrict__ state, long long state_stride, long long state_offset,
+                        const int* __restrict__ seq_of_token, const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start,
+                        const int* __restrict__ seq_q_len, int move_single, int n_rows, int channels, int unit_heads,
+                        int scaled_heads, float head_scale, float unit_eps) {
+    constexpr int R = TW_CONV_HEAD_ROWS, P = TAPS - 1;
+    tw_grid_wait();
+    tw_grid_launch_dependents();
+    const int lane = threadIdx.x & 31;
+    const int head = blockIdx.y * 4 + (threadIdx.x >> 5);
+    const int c0 = head * 32 * PER + lane;               // this lane's channels: c0 + 32 k
+    if (head * 32 * PER >= channels) return;
+    const int row0 = blockIdx.x * R, nr = min(R, n_rows - row0);
+    int seq = -1, before = 0;                            // lane i: row i's request, and its rows before this one in the step
+    if (lane < nr) {
+        seq = seq_of_token[row0 + lane];
+        if (seq >= 0) before = row0 + lane - seq_q_start[seq];
+    }
+    const bool near_start = __any_sync(0xffffffffu, seq >= 0 && before < P);
+    float wt[TAPS][PER], b[PER], xr[P + R][PER];         // the rows before (whichever request they belong to), then the warp's own
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int c = c0 + 32 * k;
+        const bool in = c < channels;
+#pragma unroll
+        for (int i = 0; i < P + R; ++i) {
+            const int rr = row0 - P + i;
+            xr[i][k] = in && rr >= 0 && i - P < nr ? tw_to_float(x[(size_t)rr * x_stride + c]) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) wt[j][k] = in ? w[(size_t)c * w_c + (size_t)j * w_j] : 0.f;
+        b[k] = in && bias ? bias[c] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int s = __shfl_sync(0xffffffffu, seq, i);
+        if (s < 0) continue;                             // (no request's row, or behind the last; the whole warp)
+        float y[PER];
+        if (near_start) {
+            const int r = __shfl_sync(0xffffffffu, before, i);
+            const bool move = move_single && TAPS > 1 && r == 0 && seq_q_len[s] == 1;
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const int c = c0 + 32 * k;
+                y[k] = b[k];
+                if (c >= channels) continue;
+                float* tc = state + (size_t)seq_slot[s] * state_stride + state_offset + (size_t)c * P;
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) {
+                    const int back = P - j;
+                    const float xv = back <= r ? xr[i + j][k] : tc[P + r - back];
+                    y[k] += wt[j][k] * xv;
+                    if (move && j > 0) tc[j - 1] = xv;   // r == 0: xv is input j of (state, own row); place j - 1 has been read
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                y[k] = b[k];
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) y[k] += wt[j][k] * xr[i + j][k];
+            }
+        }
+        float f = 1.0f;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) y[k] = y[k] / (1.0f + expf(-y[k]));
+        if (head < unit_heads) {
+            float ss = 0.f;
+#pragma unroll
+            for (int k = 0; k < PER; ++k) ss += y[k] * y[k];
+            ss = tw_warp_sum(ss);
+            f = (head < scaled_heads ? head_scale : 1.0f) / sqrtf(ss + unit_eps);
+        }
+        OT* orow = out + (size_t)(row0 + i) * channels + c0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (c0 + 32 * k < channels) orow[32 * k] = tw_from_float<OT>(head < unit_heads ? y[k] * f : y[k]);
+    }
+}
+
 // bf16 in and out, no unit heads, four taps or fewer, channels in groups of eight on 16-byte boundaries: a thread serves
 // eight channels of TW_CONV_WIDE_ROWS consecutive rows with 16-byte accesses, the inputs of the rows before in registers.
 #define TW_CONV_WIDE_ROWS 8
@@ -687,6 +777,29 @@ static int launch_short_conv(OT* out, const T* x, int x_stride, const float* w, 
             TW_CONV_WIDE_LAUNCH(4)
 #undef TW_CONV_WIDE_LAUNCH
         }
+    }
+    // Many rows and heads of a warp's size (or none): no shared memory.  Other head sizes go on below.
+    if (n_rows >= 8 * TW_CONV_ROWS && taps <= TW_CONV_FAST_TAPS && (unit_heads == 0 || unit_dim == 32 || unit_dim == 64 || unit_dim == 128)) {
+        const int per = unit_heads == 0 ? 4 : unit_dim / 32;
+        const dim3 hgrid((n_rows + TW_CONV_HEAD_ROWS - 1) / TW_CONV_HEAD_ROWS, (channels + 4 * 32 * per - 1) / (4 * 32 * per));
+#define TW_CONV_HEADS_LAUNCH(TAPS, PER)                                                                                          \
+        return tw_launch(short_conv_heads_kernel<T, OT, TAPS, PER>, hgrid, dim3(128), 0, stream, 1, out, x, x_stride, w, w_c, w_j, bias, state, \
+                         state_stride, state_offset, seq_of_token, seq_slot, seq_q_start, seq_q_len, move_single, n_rows,       \
+                         channels, unit_heads, scaled_heads, head_scale, unit_eps);
+#define TW_CONV_HEADS_TAPS(TAPS)                                                                                                 \
+        {                                                                                                                        \
+            if (per == 1) { TW_CONV_HEADS_LAUNCH(TAPS, 1) }                                                                      \
+            if (per == 2) { TW_CONV_HEADS_LAUNCH(TAPS, 2) }                                                                      \
+            TW_CONV_HEADS_LAUNCH(TAPS, 4)                                                                                        \
+        }
+        switch (taps) {
+        case 1: TW_CONV_HEADS_TAPS(1)
+        case 2: TW_CONV_HEADS_TAPS(2)
+        case 3: TW_CONV_HEADS_TAPS(3)
+        default: TW_CONV_HEADS_TAPS(4)
+        }
+#undef TW_CONV_HEADS_TAPS
+#undef TW_CONV_HEADS_LAUNCH
     }
     // about 512 channels per block, in whole unit heads while there are any (a head larger than that has a block of its own)
     int chunk = 512;

@@ -1094,3 +1094,42 @@ def test_short_convolution_over_a_mixed_batch(dtype, taps, lengths):
     assert float((out[:n].cpu().double() - want).abs().max()) <= 2e-5
     assert bool((out[n:] == 7.0).all()), "padding rows were written"
     assert float((st.cpu().double() - want_state).abs().max()) <= 1e-6, "the convolutions' last inputs"
+
+
+@pytest.mark.parametrize("dtype,out", [("float32", "float32"), ("bfloat16", "float32"), ("bfloat16", "bfloat16")])
+@pytest.mark.parametrize("taps,unit_heads,unit_dim,channels", [(4, 3, 128, 640), (4, 2, 64, 200), (2, 3, 32, 104), (1, 1, 128, 129), (3, 0, 0, 517)])
+def test_short_convolution_a_head_per_warp(dtype, out, taps, unit_heads, unit_dim, channels):
+    """Steps with many rows (a warp per head) give the bits of steps with few rows (a block per row): requests of one row,
+    shorter than the taps, ending inside and at the edge of eight rows, rows of no request, and the states moved on."""
+    from tessweave_engine_b200.csrc import ops
+    dev, keep, offset = torch.device("cuda"), taps - 1, 3
+    g = torch.Generator().manual_seed(channels)
+    lengths = [1, 37, 2, 8, 1, 41, 3]
+    n, pad = sum(lengths), 3
+    x = torch.randn(n + pad, channels + 2, generator=g).to(DTYPES[dtype]).to(dev)
+    w = (torch.randn(channels, taps, generator=g) * 0.5).to(dev)
+    bias = torch.randn(channels, generator=g).to(dev)
+    state = torch.randn(len(lengths) + 1, offset + channels * keep, generator=g).to(dev)
+    slots = torch.randperm(len(lengths), generator=g).to(torch.int32).to(dev)
+    kw = dict(unit_heads=unit_heads, unit_dim=unit_dim, scaled_heads=min(1, unit_heads), head_scale=0.25, unit_eps=1e-6, bias=bias)
+
+    def step(rows, lens, slots, st):
+        many = torch.full((rows.shape[0], channels), 7.0, device=dev, dtype=DTYPES[out])
+        seq = torch.cat([torch.full((L,), i, dtype=torch.int32) for i, L in enumerate(lens)]
+                        + [torch.full((rows.shape[0] - sum(lens),), -1, dtype=torch.int32)]).to(dev)
+        starts = torch.tensor([sum(lens[:i]) for i in range(len(lens))], dtype=torch.int32, device=dev)
+        count = torch.tensor(lens, dtype=torch.int32, device=dev)
+        ops.short_conv(many, rows, w, st, offset, seq, slots, starts, rows.shape[0], move_single=count, **kw)
+        if keep:
+            ops.short_conv_state(rows, taps, channels, st, offset, slots, starts, count, len(lens), skip_single=True)
+        return many
+
+    moved, want_state = state.clone(), state.clone()
+    got = step(x, lengths, slots, moved)
+    want, at = [], 0
+    for i, L in enumerate(lengths):
+        want.append(step(x[at:at + L].contiguous(), [L], slots[i:i + 1].contiguous(), want_state))
+        at += L
+    torch.cuda.synchronize()
+    assert torch.equal(got[:n], torch.cat(want)) and torch.equal(moved, want_state)
+    assert bool((got[n:] == 7.0).all()), "rows of no request were written"
