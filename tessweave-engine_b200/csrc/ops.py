@@ -1408,6 +1408,28 @@ def gemm_small_m(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, kp
     _check(code, "gemm_small_m")
 
 
+NARROW_MOST = 64                 # outputs up to which csrc/gemm_smallm.cu: tw_gemm_narrow takes a product
+
+
+def gemm_narrow_supported(x: torch.Tensor, w: torch.Tensor, m: int) -> bool:
+    """Whether a product of many rows and few outputs goes through ``gemm_narrow``: bfloat16 on 16-byte boundaries."""
+    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and m > SMALL_M_LIMIT and 0 < w.shape[0] <= NARROW_MOST
+            and w.shape[1] % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0 and x.stride(1) == 1
+            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+
+
+def gemm_narrow(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int) -> None:
+    """out[:m] = x[:m] @ w.T for few outputs; ``out`` is bf16 or fp32 [>=m, n]."""
+    _cuda(out, x, w)
+    n, k = w.shape
+    _need(gemm_narrow_supported(x, w, m) and x.shape[0] >= m and x.shape[1] == k, "gemm_narrow: bf16 operands on 16-byte boundaries, at most 64 outputs")
+    _need(out.dim() == 2 and out.stride(1) == 1 and out.shape[0] >= m and out.shape[1] == n and out.dtype in (torch.bfloat16, torch.float32),
+          "gemm_narrow: bad output")
+    code = _fn("gemm_smallm", "tw_gemm_narrow")(_ptr(out), c_int(out.stride(0)), _ptr(x), c_int(x.stride(0)), _ptr(w), c_int(m), c_int(n),
+                                                c_int(k), c_int(dtype_code(out.dtype)), _stream())
+    _check(code, "gemm_narrow")
+
+
 # ---------------------------------------------------------------------------
 # matrix products of prompt steps on pairs of thread blocks
 # ---------------------------------------------------------------------------

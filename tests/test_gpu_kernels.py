@@ -1133,3 +1133,25 @@ def test_short_convolution_a_head_per_warp(dtype, out, taps, unit_heads, unit_di
     torch.cuda.synchronize()
     assert torch.equal(got[:n], torch.cat(want)) and torch.equal(moved, want_state)
     assert bool((got[n:] == 7.0).all()), "rows of no request were written"
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k,stride", [(9, 1, 8, 8), (17, 8, 520, 528), (100, 28, 3584, 3584), (2048, 28, 3584, 3584),
+                                          (333, 9, 72, 80), (65, 33, 1000, 1000), (16, 64, 4104, 4104)])
+def test_product_of_many_rows_and_few_outputs(m, n, k, stride, out_dtype):
+    """Remainders of rows, outputs and k, rows that lie apart.  The bound: fp32 sums of k products, k 2^-24 of the sum of
+    their sizes and as much again for the tensor cores' shorter additions; one rounding more in bfloat16 (2^-8)."""
+    from tessweave_engine_b200.csrc import ops
+    g = torch.Generator().manual_seed(m + n + k)
+    x = torch.randn(m + 1, stride, generator=g).to(torch.bfloat16)[:, :k]
+    w = torch.randn(n, k, generator=g).to(torch.bfloat16)
+    out = torch.full((m + 2, n + 3), 7.0, device="cuda", dtype=out_dtype)
+    xd = x.cuda()
+    xd = torch.as_strided(torch.nn.functional.pad(xd, (0, stride - k)).contiguous(), (m + 1, k), (stride, 1))
+    ops.gemm_narrow(out[:, :n], xd, w.cuda(), m)
+    torch.cuda.synchronize()
+    want = x[:m].double() @ w.double().t()
+    size = x[:m].double().abs() @ w.double().abs().t()
+    bound = 2 * k * 2.0 ** -24 * size + (want.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out[:m, :n].cpu().double() - want).abs() <= bound + 1e-30).all())
+    assert bool((out[m:] == 7.0).all()) and bool((out[:, n:] == 7.0).all()), "values behind the result were written"
