@@ -70,8 +70,8 @@ class MinGRU(Mixer):
 
 class MatrixStateMixer(Mixer):
     """What the mixers below share: a matrix state S [key_dim, value_dim] per head in a fixed-size slot, walked by
-    ``ops.linear_recurrence`` (one rule per mixer), then the norm over each head, an optional weight and a gate
-    (``ops.head_norm_gate``), then the output matrix.  The raw outputs and the state are fp32."""
+    ``ops.linear_recurrence`` (one rule per mixer) or, over prompt portions where the rule has a form in chunks, by that,
+    then the norm over each head, an optional weight and a gate (``ops.head_norm_gate``), then the output matrix.  The raw outputs and the state are fp32."""
 
     rule: int = -1
     gate_act: int = ops.GATE_NONE
