@@ -18,9 +18,17 @@
 // its share of them to be brought into L2 when its own stream is over, so that the memory system has work
 // while the last blocks finish and the next kernel starts (gate/up before down, 7B-size layer: 0.7 % of a step).
 //
+// Where the consumer cannot add slices, the blocks of a row tile, one per slice, form a cluster: every block sends its
+// sums to the shared memory of the block that adds those values, in the order above, so the product takes no second
+// kernel and its sums no way through memory (8 rows of 3,584 to 1,792 values: 5.1 us and 3.9 to add the slices, 6.1 so).
+//
 // The reference runs these products through a library (nn.Linear: flow_engine/model.py:54,
 // 76-80,201,204).
 #include "common.cuh"
+
+#include <cooperative_groups.h>
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -49,6 +57,8 @@ constexpr int WARPS = TW_GEMM_WARPS;
 constexpr int ROWS_PER_BLOCK = WARPS * 16;
 constexpr int CHUNK = 64;      // values of k per step: a thread reads 32 contiguous bytes of each of its rows
 
+constexpr int MERGE_MOST = 8;  // slices a cluster adds (the portable cluster size)
+
 enum : int { OUT_BF16 = 0, OUT_F32 = 1, OUT_PARTIAL = 2, OUT_GATED = 3, OUT_EARLY_DEPENDENTS = 16 /* flag, or-ed in */ };
 
 struct Frag {          // 16 consecutive values of k of one row
@@ -61,13 +71,18 @@ struct Frag {          // 16 consecutive values of k of one row
 // at 8 rows 52 -> 45 us.
 // EPI: the sums get a bias or an activation other than SiLU on gates (kept apart, since it takes registers from the
 // stream of the plain form).
-template <int NT, int KS, bool EPI>
+// MERGE: the grid is (slices, row tiles) and the slices of a row tile a cluster that merges its sums (up to 8 rows).
+template <int NT, int KS, bool EPI, bool MERGE>
 __global__ void __launch_bounds__(WARPS * 32, (NT == 1 ? 5 : 0))
 gemm_smallm_kernel(const bf16* __restrict__ w, const bf16* __restrict__ x, int M, int N, int K, int kper,
                    void* __restrict__ out, int out_mode, int out_stride, const TwEpilogue ep, const void* next_weights,
                    long long next_bytes) {
     constexpr int TILES = WARPS / KS;                  // 16-row tiles of a block
     __shared__ float s_part[KS > 1 ? TILES * 32 * NT * 4 : 1];
+    constexpr int TILE_ROWS = TILES * 16;
+    __shared__ float s_merge[MERGE ? (TILE_ROWS + 1) * 8 * NT : 1];      // [slice][this block's share of the tile's sums]
+    const int row_block = MERGE ? blockIdx.y : blockIdx.x, slice = MERGE ? blockIdx.x : blockIdx.y;
+    if constexpr (MERGE) cg::this_cluster().barrier_arrive();            // (waited for before the first remote store)
     TW_TIMELINE_SCOPE(TW_K_GEMM_SMALLM);
     tw_grid_wait();
     TW_TIMELINE_MARK();
@@ -80,9 +95,9 @@ gemm_smallm_kernel(const bf16* __restrict__ w, const bf16* __restrict__ x, int M
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;
     const int tile = warp % TILES, khalf = warp / TILES;
-    const int r0 = blockIdx.x * (TILES * 16) + tile * 16;
-    if (KS == 1 && r0 >= N) return;
-    const int kbeg0 = blockIdx.y * kper, kend0 = min(K, kbeg0 + kper);
+    const int r0 = row_block * TILE_ROWS + tile * 16;
+    if (!MERGE && KS == 1 && r0 >= N) return;
+    const int kbeg0 = slice * kper, kend0 = min(K, kbeg0 + kper);
     // with KS > 1: this warp's share of the block's values of k, in whole steps
     const int span = KS > 1 ? ((kend0 - kbeg0 + KS - 1) / KS + CHUNK - 1) / CHUNK * CHUNK : 0;
     const int kbeg = KS > 1 ? kbeg0 + khalf * span : kbeg0;
@@ -163,11 +178,49 @@ gemm_smallm_kernel(const bf16* __restrict__ w, const bf16* __restrict__ x, int M
             for (int t = 0; t < NT; ++t) { mine[4 * t] = acc[t][0]; mine[4 * t + 1] = acc[t][1]; mine[4 * t + 2] = acc[t][2]; mine[4 * t + 3] = acc[t][3]; }
         }
         __syncthreads();
-        if (khalf > 0) return;
+        if (!MERGE && khalf > 0) return;
+        if (khalf == 0)
 #pragma unroll
         for (int t = 0; t < NT; ++t) { acc[t][0] += mine[4 * t]; acc[t][1] += mine[4 * t + 1]; acc[t][2] += mine[4 * t + 2]; acc[t][3] += mine[4 * t + 3]; }
     }
     const bool wa_ok = ra < N, wb_ok = rb < N;        // rows of the matrix (va / vb also say whether this warp had values of k)
+    if constexpr (MERGE) {
+        // value e = token * TILE_ROWS + row of the tile is added by block e / share of the cluster
+        cg::cluster_group cluster = cg::this_cluster();
+        const int slices = gridDim.x, total = M * TILE_ROWS, share = (total + slices - 1) / slices;
+        cluster.barrier_wait();                       // every block of the cluster runs: its shared memory may be written
+        if (khalf == 0) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int tok = t * 8 + 2 * c + (e & 1), row = tile * 16 + g + (e >> 1) * 8;
+                    if (tok >= M) continue;
+                    float v = acc[t][e];
+                    if constexpr (EPI) {
+                        if (slice == 0 && row_block * TILE_ROWS + row < N) v = tw_biased(ep, v, row_block * TILE_ROWS + row);
+                    }
+                    const int at = tok * TILE_ROWS + row, owner = at / share;
+                    *cluster.map_shared_rank(&s_merge[slice * share + (at - owner * share)], owner) = v;
+                }
+        }
+        cluster.sync();                               // (no block touches another's memory behind this)
+        const int whole = slices & ~3;
+        for (int i = threadIdx.x; i < share; i += WARPS * 32) {
+            const int at = slice * share + i, tok = at / TILE_ROWS, row = row_block * TILE_ROWS + at % TILE_ROWS;
+            if (tok >= M || row >= N) continue;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int q = 0; q < MERGE_MOST; ++q) {
+                if (q < whole) sum[q & 3] += s_merge[q * share + i];
+                else if (q < slices) sum[0] += s_merge[q * share + i];
+            }
+            const float v = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            if (out_mode == OUT_BF16) reinterpret_cast<bf16*>(out)[(size_t)tok * out_stride + row] = __float2bfloat16_rn(v);
+            else reinterpret_cast<float*>(out)[(size_t)tok * out_stride + row] = v;
+        }
+        return;
+    }
     // acc[t][0..1]: weight row ra, tokens t*8 + 2c, +1;  acc[t][2..3]: weight row rb
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
@@ -188,7 +241,7 @@ gemm_smallm_kernel(const bf16* __restrict__ w, const bf16* __restrict__ x, int M
             }
             float xa = acc[t][e], xb = acc[t][2 + e];
             if constexpr (EPI) {
-                if (blockIdx.y == 0) {
+                if (slice == 0) {
                     if (wa_ok) xa = tw_biased(ep, xa, ra);
                     if (wb_ok) xb = tw_biased(ep, xb, rb);
                 }
@@ -200,7 +253,7 @@ gemm_smallm_kernel(const bf16* __restrict__ w, const bf16* __restrict__ x, int M
                 if (wb_ok) o[rb] = __float2bfloat16_rn(xb);
             } else {
                 float* o = reinterpret_cast<float*>(out) +
-                           (out_mode == OUT_PARTIAL ? ((size_t)blockIdx.y * M + tok) * out_stride : (size_t)tok * out_stride);
+                           (out_mode == OUT_PARTIAL ? ((size_t)slice * M + tok) * out_stride : (size_t)tok * out_stride);
                 if (wa_ok) o[ra] = xa;
                 if (wb_ok) o[rb] = xb;
             }
@@ -298,7 +351,7 @@ __global__ void reduce_partial_kernel(T* __restrict__ out, const float* __restri
 }  // namespace
 
 // out_mode 0: bf16 [M, out_stride]; 1: fp32 [M, out_stride]; 2: fp32 partial sums [ksplit, M, out_stride]
-// (then kper < K); 3: bf16 [M, out_stride] = act(gate) * up for weights whose rows alternate between eight
+// (then kper < K); with kper < K, at most 8 slices, at most 8 rows and no `act`, 0 and 1 are added up in clusters; 3: bf16 [M, out_stride] = act(gate) * up for weights whose rows alternate between eight
 // gate rows and their eight up rows (N a multiple of 16, no split).  K must be a multiple of 8; kper of 32.
 // `bias` (bf16 [N], in the order of the rows, or null) and `act`: see TwEpilogue.
 TW_EXPORT int tw_gemm_smallm(const void* w, const void* x, int M, int N, int K, int kper, void* out, int out_mode,
@@ -311,7 +364,8 @@ TW_EXPORT int tw_gemm_smallm(const void* w, const void* x, int M, int N, int K, 
         act < TW_ACT_NONE || act > TW_ACT_RELU_SQUARED || (act != TW_ACT_NONE && (out_mode & ~OUT_EARLY_DEPENDENTS) == OUT_PARTIAL))
         return (int)cudaErrorInvalidValue;
     const int ksplit = (K + kper - 1) / kper;
-    if (ksplit > 1 && (out_mode & ~OUT_EARLY_DEPENDENTS) != OUT_PARTIAL) return (int)cudaErrorInvalidValue;
+    const bool merge = ksplit > 1 && (out_mode & ~OUT_EARLY_DEPENDENTS) != OUT_PARTIAL;
+    if (merge && ((out_mode & ~OUT_EARLY_DEPENDENTS) == OUT_GATED || M > 8 || ksplit > MERGE_MOST || act != TW_ACT_NONE)) return (int)cudaErrorInvalidValue;
     dim3 grid((N + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, ksplit);
     const TwEpilogue ep{(const bf16*)bias, act};
     const bf16* wp = (const bf16*)w;
@@ -326,11 +380,17 @@ TW_EXPORT int tw_gemm_smallm(const void* w, const void* x, int M, int N, int K, 
     const bool pair_warps = M <= 8 && (long)grid.x * grid.y * 10 <= (long)sm_count * 32 && kper >= 512;
     const bool epi = bias || act != ((out_mode & ~OUT_EARLY_DEPENDENTS) == OUT_GATED ? TW_ACT_SILU : TW_ACT_NONE);
     if (pair_warps) grid.x = (N + (WARPS / 2) * 16 - 1) / ((WARPS / 2) * 16);
-    auto kernel = pair_warps ? (epi ? gemm_smallm_kernel<1, 2, true> : gemm_smallm_kernel<1, 2, false>)
-                : M <= 8     ? (epi ? gemm_smallm_kernel<1, 1, true> : gemm_smallm_kernel<1, 1, false>)
-                : M <= 16    ? (epi ? gemm_smallm_kernel<2, 1, true> : gemm_smallm_kernel<2, 1, false>)
-                : M <= 32    ? (epi ? gemm_smallm_kernel<4, 1, true> : gemm_smallm_kernel<4, 1, false>)
-                             : (epi ? gemm_smallm_kernel<8, 1, true> : gemm_smallm_kernel<8, 1, false>);
+    if (merge) {
+        auto merging = pair_warps ? (epi ? gemm_smallm_kernel<1, 2, true, true> : gemm_smallm_kernel<1, 2, false, true>)
+                                  : (epi ? gemm_smallm_kernel<1, 1, true, true> : gemm_smallm_kernel<1, 1, false, true>);
+        return tw_launch(merging, dim3(ksplit, grid.x), dim3(WARPS * 32), 0, stream, ksplit, wp, xp, M, N, K, kper, out, out_mode, out_stride, ep,
+                         next_weights, next_bytes);
+    }
+    auto kernel = pair_warps ? (epi ? gemm_smallm_kernel<1, 2, true, false> : gemm_smallm_kernel<1, 2, false, false>)
+                : M <= 8     ? (epi ? gemm_smallm_kernel<1, 1, true, false> : gemm_smallm_kernel<1, 1, false, false>)
+                : M <= 16    ? (epi ? gemm_smallm_kernel<2, 1, true, false> : gemm_smallm_kernel<2, 1, false, false>)
+                : M <= 32    ? (epi ? gemm_smallm_kernel<4, 1, true, false> : gemm_smallm_kernel<4, 1, false, false>)
+                             : (epi ? gemm_smallm_kernel<8, 1, true, false> : gemm_smallm_kernel<8, 1, false, false>);
     tw_launch(kernel, dim3(grid), dim3(WARPS * 32), 0, stream, 1, wp, xp, M, N, K, kper, out, out_mode, out_stride, ep,
               next_weights, next_bytes);
     return TW_LAUNCH_CHECK();

@@ -1329,6 +1329,7 @@ def small_m_supported(x: torch.Tensor, w: torch.Tensor, m: int) -> bool:
 
 
 SMALL_M_ROWS_PER_BLOCK = 64      # weight rows of a block of csrc/gemm_smallm.cu (four warps of 16 rows)
+MERGE_SLICES = 8                 # slices a cluster of its blocks adds
 SMALL_M_BLOCKS_PER_SM = 5        # how many of its blocks an SM holds
 
 
@@ -1368,9 +1369,11 @@ def small_m_split(n: int, k: int, max_slices: int = 12, sms: int | None = None) 
 
 def gemm_small_m(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, kper: int | None = None,
                  silu_mul_pairs: bool = False, early_dependents: bool = False,
-                 prefetch: torch.Tensor | None = None, bias: torch.Tensor | None = None, act: int | None = None) -> None:
+                 prefetch: torch.Tensor | None = None, bias: torch.Tensor | None = None, act: int | None = None,
+                 merge: bool = False) -> None:
     """out[:m] = x[:m] @ w.T for m <= 64 rows.  ``out`` is bf16 or fp32 [>=m, n]; or, when the
-    product is split over k (kper < k), fp32 slices [slices, m, n]; or, with ``silu_mul_pairs``
+    product is split over k (kper < k), fp32 slices [slices, m, n] (with ``merge``, for up to 8 rows and 8 slices, their
+    sum in the order ``SplitSum.dense`` adds them: ``out`` as without a split); or, with ``silu_mul_pairs``
     (rows of w in groups of eight gates and their eight ups), bf16 [>=m, n / 2] = act(gate) * up (silu by default).
     ``bias`` (bf16 [n], in the order of the rows of w) is added first, of a split product to slice 0; without pairs an
     ``act`` is applied to every value (not to slices).
@@ -1391,13 +1394,14 @@ def gemm_small_m(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, kp
         _need(split == 1 and n % 16 == 0 and out.dtype == torch.bfloat16 and out.dim() == 2 and out.stride(1) == 1
               and out.shape[0] >= m and out.shape[1] == n // 2, "gemm_small_m: bad fused silu output")
         mode, stride = 3, out.stride(0)
-    elif split > 1:
+    elif split > 1 and not merge:
         _need(out.dtype == torch.float32 and out.dim() == 3 and out.shape[0] == split and out.shape[1] == m
               and out.shape[2] == n and out.is_contiguous(), "gemm_small_m: split output must be fp32 [slices, m, n]")
         mode, stride = 2, n
     else:
         _need(out.dim() == 2 and out.stride(1) == 1 and out.shape[0] >= m and out.shape[1] == n
               and out.dtype in (torch.bfloat16, torch.float32), "gemm_small_m: bad output")
+        _need(split == 1 or (split <= MERGE_SLICES and m <= 8 and act == ACT_NONE), "gemm_small_m: at most 8 rows and 8 slices are merged, without an activation")
         mode, stride = (0 if out.dtype == torch.bfloat16 else 1), out.stride(0)
     if early_dependents:
         mode |= 16          # the kernel after this one may become resident while this one runs

@@ -95,17 +95,14 @@ def linear(ctx, name: str, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dt
             return out
         # slices that nobody would add: the library's product below, which reduces its own split inside the kernel
     if x.is_cuda and ops.small_m_supported(x, w, m):
-        split, kper = ops.small_m_split(n, w.shape[1], max_slices if allow_split else 12)
+        split, kper = ops.small_m_split(n, w.shape[1], max_slices if allow_split else ops.MERGE_SLICES)
         if split > 1 and allow_split:
             slices = ctx.workspace.get(name + ".slices", (split, m, n), torch.float32)
             ops.gemm_small_m(slices, x, w, m, kper, early_dependents=consumer_early, prefetch=prefetch, bias=bias)
             return SplitSum(slices)
-        if split > 1:
-            slices = ctx.workspace.get(name + ".slices", (split, m, n), torch.float32)
-            ops.gemm_small_m(slices, x, w, m, kper, bias=bias)
-            return SplitSum(slices).dense(dtype, ctx.workspace.get(name, (m, n), dtype))
+        # slices that the caller cannot add are added by clusters of the product's own blocks
         out = ctx.workspace.get(name, (m, n), dtype)
-        ops.gemm_small_m(out, x, w, m, early_dependents=consumer_early, prefetch=prefetch, bias=bias)
+        ops.gemm_small_m(out, x, w, m, kper, merge=split > 1, early_dependents=consumer_early, prefetch=prefetch, bias=bias)
         return out
     if x.is_cuda and bias is None and ops.gemm_narrow_supported(x, w, m):
         # few outputs: the library runs such a product on a handful of blocks (2,048 x 3,584 -> 28: 17 us, 7 here)

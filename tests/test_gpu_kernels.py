@@ -1155,3 +1155,25 @@ def test_product_of_many_rows_and_few_outputs(m, n, k, stride, out_dtype):
     bound = 2 * k * 2.0 ** -24 * size + (want.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
     assert bool(((out[:m, :n].cpu().double() - want).abs() <= bound + 1e-30).all())
     assert bool((out[m:] == 7.0).all()) and bool((out[:, n:] == 7.0).all()), "values behind the result were written"
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k,kper", [(1, 16, 512, 256), (8, 1792, 3584, 448), (5, 40, 1000, 256), (3, 200, 4096, 1024), (8, 33, 2056, 288),
+                                        (7, 5376, 1536, 512), (2, 72, 3592, 512)])
+def test_split_product_merged_in_clusters(m, n, k, kper, out_dtype):
+    """The sums that clusters add are those of the slices, added in the same order: the same bits, with a bias and without,
+    one warp per row tile and two, remainders of rows and k."""
+    from tessweave_engine_b200.csrc import ops as o
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn(m, k, generator=g).to(torch.bfloat16).cuda()
+    w = torch.randn(n, k, generator=g).to(torch.bfloat16).cuda()
+    split = -(-k // kper)
+    for bias in (None, torch.randn(n, generator=g).to(torch.bfloat16).cuda()):
+        slices = torch.empty(split, m, n, device="cuda")
+        o.gemm_small_m(slices, x, w, m, kper, bias=bias)
+        out = torch.full((m + 1, n + 2), 7.0, device="cuda", dtype=out_dtype)
+        o.gemm_small_m(out[:, :n], x, w, m, kper, bias=bias, merge=True)
+        assert torch.equal(out[:m, :n], o.SplitSum(slices).dense(out_dtype))
+        assert bool((out[m:] == 7.0).all()) and bool((out[:, n:] == 7.0).all()), "values behind the result were written"
+    with pytest.raises(RuntimeError, match="merged"):
+        o.gemm_small_m(torch.empty(m, n, device="cuda"), x, w, m, 32, merge=True)
