@@ -1413,22 +1413,23 @@ def gemm_small_m(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, kp
 
 
 NARROW_MOST = 64                 # outputs up to which csrc/gemm_smallm.cu: tw_gemm_narrow takes a product
+NARROW_MIN_ROWS = 1024           # and the rows from which it does: shorter steps of one layer are bound by the host, to which the library's call is cheaper
 
 
-def gemm_narrow_supported(x: torch.Tensor, w: torch.Tensor, m: int) -> bool:
-    """Whether a product of many rows and few outputs goes through ``gemm_narrow``: bfloat16 on 16-byte boundaries."""
-    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and m > SMALL_M_LIMIT and 0 < w.shape[0] <= NARROW_MOST
-            and w.shape[1] % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0 and x.stride(1) == 1
-            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+def gemm_narrow_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``gemm_narrow`` takes these operands: bfloat16 on 16-byte boundaries."""
+    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.is_contiguous()
+            and w.data_ptr() % 16 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
 
 
 def gemm_narrow(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int) -> None:
     """out[:m] = x[:m] @ w.T for few outputs; ``out`` is bf16 or fp32 [>=m, n]."""
     _cuda(out, x, w)
     n, k = w.shape
-    _need(gemm_narrow_supported(x, w, m) and x.shape[0] >= m and x.shape[1] == k, "gemm_narrow: bf16 operands on 16-byte boundaries, at most 64 outputs")
-    _need(out.dim() == 2 and out.stride(1) == 1 and out.shape[0] >= m and out.shape[1] == n and out.dtype in (torch.bfloat16, torch.float32),
-          "gemm_narrow: bad output")
+    # (boundaries and sizes are checked behind the call)
+    _need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[0] >= m and x.shape[1] == k and x.stride(1) == 1
+          and w.is_contiguous(), "gemm_narrow: bf16 operands")
+    _need(out.shape[0] >= m and out.shape[1] == n and out.stride(1) == 1, "gemm_narrow: bad output")
     code = _fn("gemm_smallm", "tw_gemm_narrow")(_ptr(out), c_int(out.stride(0)), _ptr(x), c_int(x.stride(0)), _ptr(w), c_int(m), c_int(n),
                                                 c_int(k), c_int(dtype_code(out.dtype)), _stream())
     _check(code, "gemm_narrow")
@@ -1687,8 +1688,10 @@ def linear_recurrence(mode: int, out: torch.Tensor, den: torch.Tensor | None, q:
 
 RECURRENCE_CHUNK = 64                   # tokens of a chunk (csrc/recurrence_chunks.cu)
 # Where a portion goes through the chunks' three launches.  14 heads of 128 x 128, mLSTM / retention: 26 / 33 us for up to 256
-# tokens (one wave of blocks), token by token 30 / 28 us for 96, 38 / 37 for 128, 71 for 256 (6 heads of 64: 18 and 36 for 128).
-RECURRENCE_CHUNK_MIN_TOKENS = 128
+# tokens (one wave of blocks), token by token 30 / 28 us for 96, 38 / 37 for 128, 71 for 256 (6 heads of 64: 18 and 36 for 128).  A step of one layer that is issued kernel by kernel is bound by the
+# host up to some 300 tokens, and two more launches cost more there than the chunks give: retention of 260 tokens 142 us by
+# tokens, 137 to 166 in chunks, 512 tokens 180 to 200 and 133 to 163; mLSTM of 200 tokens 146 to 174 and 155 to 189, 512 tokens 215 to 231 and 155.
+RECURRENCE_CHUNK_MIN_TOKENS = 320
 # Beside such a portion, how many rows a request needs to go with it (a chunk more hardly counts; token by token it would be a
 # launch of its own, 0.25 us a token: the delta rule over portions of 777, 1,024 and 201, 195 + 67 us with the last by tokens).
 RECURRENCE_CHUNK_MIN_ROWS = 32
@@ -1738,8 +1741,9 @@ def recurrence_chunks(mode: int, out: torch.Tensor, den: torch.Tensor | None, q:
     _check(code, "recurrence_chunks")
 
 
-# The delta rule's three launches take 45 us for 128 tokens, 51 for 256 (14 heads of 128 x 128); token by token 36 and 67.
-DELTA_CHUNK_MIN_TOKENS = 256
+# The delta rule's three launches take 45 us for 128 tokens, 51 for 256 (14 heads of 128 x 128); token by token 36 and 67; a
+# whole layer issued kernel by kernel 188 to 201 us by tokens and 190 to 218 in chunks for 260 tokens, 239 to 262 and 197 to 225 for 512.
+DELTA_CHUNK_MIN_TOKENS = 384
 
 
 def delta_chunks_supported(q: torch.Tensor, k: torch.Tensor, key_dim: int, value_dim: int, channel_decay: bool) -> bool:

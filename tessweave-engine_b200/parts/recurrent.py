@@ -102,13 +102,18 @@ class MatrixStateMixer(Mixer):
         common = (cache.state, ctx.positions, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.n_seqs, self.n_heads, self.key_dim,
                   self.value_dim)
         below, longest = 0, ctx.max_q_len
-        delta = self.rule == ops.RECURRENCE_DELTA and ops.delta_chunks_supported(q, k, self.key_dim, self.value_dim,
-                                                                                 rule_args["channel_decay"])
-        if delta or ops.recurrence_chunks_supported(self.rule, q.dtype, self.key_dim, self.value_dim, rule_args.get("rot_dims", 0)):
-            # a long portion, and with it all but the shortest, in chunks; the others token by token.  The chunks' scratch is asked for in captured steps too, so
-            # that the workspace has its final size after the largest one
+        # (short steps are bound by the host: one comparison and on)
+        long_enough = ctx.fixed_shape or longest >= ops.RECURRENCE_CHUNK_MIN_TOKENS
+        delta = long_enough and self.rule == ops.RECURRENCE_DELTA and ops.delta_chunks_supported(q, k, self.key_dim, self.value_dim,
+                                                                                                 rule_args["channel_decay"])
+        if long_enough and (delta or ops.recurrence_chunks_supported(self.rule, q.dtype, self.key_dim, self.value_dim,
+                                                                     rule_args.get("rot_dims", 0))):
+            # A long portion, and with it all but the shortest, in chunks; the others token by token.  A captured step knows no
+            # row counts and goes token by token, but asks for the chunks' scratch as well, so that the workspace has its
+            # final size after the largest one.
             enough = ops.DELTA_CHUNK_MIN_TOKENS if delta else ops.RECURRENCE_CHUNK_MIN_TOKENS
-            chunks = ops.recurrence_chunk_count(n, ctx.n_seqs)
+            longest_known = 0 if ctx.fixed_shape else max(ctx.host_q_len, default=0)
+            chunks = ops.recurrence_chunk_count(n, ctx.n_seqs) if ctx.fixed_shape or longest_known >= enough else 0
             if chunks > 0 and delta:
                 scratch = ws.get("recurrence.delta_chunks", (chunks, ops.delta_chunk_floats(self.n_heads, rule_args["qk_group"], self.key_dim,
                                                                                             self.value_dim)), torch.float32)
@@ -116,7 +121,6 @@ class MatrixStateMixer(Mixer):
                 scratch = (ws.get("recurrence.chunk_state", (chunks, self.n_heads * self.key_dim * (self.value_dim + 1)), torch.float32),
                            ws.get("recurrence.chunk_gate", (chunks, self.n_heads, 2), torch.float64),
                            ws.get("recurrence.chunk_max", (chunks, self.n_heads), torch.float32))
-            longest_known = 0 if ctx.fixed_shape else max(ctx.host_q_len, default=0)     # (a captured step knows no row counts)
             if longest_known >= enough:
                 if delta:
                     ops.delta_chunks(raw, q, k, v, cache.state, *common[2:], longest_known, scratch, write_state,
