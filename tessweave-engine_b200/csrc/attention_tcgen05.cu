@@ -12,8 +12,17 @@
 //                      for the whole walk
 // The two row tiles alternate, so the tensor cores work on one while the softmax warps work on
 // the other.  Keys and values travel by TMA (cp.async.bulk.tensor.2d, no multicast), one box
-// per page and 64 columns of d, into the swizzled layout the MMAs read; a warp of its own
+// per page and 64 columns of d, into the swizzled layout the MMAs read; a warp each
 // issues them.  Another warp issues every MMA.
+//
+// What bounds it: a key tile takes 3,600 cycles of which the tensor pipe is busy for 2,048; a tile's chain is its softmax
+// (1,650: 1,024 for its exponentials), its products (1,250) and the hand-overs between the two, and the longest blocks of a
+// prompt run through 16 such tiles one behind the other.  So what shortens the chain counts: exponentials that do not wait
+// for the tile's own maximum, one wait and no commits beside the products', copies from two warps, query rows whose loads
+// hang on no condition (8,500 -> 2,500 cycles), results written by whole rows (5,300 -> 2,400), masks off the path that all
+// tiles take (the first tile of a block fetches its instructions: 6,600 -> 3,000).  us before and after: 2,048 tokens of
+// 28 heads of 128 50.4 and 42.4, of 14 heads of 64 39.3 and 37.2; 777 + 300 + 201 tokens of 12 heads behind 0, 512 and 1,030
+// keys 30.9 and 27.0; 400 tokens of 28 heads 21.5 and 16.5; 301 + 182 of 40 heads 25.2 and 23.4.
 //
 // O is only rescaled when a row's maximum grows by more than 2^8 (the sums carry the same
 // stale maximum, so the quotient is exact); rows of values beyond the request's last key are
@@ -57,7 +66,12 @@ constexpr int Q_BYTES = NQ * KB * BLK;
 constexpr int K_STAGE_BYTES = KB * BLK, V_STAGE_BYTES = VB * BLK;
 constexpr int SMEM_TILES = Q_BYTES + KV_STAGES * (K_STAGE_BYTES + V_STAGE_BYTES);
 constexpr int SMEM = SMEM_TILES + 1024 /* alignment slack */ + 256 /* barriers */;
-constexpr int THREADS = 320;                  // warp 0: TMA, warp 1: MMA, warps 2-5 / 6-9: softmax of tile 0 / 1
+constexpr int THREADS = 384;                  // warps 0-3 / 4-7: softmax of tile 0 / 1, warps 8 / 9: copies of K / V, warps 10 / 11: MMAs of tile 0 / 1
+constexpr int K_WARP = 8, V_WARP = 9, MMA_WARP = 10;
+// A softmax thread holds a row of 128 scores; the others need few registers.  256 x 200 + 128 x 104 = 384 x 168, which the
+// block is launched with.
+constexpr int SOFTMAX_REGS = 200, OTHER_REGS = 104, LAUNCH_REGS = 168;
+static_assert(256 * SOFTMAX_REGS + 128 * OTHER_REGS <= THREADS * LAUNCH_REGS, "registers of the block");
 constexpr int TMEM_COLS = 512;                // S of both tiles (2 x 128 columns; P over its first 64), O of both tiles (2 x DV)
 constexpr int O_COL = 256;
 constexpr float RESCALE_THRESHOLD = 8.f;      // log2 units
@@ -66,7 +80,7 @@ constexpr float RESCALE_THRESHOLD = 8.f;      // log2 units
 // -DTW_TRACE: block (0, 0, 0) records clock64() at the hand-over points of its roles, for a
 // timeline of one block (tw_attn_tc5_trace_ptr gives the buffer).  Off in the product.
 #ifdef TW_TRACE
-constexpr int TRACE_SLOTS = 12, TRACE_TILES = 80, TRACE_ROLES = 10;     // a role = a warp
+constexpr int TRACE_SLOTS = 12, TRACE_TILES = 80, TRACE_ROLES = 12;     // a role: a softmax warp, 8 both MMA warps, 9 and 10 the copies, 11 the block
 __device__ long long g_trace[TRACE_ROLES * TRACE_TILES * TRACE_SLOTS];
 #define TW_TRACE_AT(role, tile, slot)                                                              \
     do {                                                                                           \
@@ -87,8 +101,8 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                         int* status) {
     extern __shared__ unsigned char smem_raw[];
     TW_TIMELINE_SCOPE(TW_K_ATTN_PREFILL);
-    if (threadIdx.x == 0) TW_TRACE_AT(0, 0, 5);
     tw_grid_wait();
+    if (threadIdx.x == 0) TW_TRACE_AT(11, 0, 5);
     TW_TIMELINE_MARK();
     // Blocks start in the order of blockIdx.x, and a block's work grows with the position of its rows: x counts
     // (row tile, key/value head) with the head fastest and the last row tile first, so that the longest blocks of
@@ -118,35 +132,36 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     unsigned char* q_s = tiles;                                      // [NQ][KB][128 rows][128 B]
     unsigned char* k_s = q_s + Q_BYTES;                              // [KV_STAGES][KB][128 keys][128 B]
     unsigned char* v_s = k_s + KV_STAGES * K_STAGE_BYTES;            // [KV_STAGES][VB][128 keys][128 B]
-    uint64_t* k_full = reinterpret_cast<uint64_t*>(tiles + SMEM_TILES);
-    uint64_t* k_empty = k_full + KV_STAGES;
-    uint64_t* v_full = k_empty + KV_STAGES;
-    uint64_t* v_empty = v_full + KV_STAGES;
-    uint64_t* s_full = v_empty + KV_STAGES;                          // S of tile X is complete
-    uint64_t* p_full = s_full + NQ;                                  // P of tile X is written, S read, O rescaled
-    uint64_t* o_done = p_full + NQ;                                  // the P V products of tile X so far have retired
-    uint64_t* v_fixed = o_done + NQ;                                 // value rows past the last key are zeroed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_fixed + 1);
+    uint64_t* k_first = reinterpret_cast<uint64_t*>(tiles + SMEM_TILES);   // K of the first tile has landed
+    uint64_t* v_last = k_first + 1;                                  // V of the last tile has (where rows of it are zeroed)
+    // Of tile i's products P V and the next tile's S: P of query tile 0 is written, V of tile i and K of tile i + 1 have landed.
+    // One barrier for all three, since each wait costs the thread that issues the MMAs some 170 cycles even if it is over.
+    uint64_t* ready = v_last + 1;                                    // [stage]
+    uint64_t* p_full = ready + KV_STAGES;                            // P of query tile 1 is written, S read, O rescaled
+    // [query tile][stage]: S of the tile is complete, its P V products have retired.  The producers take them as the sign that
+    // a stage is free as well (commits to barriers of their own took 200 cycles each).
+    uint64_t* s_full = p_full + 1;
+    uint64_t* o_done = s_full + NQ * KV_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + NQ * KV_STAGES);
     volatile int* aborted = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < KV_STAGES; ++i) {
-            mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
-            mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-        }
-        for (int x = 0; x < NQ; ++x) { mbar_init(&s_full[x], 1); mbar_init(&p_full[x], BM / 32); mbar_init(&o_done[x], 1); }
-        mbar_init(v_fixed, 1);
+        mbar_init(k_first, 1);
+        mbar_init(v_last, 1);
+        mbar_init(p_full, BM / 32);
+        for (int i = 0; i < KV_STAGES; ++i) mbar_init(&ready[i], BM / 32 + 2);
+        for (int i = 0; i < NQ * KV_STAGES; ++i) { mbar_init(&s_full[i], 1); mbar_init(&o_done[i], 1); }
         *aborted = 0;
         mbar_fence_init();
     }
-    // The producer's work for key tile i: one TMA box per page (and 64 columns of d) for the keys, then for the
-    // values; lane b owns box b of a tile.  False if a wait ran out.
+    // A producer's work for key tile i: one TMA box per page and 64 columns of d; lane b owns box b of the tile (one lane
+    // that issues them all takes 160 cycles a copy, eight lanes 100).  Keys and values have a warp each: the 32 copies of
+    // both take one warp as long as the products of the tile take.  False if a wait ran out.
     const int box_rows = min(page_size, BN);
     const int boxes = BN / box_rows;
-    auto issue_tile = [&](int i) -> bool {
+    auto issue_tile = [&](int i, const CUtensorMap* map, unsigned char* ring, int stage_bytes, int blocks, uint64_t* full, uint64_t* freed) -> bool {
         const int st = i % KV_STAGES;
-        const uint32_t parity = (i / KV_STAGES) & 1;
         int row_coord = -1;
         if (lane < boxes) {
             const int key0 = (j_begin + i) * BN + lane * box_rows;
@@ -162,68 +177,61 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         const uint32_t box_bytes = (uint32_t)__popc(__ballot_sync(0xffffffffu, row_coord >= 0)) * box_rows * 128;
         int ok = 1;
         if (lane == 0) {
-            ok = (!*aborted && mbar_wait(&k_empty[st], parity ^ 1, status)) ? 1 : 0;
-            if (ok) mbar_expect_tx(&k_full[st], box_bytes * KB); else *aborted = 1;
+            ok = (!*aborted && (i < KV_STAGES || mbar_wait(&freed[st], (i / KV_STAGES - 1) & 1, status))) ? 1 : 0;
+            if (ok) mbar_expect_tx(full, box_bytes * blocks); else *aborted = 1;
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) return false;
-        if (lane == 0) TW_TRACE_AT(0, i, 0);
+        if (lane == 0) TW_TRACE_AT(ring == k_s ? 9 : 10, i, 0);
         if (row_coord >= 0) {
-#pragma unroll
-            for (int kb = 0; kb < KB; ++kb)
-                tma_load_2d(k_s + st * K_STAGE_BYTES + kb * BLK + lane * box_rows * 128, &map_k, &k_full[st], kb * 64, row_coord);
-        }
-        if (lane == 0) {
-            ok = (!*aborted && mbar_wait(&v_empty[st], parity ^ 1, status)) ? 1 : 0;
-            if (ok) mbar_expect_tx(&v_full[st], box_bytes * VB); else *aborted = 1;
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) {                                   // K of this tile is in flight: let it land
-            if (lane == 0) mbar_wait(&k_full[st], parity, status);
-            return false;
-        }
-        if (lane == 0) TW_TRACE_AT(1, i, 2);
-        if (row_coord >= 0) {
-#pragma unroll
-            for (int vb = 0; vb < VB; ++vb)
-                tma_load_2d(v_s + st * V_STAGE_BYTES + vb * BLK + lane * box_rows * 128, &map_v, &v_full[st], vb * 64, row_coord);
+            for (int b = 0; b < blocks; ++b)
+                tma_load_2d(ring + st * stage_bytes + b * BLK + lane * box_rows * 128, map, full, b * 64, row_coord);
         }
         return true;
     };
-    if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
-    // The first key and value tiles need nothing of what follows: the producer warp (whose first thread has just
-    // set up the barriers) asks for them now, and the other warps bring the query rows in meanwhile.
+    // the barrier that tells of tile i's keys, of its values
+    auto k_full = [&](int i) { return i == 0 ? k_first : &ready[(i - 1) % KV_STAGES]; };
+    auto v_full = [&](int i) { return i == ntiles - 1 && tail_rows ? v_last : &ready[i % KV_STAGES]; };
+    auto issue_k = [&](int i) { return issue_tile(i, &map_k, k_s, K_STAGE_BYTES, KB, k_full(i), s_full + (nq - 1) * KV_STAGES); };
+    auto issue_v = [&](int i) { return issue_tile(i, &map_v, v_s, V_STAGE_BYTES, VB, v_full(i), o_done + (nq - 1) * KV_STAGES); };
+    // The first key and value tiles need nothing of what follows: their producers ask for them as soon as the barriers
+    // stand, and the other warps bring the query rows in meanwhile.
+    __syncthreads();
+    if (warp == MMA_WARP) tmem_alloc(tmem_slot, TMEM_COLS);
     int issued = 0;
-    if (warp == 0) {
-        __syncwarp();
-        while (issued < ntiles && issued < KV_STAGES && issue_tile(issued)) ++issued;
+    if (warp == K_WARP) {
+        while (issued < ntiles && issued < KV_STAGES && issue_k(issued)) ++issued;
+    } else if (warp == V_WARP) {
+        while (issued < ntiles && issued < KV_STAGES && issue_v(issued)) ++issued;
     }
 
     // the block's query rows into shared memory, in the swizzled K-major layout (rows beyond the portion are zero).
     // All of a thread's loads are issued before the first store: one round trip to L2, not thirteen in a row
     // (which was 9 of the 13 us a block spent outside its key tiles).
-    {
+    if (warp != K_WARP && warp != V_WARP) {
         constexpr int Q_ITEMS = NQ * BM * (D / 8);
-        constexpr int Q_THREADS = THREADS - 32;                          // every warp but the producer
+        constexpr int Q_THREADS = THREADS - 64;                          // every warp but the producers
         constexpr int Q_PER_THREAD = (Q_ITEMS + Q_THREADS - 1) / Q_THREADS;
+        constexpr int STEP = Q_THREADS / (D / 8);                        // rows between two of a thread's loads: its columns stay
+        static_assert(Q_THREADS % (D / 8) == 0, "a thread keeps its columns");
+        const int first = (warp < K_WARP ? warp : warp - 2) * 32 + lane;
+        const int c = first % (D / 8), rr0 = first / (D / 8), step_t = STEP / G, step_h = STEP - step_t * G;
+        int t = (row0 + rr0) / G, hg = row0 + rr0 - t * G;
+        const bf16* src = q + (size_t)n0 * q_stride + (size_t)kvh * G * D + c * 8;
         uint4 vals[Q_PER_THREAD];
 #pragma unroll
         for (int j = 0; j < Q_PER_THREAD; ++j) {
-            const int i = (int)threadIdx.x - 32 + j * Q_THREADS;
-            const int rr = i / (D / 8), c = i - rr * (D / 8);
-            const int r = row0 + rr;
-            vals[j] = make_uint4(0u, 0u, 0u, 0u);
-            if (warp != 0 && i < Q_ITEMS && r < rows_total) {
-                const int t = r / G;
-                vals[j] = *reinterpret_cast<const uint4*>(q + (size_t)(n0 + t) * q_stride + (size_t)(kvh * G + (r - t * G)) * D + c * 8);
-            }
+            // no load hangs on a condition (a row behind the last reads the last token's): all of them are under way at once
+            vals[j] = *reinterpret_cast<const uint4*>(src + (size_t)min(t, q_len - 1) * q_stride + hg * D);
+            t += step_t; hg += step_h;
+            if (hg >= G) { hg -= G; ++t; }
         }
 #pragma unroll
         for (int j = 0; j < Q_PER_THREAD; ++j) {
-            const int i = (int)threadIdx.x - 32 + j * Q_THREADS;
-            if (warp != 0 && i < Q_ITEMS) {
-                const int rr = i / (D / 8), c = i - rr * (D / 8);
+            const int rr = rr0 + j * STEP;
+            if (rr < NQ * BM) {
                 const int x = rr / BM, rt = rr - x * BM;
+                if (row0 + rr >= rows_total) vals[j] = make_uint4(0u, 0u, 0u, 0u);
                 *reinterpret_cast<uint4*>(q_s + (x * KB + (c >> 3)) * BLK + rt * 128 + (((c & 7) ^ (rt & 7)) << 4)) = vals[j];
             }
         }
@@ -233,17 +241,29 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (threadIdx.x == 0) TW_TRACE_AT(0, 0, 6);
+    if (threadIdx.x == 0) TW_TRACE_AT(11, 0, 6);
 
-    if (warp == 0) {
-        // ---- producer: the remaining tiles, each as soon as its stage is free
-        while (issued < ntiles && !*aborted && issue_tile(issued)) ++issued;
-        if (tail_rows && issued == ntiles) {
+    if (warp >= K_WARP) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGS));
+        if (warp < MMA_WARP) {
+        // ---- producers: the remaining tiles, each as soon as its stage is free
+        if (warp == K_WARP) {
+            while (issued < ntiles && !*aborted && issue_k(issued)) ++issued;
+        } else {
+            while (issued < ntiles && !*aborted && issue_v(issued)) ++issued;
+        }
+        if (warp == K_WARP && issued == ntiles && ntiles > 0 && lane == 0) {
+            // no keys behind the last tile's: its barrier gets the arrival alone, once the phase before is over there
+            if (ntiles < KV_STAGES || mbar_wait(&s_full[(nq - 1) * KV_STAGES + ntiles % KV_STAGES], (ntiles / KV_STAGES - 1) & 1, status))
+                mbar_arrive(&ready[(ntiles - 1) % KV_STAGES]);
+            else *aborted = 1;
+        }
+        if (warp == V_WARP && tail_rows && issued == ntiles) {
             // The last tile reaches past the request's last key.  What its value rows hold there (the rest
             // of a page, or whatever the stage held before) must not reach a product, since 0 x NaN is NaN:
             // zero them once the copies have landed, then tell the MMA thread.
             const int last = ntiles - 1;
-            if (mbar_wait(&v_full[last % KV_STAGES], (last / KV_STAGES) & 1, status)) {
+            if (mbar_wait(v_last, 0, status)) {
                 unsigned char* vt = v_s + (last % KV_STAGES) * V_STAGE_BYTES;
                 for (int idx = lane; idx < tail_rows * VB * 8; idx += 32) {
                     const int r = BN - tail_rows + idx / (VB * 8), rest = idx % (VB * 8);
@@ -251,7 +271,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(v_fixed);
+                if (lane == 0) mbar_arrive(&ready[last % KV_STAGES]);
             } else {
                 *aborted = 1;
             }
@@ -259,15 +279,16 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         if (*aborted && lane == 0) {
             // wait (bounded) for the copies already in flight, so that none lands after the block has gone
             for (int i = max(0, issued - KV_STAGES); i < issued; ++i) {
-                mbar_wait(&k_full[i % KV_STAGES], (i / KV_STAGES) & 1, status);
-                mbar_wait(&v_full[i % KV_STAGES], (i / KV_STAGES) & 1, status);
+                if (warp == K_WARP) mbar_wait(k_full(i), i == 0 ? 0 : ((i - 1) / KV_STAGES) & 1, status);
+                else mbar_wait(v_full(i), i == ntiles - 1 && tail_rows ? 0 : (i / KV_STAGES) & 1, status);
             }
         }
-    } else if (warp == 1) {
+        } else {
         // ---- tensor cores: lane 0 issues every MMA of the block.  The tensor pipe runs dry as soon as
-        // this thread does anything else, so whatever a group of MMAs needs beside P (V of the tile, K of
-        // the next one) is waited for before P, and the groups follow one another without a break.
-        if (lane == 0 && ntiles > 0) {
+        // this thread does anything else, so it waits once for all that a group of MMAs needs.  (A thread for each
+        // query tile was no faster: left alone the tiles fall into step, both in their softmax at a time and both at the
+        // tensor pipe at a time, 5,080 cycles a key tile; taking turns, 3,700, they are as fast as with one thread.)
+        if (warp == MMA_WARP && lane == 0 && ntiles > 0) {
             const uint32_t idesc_s = instr_desc(BN), idesc_o = instr_desc(DV, true);
             // Descriptors are built once; per MMA only a constant is added to the address field (a thread
             // that computes a descriptor from scratch before each MMA issues them slower than they execute).
@@ -281,7 +302,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                     for (int k = 0; k < 4; ++k)
                         umma_bf16(tmem_base + x * BN, qd + (uint64_t)(kb * (BLK >> 4) + k * 2), kd + (uint64_t)(kb * (BLK >> 4) + k * 2),
                                   idesc_s, (kb > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&s_full[x]);
+                umma_commit(&s_full[x * KV_STAGES + i % KV_STAGES]);
             };
             auto issue_o = [&](int x, int i) {
                 const uint64_t vd = v_desc + (uint64_t)((i % KV_STAGES) * (V_STAGE_BYTES >> 4));
@@ -289,45 +310,34 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 for (int k = 0; k < BN / 16; ++k)
                     umma_bf16_ts(tmem_base + O_COL + x * DV, tmem_base + x * BN + k * 8, vd + (uint64_t)(k * (2048 >> 4)),
                                  idesc_o, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&o_done[x]);
+                umma_commit(&o_done[x * KV_STAGES + i % KV_STAGES]);
             };
-            bool ok = mbar_wait(&k_full[0], 0, status);
+            bool ok = mbar_wait(k_first, 0, status);
             if (ok) {
                 tc_fence_after();
                 for (int x = 0; x < nq; ++x) issue_s(x, 0);
-                umma_commit(&k_empty[0]);
             }
             for (int i = 0; ok && i < ntiles; ++i) {
-                const int st = i % KV_STAGES;
-                TW_TRACE_AT(1, i, 10);
-                ok = mbar_wait(&v_full[st], (i / KV_STAGES) & 1, status);
-                TW_TRACE_AT(1, i, 2);
-                if (ok && i == ntiles - 1 && tail_rows) ok = mbar_wait(v_fixed, 0, status);
-                if (ok && i + 1 < ntiles) ok = mbar_wait(&k_full[(i + 1) % KV_STAGES], ((i + 1) / KV_STAGES) & 1, status);
-                TW_TRACE_AT(1, i, 4);
                 for (int x = 0; ok && x < nq; ++x) {
-                    TW_TRACE_AT(1, i, x * 6 + 0);
-                    ok = mbar_wait(&p_full[x], i & 1, status);
+                    TW_TRACE_AT(8, i, x * 6 + 1);
+                    ok = x == 0 ? mbar_wait(&ready[i % KV_STAGES], (i / KV_STAGES) & 1, status) : mbar_wait(p_full, i & 1, status);
                     if (!ok) break;
-                    TW_TRACE_AT(1, i, x * 6 + 1);
+                    TW_TRACE_AT(8, i, x * 6 + 2);
                     tc_fence_after();
                     issue_o(x, i);
-                    TW_TRACE_AT(1, i, x * 6 + 3);
                     if (i + 1 < ntiles) issue_s(x, i + 1);
-                    TW_TRACE_AT(1, i, x * 6 + 5);
+                    TW_TRACE_AT(8, i, x * 6 + 4);
                 }
-                if (ok) {
-                    umma_commit(&v_empty[st]);
-                    if (i + 1 < ntiles) umma_commit(&k_empty[(i + 1) % KV_STAGES]);
-                }
-                TW_TRACE_AT(1, i, 8);
             }
             if (!ok) *aborted = 1;
         }
         __syncwarp();
-    } else if ((warp - 2) / 4 < nq) {
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGS));
+        if (warp / 4 < nq) {
         // ---- softmax: thread = row rt of tile x = TMEM lane rt
-        const int x = (warp - 2) / 4;
+        const int x = warp / 4;
         const int quarter = warp & 3;                        // the TMEM lanes this warp may touch
         const int rt = quarter * 32 + lane;
         const int r = row0 + x * BM + rt;
@@ -342,56 +352,89 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         for (int i = 0; i < ntiles; ++i) {
             const int kbase = (j_begin + i) * BN;
             if (lane == 0) TW_TRACE_AT(warp, i, 0);
-            ok = !*aborted && mbar_wait(&s_full[x], i & 1, status);
+            ok = !*aborted && mbar_wait(&s_full[x * KV_STAGES + i % KV_STAGES], (i / KV_STAGES) & 1, status);
             if (!ok) break;
             if (lane == 0) TW_TRACE_AT(warp, i, 1);
             tc_fence_after();
-            uint32_t v[BN];
+            uint32_t v[2][32], packed[BN / 2];
+            if (!__all_sync(0xffffffffu, kbase + BN - 1 <= pos && kbase >= lo)) {
+                // keys that the row does not see: -infinity in tensor memory, so that what follows, which every tile runs
+                // through, need not ask (its instructions are fetched anew by every block's first tile)
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 32) {
+                    tmem_ld32_nowait(s_addr + c, v[0]);
+                    tmem_wait_ld_of(v[0]);
 #pragma unroll
-            for (int c = 0; c < BN; c += 32) tmem_ld32_nowait(s_addr + c, v + c);
-            tmem_wait_ld();
-            if (lane == 0) TW_TRACE_AT(warp, i, 2);
-            const bool all_visible = kbase + BN - 1 <= pos && kbase >= lo;
-            if (!__all_sync(0xffffffffu, all_visible)) {
-#pragma unroll
-                for (int c = 0; c < BN; ++c) {
-                    const int key = kbase + c;
-                    if (key > pos || key < lo) v[c] = __float_as_uint(NEG_INF);
+                    for (int e = 0; e < 32; ++e)
+                        if ((unsigned)(kbase + c + e - lo) > (unsigned)(pos - lo)) v[0][e] = __float_as_uint(NEG_INF);
+                    tmem_st32_nowait(s_addr + c, v[0]);
                 }
+                tmem_wait_st();
             }
             // four independent chains of three-input maxima
-            float mx[4] = {NEG_INF, NEG_INF, NEG_INF, NEG_INF};
+            auto maxima = [&](float (&mx)[4], const uint32_t (&v)[32]) {
 #pragma unroll
-            for (int c = 0; c < BN; c += 8) {
+                for (int c = 0; c < 32; c += 8)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mx[k] = max3(mx[k], __uint_as_float(v[c + 2 * k]), __uint_as_float(v[c + 2 * k + 1]));
+                    for (int k = 0; k < 4; ++k) mx[k] = max3(mx[k], __uint_as_float(v[c + 2 * k]), __uint_as_float(v[c + 2 * k + 1]));
+            };
+            auto largest = [&](const float (&mx)[4]) {      // scale > 0: the maximum commutes with it
+                return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2e;
+            };
+            if (i == 0) {
+                float mx[4] = {NEG_INF, NEG_INF, NEG_INF, NEG_INF};
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 32) {
+                    tmem_ld32_nowait(s_addr + c, v[0]);
+                    tmem_wait_ld_of(v[0]);
+                    maxima(mx, v[0]);
+                }
+                m_used = largest(mx);
             }
-            const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2e;   // scale > 0: the maximum commutes with it
-            const bool rescale = mt > m_used + RESCALE_THRESHOLD;     // also the first finite maximum (m_used = -inf)
-            float factor = 1.f;
-            if (rescale) {
-                factor = m_used == NEG_INF ? 0.f : ex2(m_used - mt);
-                m_used = mt;
-            }
-            const float neg_mu = m_used == NEG_INF ? 0.f : -m_used;
-            // p = 2^(s c - m) two at a time (packed fp32 multiply-add and add), four independent sums of pairs
-            float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            // The exponentials are taken against the maximum as it was, 32 scores at a time while the next 32 come in, and the
+            // tile's own maximum is found beside them: waiting for it first took 400 of the 1,830 cycles between S and P.  Only
+            // where a row's maximum has grown by more than the threshold (the first tiles of a request) are they taken again.
+            bool rescale = false;
+            float factor = 1.f, sum;
+            while (true) {
+                float mx[4] = {NEG_INF, NEG_INF, NEG_INF, NEG_INF};
+                const float neg_mu = m_used == NEG_INF ? 0.f : -m_used;
+                // p = 2^(s c - m) two at a time (packed fp32 multiply-add and add), four independent sums of pairs
+                float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+                tmem_ld32_nowait(s_addr, v[0]);
 #pragma unroll
-            for (int c = 0; c < BN; c += 8) {
+                for (int c = 0; c < BN; c += 32) {
+                    uint32_t (&w)[32] = v[(c >> 5) & 1];
+                    tmem_wait_ld_of(w);
+                    if (c + 32 < BN) tmem_ld32_nowait(s_addr + c + 32, v[((c >> 5) & 1) ^ 1]);
+                    maxima(mx, w);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float2 e = fma2(__uint_as_float(v[c + 2 * k]), __uint_as_float(v[c + 2 * k + 1]), scale_log2e, neg_mu);
-                    e.x = ex2(e.x);
-                    e.y = ex2(e.y);
-                    acc[k] = add2(acc[k], e);
-                    v[(c >> 1) + k] = pack_bf16(e.x, e.y);
+                    for (int e8 = 0; e8 < 32; e8 += 8) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            float2 e = fma2(__uint_as_float(w[e8 + 2 * k]), __uint_as_float(w[e8 + 2 * k + 1]), scale_log2e, neg_mu);
+                            e.x = ex2(e.x);
+                            e.y = ex2(e.y);
+                            acc[k] = add2(acc[k], e);
+                            packed[((c + e8) >> 1) + k] = pack_bf16(e.x, e.y);
+                        }
+                    }
+                }
+                sum = ((acc[0].x + acc[0].y) + (acc[1].x + acc[1].y)) + ((acc[2].x + acc[2].y) + (acc[3].x + acc[3].y));
+                const float mt = largest(mx);
+                const bool grown = mt > m_used + RESCALE_THRESHOLD;
+                if (!__any_sync(0xffffffffu, grown)) break;
+                rescale = true;
+                if (grown) {
+                    factor = m_used == NEG_INF ? 0.f : ex2(m_used - mt);
+                    m_used = mt;
                 }
             }
-            const float sum = ((acc[0].x + acc[0].y) + (acc[1].x + acc[1].y)) + ((acc[2].x + acc[2].y) + (acc[3].x + acc[3].y));
+            if (lane == 0) TW_TRACE_AT(warp, i, 2);
             l = l * factor + sum;
-            if (i > 0 && __any_sync(0xffffffffu, rescale)) {
+            if (i > 0 && rescale) {
                 // P V of the tile before has retired (it was issued before the S just read): O is complete up to it
-                ok = mbar_wait(&o_done[x], (i - 1) & 1, status);
+                ok = mbar_wait(&o_done[x * KV_STAGES + (i - 1) % KV_STAGES], ((i - 1) / KV_STAGES) & 1, status);
                 if (!ok) break;
                 tc_fence_after();
                 {
@@ -409,15 +452,15 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             }
             if (lane == 0) TW_TRACE_AT(warp, i, 3);
             // P over the first 64 columns of S: the whole row of S is in registers by now
-            tmem_st32_nowait(s_addr, v);
-            tmem_st32_nowait(s_addr + 32, v + 32);
+            tmem_st32_nowait(s_addr, packed);
+            tmem_st32_nowait(s_addr + 32, packed + 32);
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[x]);      // one arrival per warp: 128 arrivals on one barrier take 450 cycles
+            if (lane == 0) mbar_arrive(x == 0 ? &ready[i % KV_STAGES] : p_full);      // one arrival per warp: 128 arrivals on one barrier take 450 cycles
             if (lane == 0) TW_TRACE_AT(warp, i, 4);
         }
-        if (ok && ntiles > 0) ok = mbar_wait(&o_done[x], (ntiles - 1) & 1, status);
+        if (ok && ntiles > 0) ok = mbar_wait(&o_done[x * KV_STAGES + (ntiles - 1) % KV_STAGES], ((ntiles - 1) / KV_STAGES) & 1, status);
         if (lane == 0) TW_TRACE_AT(warp, TRACE_TILES - 1, 0);
         if (!ok) {
             *aborted = 1;
@@ -425,13 +468,16 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             tc_fence_after();
             float inv = l > 0.f ? 1.f / l : 0.f;
             if (gate && valid) inv *= __ldg(gate + (size_t)(n0 + t) * Hq + kvh * G + (r - t * G));
-            bf16* orow = out + (size_t)(n0 + t) * out_stride + (size_t)(kvh * G + (r - t * G)) * DV;
+            const long long at = (long long)(n0 + t) * out_stride + (long long)(kvh * G + (r - t * G)) * DV;
+            if constexpr (DV <= D) {
+                // through the tile's query rows, which nobody reads any more, so that a warp writes whole rows: with a row per
+                // thread, 16 bytes at a time, the stores of a block took 5,000 cycles
+                unsigned char* stage = q_s + x * KB * BLK + quarter * 32 * (DV * 2);
 #pragma unroll
-            for (int c = 0; c < DV; c += 32) {
-                uint32_t o[32];
-                tmem_ld32_nowait(o_addr + c, o);
-                tmem_wait_ld();
-                if (valid) {
+                for (int c = 0; c < DV; c += 32) {
+                    uint32_t o[32];
+                    tmem_ld32_nowait(o_addr + c, o);
+                    tmem_wait_ld();
 #pragma unroll
                     for (int k = 0; k < 32; k += 8) {
                         uint4 w;
@@ -439,18 +485,49 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                         w.y = pack_bf16(__uint_as_float(o[k + 2]) * inv, __uint_as_float(o[k + 3]) * inv);
                         w.z = pack_bf16(__uint_as_float(o[k + 4]) * inv, __uint_as_float(o[k + 5]) * inv);
                         w.w = pack_bf16(__uint_as_float(o[k + 6]) * inv, __uint_as_float(o[k + 7]) * inv);
-                        *reinterpret_cast<uint4*>(orow + c + k) = w;
+                        *reinterpret_cast<uint4*>(stage + lane * (DV * 2) + ((((c + k) >> 3) ^ (lane & (DV / 8 < 8 ? DV / 8 - 1 : 7))) << 4)) = w;
+                    }
+                }
+                __syncwarp();
+                constexpr int LANES = DV / 8, ROWS = 32 / LANES;         // lanes a row, rows a store
+                const uint32_t live = __ballot_sync(0xffffffffu, valid);
+                const int c = lane % LANES;
+#pragma unroll
+                for (int j = 0; j < 32 / ROWS; ++j) {
+                    const int row = j * ROWS + lane / LANES;
+                    const long long dst = __shfl_sync(0xffffffffu, at, row);
+                    const uint4 w = *reinterpret_cast<const uint4*>(stage + row * (DV * 2) + ((c ^ (row & (LANES < 8 ? LANES - 1 : 7))) << 4));
+                    if ((live >> row) & 1) *reinterpret_cast<uint4*>(out + dst + c * 8) = w;
+                }
+            } else {
+                bf16* orow = out + at;
+#pragma unroll
+                for (int c = 0; c < DV; c += 32) {
+                    uint32_t o[32];
+                    tmem_ld32_nowait(o_addr + c, o);
+                    tmem_wait_ld();
+                    if (valid) {
+#pragma unroll
+                        for (int k = 0; k < 32; k += 8) {
+                            uint4 w;
+                            w.x = pack_bf16(__uint_as_float(o[k]) * inv, __uint_as_float(o[k + 1]) * inv);
+                            w.y = pack_bf16(__uint_as_float(o[k + 2]) * inv, __uint_as_float(o[k + 3]) * inv);
+                            w.z = pack_bf16(__uint_as_float(o[k + 4]) * inv, __uint_as_float(o[k + 5]) * inv);
+                            w.w = pack_bf16(__uint_as_float(o[k + 6]) * inv, __uint_as_float(o[k + 7]) * inv);
+                            *reinterpret_cast<uint4*>(orow + c + k) = w;
+                        }
                     }
                 }
             }
         }
     }
-    if (lane == 0) TW_TRACE_AT(warp, TRACE_TILES - 1, 1);
+    }
+    if (lane == 0 && warp < K_WARP) TW_TRACE_AT(warp, TRACE_TILES - 1, 1);
     __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
-    if (threadIdx.x == 32) TW_TRACE_AT(0, 0, 7);
+    if (warp == MMA_WARP) tmem_dealloc(tmem_base, TMEM_COLS);
+    if (threadIdx.x == 0) TW_TRACE_AT(11, 0, 7);
 }
 
 }  // namespace
@@ -488,6 +565,10 @@ TW_EXPORT int tw_attn_prefill_tc5(void* out, int out_stride, const void* q, int 
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return (int)e;
+        cudaFuncAttributes built;
+        e = cudaFuncGetAttributes(&built, attn_prefill_tc5_kernel);
+        if (e != cudaSuccess) return (int)e;
+        if (built.numRegs != LAUNCH_REGS) return (int)cudaErrorInvalidConfiguration;       // the warps would wait for registers that are not there
         attr_set = true;
     }
     const int box_rows = page_size < BN ? page_size : BN;

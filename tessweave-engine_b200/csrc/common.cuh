@@ -222,7 +222,7 @@ static inline int tw_allow_shared() {
 // (the kernel itself waits where it must), optionally as clusters of `cluster_x` blocks.
 //
 // Plain launches of TW_PDL_THREADS threads and more are launched that way too: between two such kernels the GPU stands idle for
-// 0.9 to 1.2 us less (one layer over 2,000 tokens, us without and with: gated delta 327.8 and 314.3, mLSTM 196.3 and 187.3, 7b
+// 0.9 to 1.2 us less (one layer over 2,000 tokens, us without and with: gated delta 327.8 and 313.6, mLSTM 196.3 and 190.7, 7b
 // attention 160.8 and 157.7, 32-bit attention 320.5 and 316.5).  Smaller ones belong to steps that the host bounds, and there
 // the attribute costs 1 to 2 % of a step.  READS_AHEAD: the kernel reads some of its step's inputs before it waits, which is sound
 // where they were there before the graph's first kernel, so it waits for everything before it on plain launches.
