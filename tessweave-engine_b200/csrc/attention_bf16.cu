@@ -969,11 +969,11 @@ static int decode_launch(void* out, int out_stride, const void* q, int q_stride,
     float* partial_ml = scratch ? scratch + (size_t)n_seqs * Hq * nsplit * DV : nullptr;
     dim3 grid(nsplit * htiles, Hkv, n_seqs);
     if (nsplit > 1 && !(flags & 1) && decode_cluster_ok(nsplit))
-        return tw_launch(attn_decode_kernel<true, false>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, nsplit,
+        return tw_launch<TW_READS_AHEAD>(attn_decode_kernel<true, false>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, nsplit,
             (bf16*)out, out_stride, (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table,
             table_stride, (const bf16*)k_cache, (const bf16*)v_cache, Hq, Hkv, page_size, num_pages, window,
             scale * 1.4426950408889634f, nsplit, partial_o, partial_ml, counters, status, FusedQkv{}, terms);
-    tw_launch(attn_decode_kernel<false, false>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, 1, 
+    tw_launch<TW_READS_AHEAD>(attn_decode_kernel<false, false>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, 1, 
         (bf16*)out, out_stride, (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table,
         table_stride, (const bf16*)k_cache, (const bf16*)v_cache, Hq, Hkv, page_size, num_pages, window,
         scale * 1.4426950408889634f, nsplit, partial_o, partial_ml, counters, status, FusedQkv{}, terms);
@@ -1035,11 +1035,11 @@ TW_EXPORT int tw_attn_decode_fused(void* out, int out_stride, const float* parti
     fq.next_weights = next_weights; fq.next_bytes = next_weights ? next_bytes : 0;
     dim3 grid(nsplit * htiles, Hkv, n_seqs);
     if (nsplit > 1 && !(flags & 1) && decode_cluster_ok(nsplit))
-        return tw_launch(attn_decode_kernel<true, true>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, nsplit,
+        return tw_launch<TW_READS_AHEAD>(attn_decode_kernel<true, true>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, nsplit,
             (bf16*)out, out_stride, (const bf16*)nullptr, 0, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table,
             table_stride, (const bf16*)k_cache, (const bf16*)v_cache, Hq, Hkv, page_size, num_pages, window,
             scale * 1.4426950408889634f, nsplit, partial_o, partial_ml, counters, status, fq, ScoreTerms{});
-    tw_launch(attn_decode_kernel<false, true>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, 1,
+    tw_launch<TW_READS_AHEAD>(attn_decode_kernel<false, true>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, 1,
         (bf16*)out, out_stride, (const bf16*)nullptr, 0, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table,
         table_stride, (const bf16*)k_cache, (const bf16*)v_cache, Hq, Hkv, page_size, num_pages, window,
         scale * 1.4426950408889634f, nsplit, partial_o, partial_ml, counters, status, fq, ScoreTerms{});
@@ -1139,7 +1139,7 @@ TW_EXPORT int tw_attn_decode_static(void* out, int out_stride, const void* q, in
     e = cudaMemsetAsync(counters, 0, counter_bytes, stream);
     if (e != cudaSuccess) return (int)e;
     dim3 grid(nsplit * htiles, Hkv, n_seqs);
-    tw_launch(attn_decode_kernel<false, false>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, 1, 
+    tw_launch<TW_READS_AHEAD>(attn_decode_kernel<false, false>, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, 1, 
         (bf16*)out, out_stride, (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table,
         table_stride, (const bf16*)k_cache, (const bf16*)v_cache, Hq, Hkv, page_size, num_pages, window,
         scale * 1.4426950408889634f, nsplit, partial_o, partial_ml, counters, status, FusedQkv{}, ScoreTerms{});

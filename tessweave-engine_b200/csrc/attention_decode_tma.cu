@@ -32,6 +32,7 @@
 #include "tcgen05.cuh"
 #include "attention_common.cuh"
 #include <cooperative_groups.h>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -144,7 +145,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                        int num_pages, int window, float scale_log2e, int nsplit, int nstages,
                        float* __restrict__ partial_o, float* __restrict__ partial_ml, int* __restrict__ counters,
                        int* status, const FusedQkv fq, const float* __restrict__ gate, const float* __restrict__ sink,
-                       const int shared_kv) {
+                       const int shared_kv, const int beside) {
     static_assert(!FUSED || SAME_DIMS, "the fused form packs q, k and v as heads of one size");
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[MAX_STAGES];
@@ -165,8 +166,12 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     TW_TIMELINE_SCOPE(TW_K_ATTN_DECODE);
     // The request arrays and the block table are written before the step's first kernel starts, not by the
     // kernel before this one: they are read before the wait for that kernel.
+    // `beside`: the kernel before this one is the prompts' attention of the same step.  It lets this kernel start once it has
+    // seen all that it reads itself (the rows of q and the cache), and neither reads what the other writes: only one block
+    // waits for it, at its end, so that what follows comes after both.
+    const bool waits_last = beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
     if (seq_q_len[s] != 1) {
-        tw_grid_wait();             // a block never finishes before the kernel before this one has
+        if (!beside || waits_last) tw_grid_wait();             // a block never finishes before the kernel before this one has
         return;
     }
     if constexpr (CLUSTER) cg::this_cluster().barrier_arrive();      // (waited for before the first store into a neighbour's memory)
@@ -219,7 +224,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // position, and the copies wait for it.
         const bool values = warp > CWARPS;
         const int stage_bytes = shared_kv ? KB * BLKB : STAGE_BYTES;     // (values that are the keys: the keys' copy serves as both)
-        if (!(FUSED && fq.k_cache)) tw_grid_wait();
+        if (!(FUSED && fq.k_cache) && !beside) tw_grid_wait();
         TW_TTRACE(9);
         const CUtensorMap* map = values ? &map_v : &map_k;
         const int boxes = values && shared_kv ? 0 : TILE / box_rows, box_bytes = (values ? VB : KB) * box_rows * 128;
@@ -269,12 +274,12 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 tw_prefetch_l2_share(fq.next_weights, fq.next_bytes);
             }
         }
-        if (FUSED && fq.k_cache) tw_grid_wait();
+        if ((FUSED && fq.k_cache) || waits_last) tw_grid_wait();
         return;
     } else {
         // ---- consumers
         if (warp == 0) TW_TTRACE(0);
-        tw_grid_wait();
+        if (!beside) tw_grid_wait();
         if (warp == 0) TW_TTRACE(1);
         TW_TIMELINE_MARK();
         constexpr int half = D / 2;
@@ -722,7 +727,8 @@ TW_EXPORT int tw_attn_decode_tma_supported(int page_size) {
 // `scratch` and `counters` as for tw_attn_decode; they are used when the slices do not fit a cluster.
 // `gate` (fp32 [rows][Hq] or null): head h's output of a row is multiplied by its entry.  `sink` (fp32 [Hq] or null, with `q`
 // only): exp(sink[h]) joins head h's denominator.  v_cache may be k_cache (with `q` only): a position's value is its key, which
-// is copied once and read as both.
+// is copied once and read as both.  `flags`: 1 merges slices in scratch memory, 2 (with `q` only) runs beside the kernel launched
+// before, which must be the prompts' attention of the same step (tw_attn_prefill_tc5 with skip_single).
 TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q_stride, const float* partial, int nslices,
                                  long long slice_stride, const void* dense, int dense_stride, const float* bias,
                                  const float* inv_freq, int write_cache, const int* seq_q_start, const int* seq_q_len,
@@ -776,13 +782,18 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
     const size_t smem = smem_bytes(nstages, shared_kv);
     const float scale_log2e = scale * 1.4426950408889634f;
     const bool cluster = nsplit > 1 && !(flags & 1) && cluster_fits(nsplit, nstages, shared_kv);
+    const bool beside = (flags & 2) != 0;
+    if (beside && fused) return (int)cudaErrorInvalidValue;
 #define TW_DECODE_TMA_LAUNCH(CL, FU)                                                                                   \
     do {                                                                                                               \
         if (int e = prepare<CL, FU>()) return e;                                                                       \
-        return tw_launch(attn_decode_tma_kernel<CL, FU>, grid, dim3(THREADS), smem, stream, CL ? nsplit : 1, mk, mv,    \
-                         (bf16*)out, out_stride, (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, \
-                         block_table, table_stride, Hq, Hkv, page_size, num_pages, window, scale_log2e, nsplit, nstages, \
-                         partial_o, partial_ml, counters, status, fq, gate, sink, (int)shared_kv);                         \
+        auto launch = [&](auto how) {                                                                                  \
+            return tw_launch<decltype(how)::value>(attn_decode_tma_kernel<CL, FU>, grid, dim3(THREADS), smem, stream, CL ? nsplit : 1, mk, mv,    \
+                             (bf16*)out, out_stride, (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, \
+                             block_table, table_stride, Hq, Hkv, page_size, num_pages, window, scale_log2e, nsplit, nstages, \
+                             partial_o, partial_ml, counters, status, fq, gate, sink, (int)shared_kv, (int)beside);    \
+        };                                                                                                             \
+        return beside ? launch(std::integral_constant<int, TW_OVERLAPS>()) : launch(std::integral_constant<int, TW_READS_AHEAD>()); \
     } while (0)
     if constexpr (SAME_DIMS) {
         if (cluster && fused) TW_DECODE_TMA_LAUNCH(true, SAME_DIMS);

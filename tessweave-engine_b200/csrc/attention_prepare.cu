@@ -234,7 +234,7 @@ int launch(void* q_out, const void* rows, int row_stride, const float* partial, 
     if (parts > room) parts = room;
     if (parts < 1) parts = 1;
     auto kernel = partial ? attention_prepare_kernel<T, VEC, true> : attention_prepare_kernel<T, VEC, false>;
-    return tw_launch<true>(kernel, dim3(n_tokens, parts), dim3(256), (size_t)(a.rot_dims / 2) * sizeof(float2),
+    return tw_launch<TW_READS_AHEAD>(kernel, dim3(n_tokens, parts), dim3(256), (size_t)(a.rot_dims / 2) * sizeof(float2),
                      stream, 1, (T*)q_out, (const T*)rows, row_stride, partial, nsplit, (size_t)split_stride, (T*)first,
                      (T*)k_cache, (T*)v_cache, a);
 }

@@ -98,22 +98,53 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                         const int* __restrict__ seq_kv_len, const int* __restrict__ seq_slot,
                         const int* __restrict__ block_table, int table_stride, int Hq, int Hkv, int page_size,
                         int num_pages, int window, float scale_log2e, int skip_single, const float* __restrict__ gate,
-                        int* status) {
+                        int* status, int n_seqs) {
     extern __shared__ unsigned char smem_raw[];
     TW_TIMELINE_SCOPE(TW_K_ATTN_PREFILL);
     tw_grid_wait();
+    // The decode attention of the same step writes other rows: it may run beside this kernel, on the SMs that have no block of it.
+    if (skip_single) tw_launch_dependents_now();
     if (threadIdx.x == 0) TW_TRACE_AT(11, 0, 5);
     TW_TIMELINE_MARK();
     // Blocks start in the order of blockIdx.x, and a block's work grows with the position of its rows: x counts
     // (row tile, key/value head) with the head fastest and the last row tile first, so that the longest blocks of
     // all heads start first and the short ones fill the gaps (with the head as blockIdx.y, the long blocks of
     // the last heads started late: 78 us against 58 us for 2,048 tokens).
-    const int s = blockIdx.y, kvh = (int)blockIdx.x % Hkv, xt = (int)blockIdx.x / Hkv;
-    const int q_len = seq_q_len[s];
-    if (q_len <= 0 || (skip_single && q_len == 1)) return;
-    const int G = Hq / Hkv;
+    const int G = Hq / Hkv, kvh = (int)blockIdx.x % Hkv;
+    int s = blockIdx.y, xt = (int)blockIdx.x / Hkv, q_len = 0;
+    auto served = [&](int len) { return len <= 0 || (skip_single && len == 1) ? 0 : len; };
+    auto tiles_of = [&](int len) { return (len * G + NQ * BM - 1) / (NQ * BM); };
+    if (n_seqs > 0) {
+        // the grid holds the row tiles of all requests one behind the other: which request's is this one?  (With a grid of
+        // every request's largest number of tiles, 1,440 of 1,520 blocks of a step of 2 prompts and 30 single tokens had
+        // nothing to do, one per SM at a time, and the decode attention could not start beside this kernel for 18 us.)
+        const int lane = threadIdx.x & 31;
+        int before = 0;
+        s = -1;
+        for (int r0 = 0; r0 < n_seqs && s < 0; r0 += 32) {
+            const int len = r0 + lane < n_seqs ? served(seq_q_len[r0 + lane]) : 0, mine = tiles_of(len);
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
+            }
+            const uint32_t beyond = __ballot_sync(0xffffffffu, xt < before + upto);
+            if (beyond) {
+                const int at = __ffs(beyond) - 1;
+                s = r0 + at;
+                q_len = __shfl_sync(0xffffffffu, len, at);
+                xt -= before + __shfl_sync(0xffffffffu, upto - mine, at);
+            } else {
+                before += __shfl_sync(0xffffffffu, upto, 31);
+            }
+        }
+        if (s < 0) return;
+    } else {
+        q_len = served(seq_q_len[s]);
+    }
     const int rows_total = q_len * G;
-    const int mtiles = (rows_total + NQ * BM - 1) / (NQ * BM);
+    const int mtiles = tiles_of(q_len);
     if (xt >= mtiles) return;
     const int row0 = (mtiles - 1 - xt) * (NQ * BM);                  // the rows with the most keys first
     const int kv_len = seq_kv_len[s];
@@ -550,12 +581,13 @@ TW_EXPORT int tw_attn_prefill_tc5_supported(int page_size) {
 
 // Attention for the requests of the batch that bring several tokens (with skip_single, requests
 // with one token are left to the decode kernel).  q [tokens, Hq * D] and out [tokens, Hq * D] are
-// bf16 with 16-byte aligned rows; the cache is [pages, Hkv, page_size, D] bf16 (values and out: heads of DV).
+// bf16 with 16-byte aligned rows; the cache is [pages, Hkv, page_size, D] bf16 (values and out: heads of DV).  `row_tiles`: the sum of
+// ceil(rows x Hq / Hkv / 256) over the requests that are served, where the caller knows it, else 0.
 TW_EXPORT int tw_attn_prefill_tc5(void* out, int out_stride, const void* q, int q_stride, const int* seq_q_start,
                                   const int* seq_q_len, const int* seq_kv_len, const int* seq_slot,
                                   const int* block_table, int table_stride, const void* k_cache, const void* v_cache,
                                   int n_seqs, int max_q_len, int Hq, int Hkv, int page_size, int num_pages, int window,
-                                  float scale, int skip_single, const float* gate, int* status, cudaStream_t stream) {
+                                  float scale, int skip_single, const float* gate, int row_tiles, int* status, cudaStream_t stream) {
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
     if (Hkv <= 0 || Hq % Hkv || !tw_attn_prefill_tc5_supported(page_size) || scale <= 0.f) return (int)cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(q) & 15) || (out_stride & 7) || (q_stride & 7) ||
@@ -578,8 +610,11 @@ TW_EXPORT int tw_attn_prefill_tc5(void* out, int out_stride, const void* q, int 
     if (int e = get_map(k_cache, rows, D, box_rows, &mk)) return e;
     if (int e = get_map(v_cache, rows, DV, box_rows, &mv)) return e;
     const int G = Hq / Hkv;
-    dim3 grid(((max_q_len * G + NQ * BM - 1) / (NQ * BM)) * Hkv, n_seqs);
+    const bool counted = row_tiles > 0;
+    const long long blocks = (long long)(counted ? row_tiles : (max_q_len * G + NQ * BM - 1) / (NQ * BM)) * Hkv;
+    if (blocks > 0x7fffffffll || (!counted && n_seqs > 65535)) return (int)cudaErrorInvalidValue;
+    dim3 grid((unsigned)blocks, counted ? 1 : n_seqs);
     return tw_launch(attn_prefill_tc5_kernel, grid, dim3(THREADS), (size_t)SMEM, stream, 1, mk, mv, (bf16*)out, out_stride,
                      (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table, table_stride,
-                     Hq, Hkv, page_size, num_pages, window, scale * 1.4426950408889634f, skip_single, gate, status);
+                     Hq, Hkv, page_size, num_pages, window, scale * 1.4426950408889634f, skip_single, gate, status, counted ? n_seqs : 0);
 }

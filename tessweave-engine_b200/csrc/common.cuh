@@ -224,10 +224,12 @@ static inline int tw_allow_shared() {
 // Plain launches of TW_PDL_THREADS threads and more are launched that way too: between two such kernels the GPU stands idle for
 // 0.9 to 1.2 us less (one layer over 2,000 tokens, us without and with: gated delta 327.8 and 313.6, mLSTM 196.3 and 190.7, 7b
 // attention 160.8 and 157.7, 32-bit attention 320.5 and 316.5).  Smaller ones belong to steps that the host bounds, and there
-// the attribute costs 1 to 2 % of a step.  READS_AHEAD: the kernel reads some of its step's inputs before it waits, which is sound
-// where they were there before the graph's first kernel, so it waits for everything before it on plain launches.
+// the attribute costs 1 to 2 % of a step.  TW_READS_AHEAD: the kernel reads some of its step's inputs before it waits, which is
+// sound where they were there before the graph's first kernel, so it waits for everything before it on plain launches.
+// TW_OVERLAPS: with the attribute whatever its size.
 #define TW_PDL_THREADS (148 * 128)
-template <bool READS_AHEAD = false, typename... KArgs, typename... Args>
+enum : int { TW_BY_SIZE = 0, TW_READS_AHEAD = 1, TW_OVERLAPS = 2 };
+template <int HOW = TW_BY_SIZE, typename... KArgs, typename... Args>
 static inline int tw_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                             int cluster_x, Args... args) {
 #ifndef __CUDA_ARCH__
@@ -238,7 +240,7 @@ static inline int tw_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
     int n = 0;
-    const bool large = !READS_AHEAD && (unsigned long long)grid.x * grid.y * grid.z * block.x >= TW_PDL_THREADS;
+    const bool large = HOW == TW_OVERLAPS || (HOW == TW_BY_SIZE && (unsigned long long)grid.x * grid.y * grid.z * block.x >= TW_PDL_THREADS);
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (tw_pdl_enabled() && (large || (cudaStreamIsCapturing(stream, &capturing) == cudaSuccess &&
                                        capturing == cudaStreamCaptureStatusActive))) {

@@ -357,7 +357,7 @@ static int launch_add_rmsnorm(T* out, float* resid, const T* delta, const float*
                               size_t split_stride, const float* weight, float eps, int n_rows, int hidden,
                               const int* rows, float dscale, TwNormPair<T> pair, cudaStream_t stream) {
     if (n_rows <= 64 && hidden >= 1024 && hidden <= TW_NORM_CLUSTER * TW_NORM_CTHREADS * TW_NORM_CMAXV) {
-        return tw_launch<true>(add_rmsnorm_cluster_kernel<T, PAIR>, dim3(n_rows * TW_NORM_CLUSTER), dim3(TW_NORM_CTHREADS), 0, stream,
+        return tw_launch<TW_READS_AHEAD>(add_rmsnorm_cluster_kernel<T, PAIR>, dim3(n_rows * TW_NORM_CLUSTER), dim3(TW_NORM_CTHREADS), 0, stream,
                          TW_NORM_CLUSTER, out, resid, delta, partial, nsplit, split_stride, weight, eps, hidden, rows, dscale, pair);
     }
     if (!partial && !(PAIR && pair.partial) && (hidden & 3) == 0 && hidden <= 4 * 256 * TW_NORM_V4) {

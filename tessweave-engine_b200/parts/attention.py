@@ -57,31 +57,39 @@ class PagedSoftmaxMixer(Mixer):
         """bfloat16: flash attention for requests with several tokens, split-KV attention for
         requests with one; both read the same flat batch and skip the other's requests."""
         singles = ctx.decode_only or ctx.fixed_shape or any(n == 1 for n in ctx.host_q_len)
+        beside = False
         if not ctx.decode_only and not self._prefill_own(ctx, out, q, cache, gate, singles):
             # long portions: tcgen05 kernel (TMA, accumulators in tensor memory); short ones, and the shapes it
             # does not take, stay on the mma.sync kernel, which starts faster
-            prefill = ops.attention_prefill
+            prefill, more = ops.attention_prefill, self._terms()
             if (not self.score_terms and self.scale > 0
                     and ops.prefer_tcgen05_attention(self.runtime.dtype, self.head_dim, cache.k_pages.shape[2], ctx.max_q_len, self.v_dim)):
-                prefill = ops.attention_prefill_tcgen05
+                prefill, beside = ops.attention_prefill_tcgen05, True
+                more["host_q_len"] = None if ctx.fixed_shape else ctx.host_q_len or None
+                if singles:     # (the scratch may be cleared when it is made: not between two kernels that run side by side)
+                    self._decode_buffers(ctx)
             prefill(out, q, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.seq_slot,
                                   cache.block_table, cache.k_pages, cache.v_pages, ctx.n_seqs, ctx.max_q_len,
                                   self.n_heads, self.n_kv_heads, self.head_dim, self.reach, self.scale, singles, ctx.status,
-                                  gate=gate, **self._terms())
+                                  gate=gate, **more)
         if singles:
-            self._decode(ctx, out, q, cache, gate=gate)
+            self._decode(ctx, out, q, cache, gate=gate, beside_prompts=beside)
+
+    def _decode_buffers(self, ctx: StepContext) -> tuple[torch.Tensor, torch.Tensor]:
+        group = self.n_heads // self.n_kv_heads
+        return (ctx.workspace.get("attn.decode_scratch", (ops.decode_scratch_floats(self.n_heads, self.v_dim),), torch.float32),
+                ctx.workspace.get("attn.decode_counters", (ops.decode_counter_ints(ctx.n_seqs, self.n_kv_heads, group),), torch.int32,
+                                  zero=True))
 
     def _decode(self, ctx: StepContext, out: torch.Tensor, q: torch.Tensor | None, cache: PagedView, fused=None,
-                gate: torch.Tensor | None = None) -> None:
+                gate: torch.Tensor | None = None, beside_prompts: bool = False) -> None:
         """Split-KV attention for the requests that bring one token; with ``fused`` = (product, rotation table,
-        write_cache) the kernel makes q, k and v of the new token from the product itself.  Head sizes that are
+        write_cache) the kernel makes q, k and v of the new token from the product itself; ``beside_prompts``: the step's
+        prompts' attention on tcgen05 has just been launched, and the kernel runs beside it (it is bound by memory, the
+        other by its longest blocks' chains).  Head sizes that are
         multiples of 64 take the kernel that is fed by TMA, the others the one that loads keys through registers."""
-        group = self.n_heads // self.n_kv_heads
         tma, nsplit, _ = self._decode_launch(ctx, cache)
-        scratch = ctx.workspace.get("attn.decode_scratch", (ops.decode_scratch_floats(self.n_heads, self.v_dim),),
-                                    torch.float32)
-        counters = ctx.workspace.get(
-            "attn.decode_counters", (ops.decode_counter_ints(ctx.n_seqs, self.n_kv_heads, group),), torch.int32, zero=True)
+        scratch, counters = self._decode_buffers(ctx)
         window = self.reach
         product, table, write_cache = fused if fused is not None else (None, None, False)
         prefetch = self._prefetch_plan(ctx)[0] if fused is not None else None
@@ -90,7 +98,7 @@ class PagedSoftmaxMixer(Mixer):
                                      ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.seq_slot, cache.block_table,
                                      cache.k_pages, cache.v_pages, ctx.n_seqs, self.n_heads, self.n_kv_heads, self.head_dim,
                                      window, self.scale, nsplit, scratch, counters, ctx.status, prefetch=prefetch, gate=gate,
-                                     sink=self.sink if self.score_terms else None)
+                                     sink=self.sink if self.score_terms else None, beside_prompts=beside_prompts)
         elif fused is not None:
             ops.attention_decode_fused(out, product, self.b_qkv, table, write_cache, ctx.seq_q_start, ctx.seq_q_len,
                                        ctx.seq_kv_len, ctx.seq_slot, cache.block_table, cache.k_pages, cache.v_pages,
