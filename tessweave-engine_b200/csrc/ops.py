@@ -1486,6 +1486,35 @@ def gemm_narrow(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int) -> 
 
 
 # ---------------------------------------------------------------------------
+# 32-bit matrix products of many rows, as three bf16 terms per number
+# ---------------------------------------------------------------------------
+def prefer_gemm_fp32(m: int, n: int, k: int) -> bool:
+    """Whether a float32 product of this size runs on the tensor cores, every number as three bf16 terms.  A round of its blocks
+    takes some 10 us and 1.65 us for every 64 values of k however few rows and outputs there are; the library's time grows with
+    both.  us here and there, by k x n: 512 rows 896 x 1,152 37 and 33, 777 rows 33 and 45; 256 rows 1,536 x 2,048 51 and 49, 512
+    rows 51 and 72; 128 rows 3,584 x 4,608 118 and 115, 256 rows 117 and 154; 64 rows 896 x 9,728 37 and 45, 256 rows 63 and 115;
+    256 rows 4,864 x 896 137 and 127, 777 rows 135 and 202."""
+    return m >= 128 and m * n >= 640 * 1024 and k >= 256
+
+
+def gemm_fp32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``gemm_fp32`` takes these operands: float32 on 16-byte boundaries, k a multiple of 4."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and w.shape[1] % 4 == 0 and w.stride(1) == 1 and w.stride(0) % 4 == 0
+            and w.data_ptr() % 16 == 0 and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0)
+
+
+def gemm_fp32(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, status: torch.Tensor) -> None:
+    """out[:m] = x[:m] @ w.T, all fp32, on the tensor cores without giving up bits: every number enters as three bf16 terms."""
+    _cuda(out, x, w, status)
+    n, k = w.shape
+    _need(gemm_fp32_supported(x, w) and x.shape[0] >= m and x.shape[1] == k, "gemm_fp32: fp32 operands on 16-byte boundaries")
+    _need(out.dtype == torch.float32 and out.shape[0] >= m and out.shape[1] == n and out.stride(1) == 1, "gemm_fp32: bad output")
+    code = _fn("gemm_fp32_tcgen05", "tw_gemm_fp32")(_ptr(out), c_int(out.stride(0)), _ptr(x), c_int(x.stride(0)), _ptr(w), c_int(w.stride(0)),
+                                                    c_int(m), c_int(n), c_int(k), _ptr(status), _stream())
+    _check(code, "gemm_fp32")
+
+
+# ---------------------------------------------------------------------------
 # matrix products of prompt steps on pairs of thread blocks
 # ---------------------------------------------------------------------------
 PAIR_MIN_M = 768           # rows from which the fused gate/up product may run on block pairs

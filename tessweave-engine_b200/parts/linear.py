@@ -3,7 +3,9 @@
 The reference's engine runs its projections through a library (nn.Linear, i.e.
 cuBLAS: flow_engine/model.py:39-43,71-73,108); so does this function where no
 hand-written kernel takes the shape.  float32 products run in true fp32: TF32 and
-every other reduced-precision matrix mode is switched off before the first call.
+every other reduced-precision matrix mode is switched off before the first call
+(large ones run on the tensor cores with every number as three bf16 terms, whose
+errors are a fifth of the library's: csrc/gemm_fp32_tcgen05.cu).
 bfloat16 products accumulate in fp32 (no reduced-precision split-K sums).
 """
 from __future__ import annotations
@@ -69,7 +71,7 @@ def linear(ctx, name: str, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dt
     Steps with up to 8 rows (decode) in bfloat16 go through the weight-streaming kernel of
     csrc/gemm_smallm.cu; products of 9 to 64 rows with a large matrix (down, logits) through the persistent
     tcgen05 kernel of csrc/gemm_tcgen05_stream.cu; 1,024 rows and more with few fp32 outputs, in no eights, through
-    csrc/gemm_smallm.cu: tw_gemm_narrow.
+    csrc/gemm_smallm.cu: tw_gemm_narrow; large float32 products through csrc/gemm_fp32_tcgen05.cu.
     When the matrix has too few rows to fill the GPU these kernels split k and, if the caller can take it
     (``allow_split``), the fp32 slices are returned as a ``SplitSum`` for the consuming kernel
     to add.  Everything else is a library product.  ``consumer_early``: the weight-streaming kernel lets the kernel
@@ -108,6 +110,11 @@ def linear(ctx, name: str, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dt
         # few fp32 outputs, a mixer's gates and step sizes
         out = ctx.workspace.get(name, (m, n), dtype)
         ops.gemm_narrow(out, x, w, m)
+        return out
+    if (x.dtype == torch.float32 and dtype == torch.float32 and bias is None and x.is_cuda and ops.prefer_gemm_fp32(m, n, w.shape[1])
+            and ops.gemm_fp32_supported(x, w)):
+        out = ctx.workspace.get(name, (m, n), dtype)
+        ops.gemm_fp32(out, x, w, m, ctx.status)
         return out
     return matmul_nt(ctx.workspace.get(name, (m, n), dtype), x, w, bias)
 
