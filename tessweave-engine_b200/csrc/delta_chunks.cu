@@ -15,7 +15,7 @@
 // What bounded the rule token by token is its chain (0.23 us a token, whatever the GPU could do beside it); now it is the
 // walk's, two products and two barriers a chunk, and the reads of W and K (96 KB a chunk and block) from L2.
 // 14 heads of 128 x 128 over 2,048 tokens: 482 us token by token, 207 in chunks (65 + 95 + 47 for the launches); portions of
-// 777, 1,024 and 201 tokens: 378 and 198; 14 heads of 64 x 64: 413 and 113.  Of the walk's 95 us a third goes when nothing
+// 777, 1,024 and 201 tokens: 378 and 186; 14 heads of 64 x 64: 413 and 113.  Of the walk's 95 us a third goes when nothing
 // is copied and a third when few products are made; six sums for the small products instead of one change nothing.
 // Against 64 bits: outputs 1.8e-7 (token by token 6.5e-7), state 2.0e-7 (6.1e-7).
 //
@@ -234,110 +234,136 @@ __global__ void __launch_bounds__(THREADS, 2) delta_solve_kernel(DcArgs a) {
     }
 }
 
-// ---- (2) the walk.  A block owns 16 values of a head's state, transposed (rows are values): warp w the key channels 16 w ...
+// ---- (2) the walk.  A block owns 16 VT values of a head's state, transposed (rows are values): warp w the key channels 16 w ...
 // of it, in its accumulators.  S and the weighted U go through shared memory as three terms, which all warps read as the row
-// operand; W and K of the next chunk are copied while this one is computed.
-template <int DV>
+// operand; the W and K of the chunks stand in a ring of four places, or of three where the state takes more room, the next ones on
+// their way while one is used.
+//
+// What bounds it is the chain of a chunk (its products, on mma.sync, and two barriers), 3.0 us with 16 values and 4.6 with 32, so 32 are
+// taken where 16 would give more blocks than the GPU has SMs (one fits an SM): portions of 777, 1,024 and 201 tokens, 14 heads of
+// 128 x 128, 336 blocks in two rounds and 168 whose longest start first, 87 us and 75.
+template <int DV, int VT>
 __global__ void __launch_bounds__(THREADS, 1) delta_walk_kernel(DcArgs a) {
     constexpr int NT = DK / 64;                             // tiles of 8 key channels per warp
-    constexpr int TERMS = 3 * L * RS, SS = DK + 8;
+    constexpr int TERMS = 3 * L * RS, SS = DK + 8, V = 16 * VT, PLACES = VT == 1 ? 4 : 3;
     extern __shared__ __align__(16) unsigned char dc_smem[];
-    bf16* ring = reinterpret_cast<bf16*>(dc_smem);          // [2][W, K][3][L][RS]
-    bf16* st = ring + 4 * TERMS;                            // [3][16][SS] the state
-    bf16* ut = st + 3 * 16 * SS;                            // [3][16][MS] the weighted U
+    bf16* ring = reinterpret_cast<bf16*>(dc_smem);          // [PLACES][3][L][RS]: W of chunk 0, K of chunk 0, W of chunk 1, ...
+    bf16* st = ring + PLACES * TERMS;                            // [3][V][SS] the state
+    bf16* ut = st + 3 * V * SS;                             // [3][V][MS] the weighted U
     __shared__ __align__(16) float2 f[2][L];
     tw_grid_wait();
     tw_grid_launch_dependents();
-    const int h = blockIdx.y, s = blockIdx.z, v0 = blockIdx.x * 16;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const int h = blockIdx.y, v0 = blockIdx.x * V;
+    int s = blockIdx.z;
+    if (a.n_seqs <= 32) {                                   // the longest request's blocks start first
+        const int mine = lane < a.n_seqs ? a.seq_q_len[lane] : -1;
+        int rank = 0;
+        for (int r = 0; r < a.n_seqs; ++r) {
+            const int other = __shfl_sync(0xffffffffu, mine, r);
+            rank += other > mine || (other == mine && r < lane);
+        }
+        s = __ffs(__ballot_sync(0xffffffffu, lane < a.n_seqs && rank == s)) - 1;
+    }
     const int len = a.seq_q_len[s];
     if (len < a.min_len) return;
     const int chunks = (len + L - 1) / L, hq = h / a.qk_group, Hq = a.H / a.qk_group;
     const size_t first = first_chunk(a.seq_q_len, s, a.min_len);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     float* slot = a.state + (size_t)a.seq_slot[s] * a.state_stride + (size_t)h * ((size_t)DK * DV);
 
-    auto fetch = [&](int c) {
+    auto copy = [&](int place, const bf16* src) {
+        bf16* dst = ring + place * TERMS;
+        for (int e = threadIdx.x; e < 3 * L * (DK / 8); e += THREADS) {
+            const int r = e / (DK / 8), i = e % (DK / 8) * 8;
+            tw_attn::cp_async16(dst + r * RS + i, src + (size_t)r * DK + i, 16);
+        }
+    };
+    auto fetch_w = [&](int c) {                             // with the chunk's decays
         if (c < chunks) {
-            const bf16* w = a.w + ((first + c) * a.H + h) * (size_t)(3 * L * DK);
-            const bf16* k = a.keys + ((first + c) * Hq + hq) * (size_t)(3 * L * DK);
-            bf16* dst = ring + (c & 1) * 2 * TERMS;
-            for (int e = threadIdx.x; e < 3 * L * (DK / 8); e += THREADS) {
-                const int r = e / (DK / 8), i = e % (DK / 8) * 8;
-                tw_attn::cp_async16(dst + r * RS + i, w + (size_t)r * DK + i, 16);
-                tw_attn::cp_async16(dst + TERMS + r * RS + i, k + (size_t)r * DK + i, 16);
-            }
+            copy((2 * c) % PLACES, a.w + ((first + c) * a.H + h) * (size_t)(3 * L * DK));
             if (threadIdx.x < L / 2)
                 tw_attn::cp_async16(&f[c & 1][2 * threadIdx.x], a.decay + ((first + c) * a.H + h) * L + 2 * threadIdx.x, 16);
         }
         tw_attn::cp_async_commit();
     };
-    // U of this block's values and warp w's tokens 8 w ..: pairs of tokens of values v0 + g and v0 + g + 8
-    auto u_place = [&](int c, int upper) {
-        return reinterpret_cast<float2*>(a.u + ((first + c) * a.H + h) * ((size_t)L * DV) + u_at(v0 + 8 * upper, warp >> 1) + lane * 4 + (warp & 1) * 2);
+    auto fetch_k = [&](int c) {
+        if (c < chunks) copy((2 * c + 1) % PLACES, a.keys + ((first + c) * Hq + hq) * (size_t)(3 * L * DK));
+        tw_attn::cp_async_commit();
+    };
+    // U of this block's values and warp w's tokens 8 w ..: pairs of tokens of values v0 + 8 x + g
+    auto u_place = [&](int c, int x) {
+        return reinterpret_cast<float2*>(a.u + ((first + c) * a.H + h) * ((size_t)L * DV) + u_at(v0 + 8 * x, warp >> 1) + lane * 4 + (warp & 1) * 2);
     };
 
-    float S[NT][4];                                         // values g, g + 8; key channels 8 (NT w + n) + 2 tq, + 1
+    float S[VT][NT][4];                                     // values 16 z + g, + 8; key channels 8 (NT w + n) + 2 tq, + 1
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int z = 0; z < VT; ++z)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            S[n][e] = slot[(size_t)((warp * NT + n) * 8 + 2 * tq + (e & 1)) * DV + v0 + g + (e < 2 ? 0 : 8)];
-    fetch(0);
-    float2 ua = *u_place(0, 0), ub = *u_place(0, 1);
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                S[z][n][e] = slot[(size_t)((warp * NT + n) * 8 + 2 * tq + (e & 1)) * DV + v0 + 16 * z + g + (e < 2 ? 0 : 8)];
+    fetch_w(0);
+    fetch_k(0);
+    float2 u0[2 * VT];
+#pragma unroll
+    for (int x = 0; x < 2 * VT; ++x) u0[x] = *u_place(0, x);
     for (int c = 0; c < chunks; ++c) {
         // the state before this chunk: for the outputs, and as terms for everybody
         float* keep = a.before + ((first + c) * a.H + h) * ((size_t)DK * DV);
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            const int k8 = warp * NT + n;
+        for (int z = 0; z < VT; ++z)
 #pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                *reinterpret_cast<float2*>(keep + (((size_t)((v0 >> 3) + x) * KT + (k8 >> 1)) * 32 + lane) * 4 + (k8 & 1) * 2) =
-                    make_float2(S[n][2 * x], S[n][2 * x + 1]);
-                uint32_t hi, mid, lo;
-                split3(S[n][2 * x], S[n][2 * x + 1], hi, mid, lo);
-                bf16* p = st + (g + 8 * x) * SS + k8 * 8 + 2 * tq;
-                *reinterpret_cast<uint32_t*>(p) = hi;
-                *reinterpret_cast<uint32_t*>(p + 16 * SS) = mid;
-                *reinterpret_cast<uint32_t*>(p + 32 * SS) = lo;
+            for (int n = 0; n < NT; ++n) {
+                const int k8 = warp * NT + n;
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    *reinterpret_cast<float2*>(keep + (((size_t)((v0 >> 3) + 2 * z + x) * KT + (k8 >> 1)) * 32 + lane) * 4 + (k8 & 1) * 2) =
+                        make_float2(S[z][n][2 * x], S[z][n][2 * x + 1]);
+                    uint32_t hi, mid, lo;
+                    split3(S[z][n][2 * x], S[z][n][2 * x + 1], hi, mid, lo);
+                    bf16* p = st + (16 * z + g + 8 * x) * SS + k8 * 8 + 2 * tq;
+                    *reinterpret_cast<uint32_t*>(p) = hi;
+                    *reinterpret_cast<uint32_t*>(p + V * SS) = mid;
+                    *reinterpret_cast<uint32_t*>(p + 2 * V * SS) = lo;
+                }
             }
-        }
-        tw_attn::cp_async_wait<0>();
-        __syncthreads();                                    // the state, W, K and the decays are there; the other stage is free
-        fetch(c + 1);
-        const bf16* ws = ring + (c & 1) * 2 * TERMS;
-        const bf16* ks = ws + TERMS;
+        tw_attn::cp_async_wait<1>();
+        __syncthreads();                                    // the state, W and the decays are there; nobody reads the keys before these
+        fetch_w(c + 1);
+        if constexpr (PLACES == 4) fetch_k(c + 1);
+        const bf16* ws = ring + (2 * c) % PLACES * TERMS;
+        const bf16* ks = ring + (2 * c + 1) % PLACES * TERMS;
         // ---- U^T = U0^T - S^T W^T, this warp's eight tokens
         // (the smaller products in sums of their own)
-        float top[4] = {0.f, 0.f, 0.f, 0.f}, low[6][4];
+        float top[VT][4], low[VT][6][4];
 #pragma unroll
-        for (int x = 0; x < 6; ++x) low[x][0] = low[x][1] = low[x][2] = low[x][3] = 0.f;
+        for (int z = 0; z < VT; ++z) {
+            top[z][0] = top[z][1] = top[z][2] = top[z][3] = 0.f;
+#pragma unroll
+            for (int x = 0; x < 6; ++x) low[z][x][0] = low[z][x][1] = low[z][x][2] = low[z][x][3] = 0.f;
+        }
 #pragma unroll
         for (int k = 0; k < KT; k += 2) {
-            uint32_t A[2][3][4];
+            uint32_t B[3][4];                               // two steps of k: (k, first and last eight), (k + 1, ...)
+#pragma unroll
+            for (int u = 0; u < 3; ++u) ldmatrix_x4(B[u], ws + (u * L + warp * 8 + (lane & 7)) * RS + k * 16 + (lane >> 3) * 8);
 #pragma unroll
             for (int x = 0; x < 2; ++x)
 #pragma unroll
-                for (int t = 0; t < 3; ++t) ldmatrix_x4(A[x][t], st + (t * 16 + (lane & 15)) * SS + (k + x) * 16 + (lane >> 4) * 8);
+                for (int z = 0; z < VT; ++z) {
+                    uint32_t A[3][4];
 #pragma unroll
-            for (int u = 2; u >= 0; --u) {
-                uint32_t B[4];                              // two steps of k: (k, first and last eight), (k + 1, ...)
-                ldmatrix_x4(B, ws + (u * L + warp * 8 + (lane & 7)) * RS + k * 16 + (lane >> 3) * 8);
+                    for (int t = 0; t < 3; ++t) ldmatrix_x4(A[t], st + (t * V + 16 * z + (lane & 15)) * SS + (k + x) * 16 + (lane >> 4) * 8);
 #pragma unroll
-                for (int x = 0; x < 2; ++x)
+                    for (int u = 2; u >= 0; --u)
 #pragma unroll
-                    for (int t = 2 - u; t >= 0; --t) {
-                        if (t + u == 0) mma_top(top, A[x][t], B[2 * x], B[2 * x + 1]);
-                        else mma_bf16(low[3 * x + u], A[x][t], B[2 * x], B[2 * x + 1]);
-                    }
-            }
+                        for (int t = 2 - u; t >= 0; --t) {
+                            if (t + u == 0) mma_top(top[z], A[t], B[u][2 * x], B[u][2 * x + 1]);
+                            else mma_bf16(low[z][3 * x + u], A[t], B[u][2 * x], B[u][2 * x + 1]);
+                        }
+                }
         }
-        float U[4] = {ua.x, ua.y, ub.x, ub.y};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) U[e] -= top[e] + (((low[0][e] + low[3][e]) + (low[1][e] + low[4][e])) + (low[2][e] + low[5][e]));
-        *u_place(c, 0) = make_float2(U[0], U[1]);
-        *u_place(c, 1) = make_float2(U[2], U[3]);
-        if (c + 1 < chunks) { ua = *u_place(c + 1, 0); ub = *u_place(c + 1, 1); }
         const float2 fl = f[c & 1][L - 1];
         const float whole = expf(fl.x + fl.y);
         {
@@ -345,58 +371,83 @@ __global__ void __launch_bounds__(THREADS, 1) delta_walk_kernel(DcArgs a) {
             const float2 fa = f[c & 1][t0], fb = f[c & 1][t0 + 1];
             const float wa = expf((fl.x - fa.x) + (fl.y - fa.y)), wb = expf((fl.x - fb.x) + (fl.y - fb.y));
 #pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                uint32_t hi, mid, lo;
-                split3(U[2 * x] * wa, U[2 * x + 1] * wb, hi, mid, lo);
-                bf16* p = ut + (g + 8 * x) * MS + t0;
-                *reinterpret_cast<uint32_t*>(p) = hi;
-                *reinterpret_cast<uint32_t*>(p + 16 * MS) = mid;
-                *reinterpret_cast<uint32_t*>(p + 32 * MS) = lo;
+            for (int z = 0; z < VT; ++z) {
+                float U[4] = {u0[2 * z].x, u0[2 * z].y, u0[2 * z + 1].x, u0[2 * z + 1].y};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    U[e] -= top[z][e] + (((low[z][0][e] + low[z][3][e]) + (low[z][1][e] + low[z][4][e])) + (low[z][2][e] + low[z][5][e]));
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    *u_place(c, 2 * z + x) = make_float2(U[2 * x], U[2 * x + 1]);
+                    uint32_t hi, mid, lo;
+                    split3(U[2 * x] * wa, U[2 * x + 1] * wb, hi, mid, lo);
+                    bf16* p = ut + (16 * z + g + 8 * x) * MS + t0;
+                    *reinterpret_cast<uint32_t*>(p) = hi;
+                    *reinterpret_cast<uint32_t*>(p + V * MS) = mid;
+                    *reinterpret_cast<uint32_t*>(p + 2 * V * MS) = lo;
+                }
             }
         }
-        __syncthreads();                                    // the weighted U is there, and nobody reads the old state any more
+        if (c + 1 < chunks) {
+#pragma unroll
+            for (int x = 0; x < 2 * VT; ++x) u0[x] = *u_place(c + 1, x);
+        }
+        tw_attn::cp_async_wait<PLACES - 2>();
+        __syncthreads();                                    // the weighted U and the keys are there, and nobody reads W or the old state any more
+        if constexpr (PLACES == 3) fetch_k(c + 1);
         // ---- S^T = e^F S^T + (w U)^T K, this warp's key channels
-        float lo2[3][NT][4];
+        float lo2[VT][3][NT][4];
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int z = 0; z < VT; ++z)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { S[n][e] *= whole; lo2[0][n][e] = lo2[1][n][e] = lo2[2][n][e] = 0.f; }
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { S[z][n][e] *= whole; lo2[z][0][n][e] = lo2[z][1][n][e] = lo2[z][2][n][e] = 0.f; }
 #pragma unroll
         for (int k = 0; k < L / 16; ++k) {
-            uint32_t A[3][4];
+            uint32_t B[3][4];
 #pragma unroll
-            for (int t = 0; t < 3; ++t) ldmatrix_x4(A[t], ut + (t * 16 + (lane & 15)) * MS + k * 16 + (lane >> 4) * 8);
-#pragma unroll
-            for (int u = 2; u >= 0; --u) {
-                uint32_t B[4];
+            for (int u = 0; u < 3; ++u) {
                 const bf16* base = ks + (u * L + k * 16 + (lane & 15)) * RS + warp * NT * 8;
                 if constexpr (NT == 2) {
-                    ldmatrix_x4_trans(B, base + (lane >> 4) * 8);
+                    ldmatrix_x4_trans(B[u], base + (lane >> 4) * 8);
                 } else {
                     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
-                                 : "=r"(B[0]), "=r"(B[1]) : "r"((uint32_t)__cvta_generic_to_shared(base)));
+                                 : "=r"(B[u][0]), "=r"(B[u][1]) : "r"((uint32_t)__cvta_generic_to_shared(base)));
                 }
+            }
 #pragma unroll
-                for (int n = 0; n < NT; ++n)
+            for (int z = 0; z < VT; ++z) {
+                uint32_t A[3][4];
 #pragma unroll
-                    for (int t = 2 - u; t >= 0; --t) {
-                        if (t + u == 0) mma_top(S[n], A[t], B[2 * n], B[2 * n + 1]);
-                        else mma_bf16(lo2[u][n], A[t], B[2 * n], B[2 * n + 1]);
-                    }
+                for (int t = 0; t < 3; ++t) ldmatrix_x4(A[t], ut + (t * V + 16 * z + (lane & 15)) * MS + k * 16 + (lane >> 4) * 8);
+#pragma unroll
+                for (int u = 2; u >= 0; --u)
+#pragma unroll
+                    for (int n = 0; n < NT; ++n)
+#pragma unroll
+                        for (int t = 2 - u; t >= 0; --t) {
+                            if (t + u == 0) mma_top(S[z][n], A[t], B[u][2 * n], B[u][2 * n + 1]);
+                            else mma_bf16(lo2[z][u][n], A[t], B[u][2 * n], B[u][2 * n + 1]);
+                        }
             }
         }
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int z = 0; z < VT; ++z)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) S[n][e] += (lo2[0][n][e] + lo2[1][n][e]) + lo2[2][n][e];
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[z][n][e] += (lo2[z][0][n][e] + lo2[z][1][n][e]) + lo2[z][2][n][e];
     }
     tw_attn::cp_async_wait<0>();
     if (!a.write_state) return;
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int z = 0; z < VT; ++z)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            slot[(size_t)((warp * NT + n) * 8 + 2 * tq + (e & 1)) * DV + v0 + g + (e < 2 ? 0 : 8)] = S[n][e];
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                slot[(size_t)((warp * NT + n) * 8 + 2 * tq + (e & 1)) * DV + v0 + 16 * z + g + (e < 2 ? 0 : 8)] = S[z][n][e];
 }
 
 // ---- (3) a chunk's outputs, as in recurrence_chunks.cu; U is read like the state, in the order the tensor cores want.
@@ -574,15 +625,21 @@ __global__ void __launch_bounds__(THREADS, 2) delta_outputs_kernel(DcArgs a) {
 template <int DV>
 int launch_delta(const DcArgs& a, int max_q_len, cudaStream_t stream) {
     constexpr size_t terms = (size_t)3 * L * RS * 2;
-    constexpr size_t smem1 = terms + (size_t)L * (L + 4) * 4, smem2 = 4 * terms + (size_t)3 * 16 * (DK + 8 + MS) * 2, smem3 = 2 * terms;
-    static_assert(smem2 + 2 * L * 8 <= 227 * 1024 && smem1 <= 112 * 1024 && smem3 <= 112 * 1024, "shared memory");
+    constexpr size_t smem1 = terms + (size_t)L * (L + 4) * 4, smem3 = 2 * terms;
+    constexpr auto smem2 = [](int vt) constexpr { return (vt == 1 ? 4 : 3) * terms + (size_t)3 * 16 * vt * (DK + 8 + MS) * 2; };
+    static_assert(smem2(1) + 2 * L * 8 <= 227 * 1024 && smem2(2) + 2 * L * 8 <= 227 * 1024 && smem1 <= 112 * 1024 && smem3 <= 112 * 1024, "shared memory");
     if (const int e = tw_allow_shared<delta_solve_kernel<DV>, (int)smem1>()) return e;
-    if (const int e = tw_allow_shared<delta_walk_kernel<DV>, (int)smem2>()) return e;
+    if (const int e = tw_allow_shared<delta_walk_kernel<DV, 1>, (int)smem2(1)>()) return e;
+    if (const int e = tw_allow_shared<delta_walk_kernel<DV, 2>, (int)smem2(2)>()) return e;
     if (const int e = tw_allow_shared<delta_outputs_kernel<DV>, (int)smem3>()) return e;
     const dim3 grid((max_q_len + L - 1) / L, a.H, a.n_seqs);
     int code = tw_launch(delta_solve_kernel<DV>, grid, dim3(THREADS), smem1, stream, 1, a);
     if (code) return code;
-    code = tw_launch(delta_walk_kernel<DV>, dim3(DV / 16, a.H, a.n_seqs), dim3(THREADS), smem2, stream, 1, a);
+    // (148 SMs: the same line on any part of the kind)
+    if ((long long)DV / 16 * a.H * a.n_seqs > 148)
+        code = tw_launch(delta_walk_kernel<DV, 2>, dim3(DV / 32, a.H, a.n_seqs), dim3(THREADS), smem2(2), stream, 1, a);
+    else
+        code = tw_launch(delta_walk_kernel<DV, 1>, dim3(DV / 16, a.H, a.n_seqs), dim3(THREADS), smem2(1), stream, 1, a);
     if (code) return code;
     return tw_launch(delta_outputs_kernel<DV>, grid, dim3(THREADS), smem3, stream, 1, a);
 }
