@@ -21,6 +21,8 @@ import threading
 import time
 from pathlib import Path
 
+from .settings import setting
+
 CSRC = Path(__file__).resolve().parent
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
@@ -120,7 +122,7 @@ def compile_library(name: str, defines: dict[str, int | str] | None = None, verb
 
 def timeline_enabled() -> bool:
     """``TESSWEAVE_TIMELINE=1``: every library is compiled with the device-side timeline (see common.cuh)."""
-    return os.environ.get("TESSWEAVE_TIMELINE") == "1"
+    return setting("TESSWEAVE_TIMELINE") == "1"
 
 
 _timeline_buffer: list[int] = [0]     # device address handed to every library loaded with the timeline

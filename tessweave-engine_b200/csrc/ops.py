@@ -14,7 +14,8 @@ from dataclasses import dataclass
 
 import torch
 
-from .build import load_library
+from .build import load_library, timeline_enabled
+from .settings import setting
 
 F32, BF16 = 0, 1
 
@@ -54,7 +55,7 @@ def _ptr(t: torch.Tensor | None) -> c_void_p:
 def _stream() -> c_void_p:
     # the raw handle of torch's current stream (what torch.cuda.current_stream().cuda_stream gives, without
     # building a Stream object for every launch)
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _need(cond: bool, message: str) -> None:
@@ -74,7 +75,6 @@ def _check(code: int, what: str) -> None:
                           f"({torch.cuda.get_device_name() if torch.cuda.is_available() else 'no device'})")
 
 
-_sigs_done: set[str] = set()
 LAUNCHES = [0]      # kernel launchers called so far (each call launches at least one kernel)
 CALL_LOG: list[str] | None = None     # when a list: the launchers called, by name (who measures asks which kernel ran)
 
@@ -84,15 +84,19 @@ def note_call(name: str) -> None:
         CALL_LOG.append(name)
 
 
+_functions: dict[tuple, object] = {}      # launchers of loaded libraries, which stay loaded
+
+
 def _fn(lib_name: str, fn_name: str, defines=None):
     LAUNCHES[0] += 1
-    note_call(fn_name)
-    lib = load_library(lib_name, defines)
-    fn = getattr(lib, fn_name)
-    key = f"{lib_name}:{fn_name}:{defines}"
-    if key not in _sigs_done:
+    if CALL_LOG is not None:
+        CALL_LOG.append(fn_name)
+    key = (fn_name, lib_name, timeline_enabled(), *defines.items()) if defines else (fn_name, lib_name, timeline_enabled())
+    fn = _functions.get(key)
+    if fn is None:
+        fn = getattr(load_library(lib_name, defines), fn_name)
         fn.restype = c_int
-        _sigs_done.add(key)
+        _functions[key] = fn
     return fn
 
 
@@ -217,8 +221,7 @@ def sigmoid_attention_tensor_cores(dtype: torch.dtype, head_dim: int, n_kv_heads
     """Whether the tensor-core kernels (csrc/sigmoid_attention_bf16.cu) take the shape: bfloat16, a head size that is a
     multiple of 16 up to 256, and a tile of 64 folded queries plus the ring of four key chunks within 227 KB of shared
     memory.  TESSWEAVE_SIGMOID_ATTENTION=exact sends everything to the exact kernel."""
-    import os
-    if os.environ.get("TESSWEAVE_SIGMOID_ATTENTION") == "exact":
+    if setting("TESSWEAVE_SIGMOID_ATTENTION") == "exact":
         return False
     if dtype != torch.bfloat16 or head_dim % 16 or not 16 <= head_dim <= 256:
         return False
@@ -228,8 +231,7 @@ def sigmoid_attention_tensor_cores(dtype: torch.dtype, head_dim: int, n_kv_heads
 def sigmoid_decode_heads_per_block() -> int:
     """0: a block of the sliced-keys kernel serves up to 32 heads of a request (the keys are read once for all of
     them); TESSWEAVE_SIGMOID_DECODE_HEADS=16 forces blocks of 16 heads (half the registers, the keys read twice)."""
-    import os
-    return 16 if os.environ.get("TESSWEAVE_SIGMOID_DECODE_HEADS") == "16" else 0
+    return 16 if setting("TESSWEAVE_SIGMOID_DECODE_HEADS") == "16" else 0
 
 
 def sigmoid_decode_splits(n_seqs: int, n_heads: int, max_kv_len: int) -> int:
@@ -237,8 +239,7 @@ def sigmoid_decode_splits(n_seqs: int, n_heads: int, max_kv_len: int) -> int:
     at least one tile of 64 keys per slice, at most 64 slices.  A block streams its slice slowly (it waits on its own
     chain of dependent tensor-core products), so the bandwidth comes from the number of blocks: one request with 4,096
     keys takes 24 us with 32 slices and 18 us with 64."""
-    import os
-    forced = os.environ.get("TESSWEAVE_SIGMOID_DECODE_SPLITS")
+    forced = setting("TESSWEAVE_SIGMOID_DECODE_SPLITS")
     tiles = max(1, -(-max_kv_len // 64))
     if forced:
         return max(1, min(int(forced), 64, tiles))
@@ -284,8 +285,7 @@ def sigmoid_tcgen05_key_tile() -> int:
     """Keys per tile of the tcgen05 sigmoid attention: 128, or 64 with TESSWEAVE_SIGMOID_KEY_TILE=64 (chunks of 64
     keys make the rings beside the folded queries twice as deep, but a tile's fixed costs come twice as often:
     measured 226 us against 199 us for 2,048 tokens at 28 heads, 4 key/value heads of 128)."""
-    import os
-    return 64 if os.environ.get("TESSWEAVE_SIGMOID_KEY_TILE") == "64" else 128
+    return 64 if setting("TESSWEAVE_SIGMOID_KEY_TILE") == "64" else 128
 
 
 def sigmoid_attention_tcgen05(dtype: torch.dtype, head_dim: int, n_kv_heads: int, page_size: int, max_q_len: int) -> bool:
@@ -294,7 +294,6 @@ def sigmoid_attention_tcgen05(dtype: torch.dtype, head_dim: int, n_kv_heads: int
     multiple of it, folded queries of 128 rows that leave room for three chunks of keys in shared memory, and a
     portion of at least 128 tokens.  TESSWEAVE_SIGMOID_PREFILL=mma|tcgen05 forces one of the two (the latter only
     for shapes the kernel takes)."""
-    import os
     if dtype != torch.bfloat16 or head_dim not in (64, 128) or page_size < 4:
         return False
     tile = sigmoid_tcgen05_key_tile()
@@ -303,7 +302,7 @@ def sigmoid_attention_tcgen05(dtype: torch.dtype, head_dim: int, n_kv_heads: int
     blocks = head_dim // 64
     if (227 * 1024 - 1024 - 512 - n_kv_heads * blocks * 16384) // (blocks * tile * 128) < 3:
         return False
-    forced = os.environ.get("TESSWEAVE_SIGMOID_PREFILL")
+    forced = setting("TESSWEAVE_SIGMOID_PREFILL")
     if forced == "mma":
         return False
     if forced == "tcgen05":
@@ -883,10 +882,9 @@ def prefer_tcgen05_attention(dtype: torch.dtype, head_dim: int, page_size: int, 
     """Whether a step whose longest portion has ``max_q_len`` tokens runs its prompt attention on
     the tcgen05 kernel.  TESSWEAVE_PREFILL_ATTENTION=mma|tcgen05 forces one of the two (the latter
     only for shapes the kernel takes)."""
-    import os
     if not tcgen05_attention_supported(dtype, head_dim, page_size, v_dim):
         return False
-    forced = os.environ.get("TESSWEAVE_PREFILL_ATTENTION")
+    forced = setting("TESSWEAVE_PREFILL_ATTENTION")
     if forced == "mma":
         return False
     if forced == "tcgen05":
@@ -909,8 +907,7 @@ def decode_splits(n_seqs: int, n_kv_heads: int, group: int, max_kv_len: int, v_d
     Values of more than 128 leave fewer blocks on an SM, and a launch of more blocks than fit at once pays for every
     further one (28 heads over cached rows of 256 values, batch 8, 4,096 keys, the kernel alone: 29.6 us with 8 slices on
     256 blocks, 46 to 62 with 9 to 16)."""
-    import os
-    forced = os.environ.get("TESSWEAVE_DECODE_SPLITS")
+    forced = setting("TESSWEAVE_DECODE_SPLITS")
     if forced:
         return max(1, min(int(forced), 128, DECODE_SCRATCH_UNITS // max(1, n_seqs)))
     head_tiles = (group + 7) // 8
@@ -1020,8 +1017,7 @@ def weight_prefetch_bytes() -> int:
     a decode step's attention asks into L2 while its slices merge.  Measured on a 7B-size layer: 24 to 32 MB is
     best at 1, 8 and 64 requests; more competes with the output product that runs in between, and asking for
     that product's own matrix gains nothing.  TESSWEAVE_WEIGHT_PREFETCH_MB overrides it; 0 switches it off."""
-    import os
-    mb = os.environ.get("TESSWEAVE_WEIGHT_PREFETCH_MB")
+    mb = setting("TESSWEAVE_WEIGHT_PREFETCH_MB")
     return WEIGHT_PREFETCH_BYTES if mb is None else max(0, int(mb)) << 20
 
 
@@ -1047,8 +1043,7 @@ def output_product_prefetch_bytes() -> int:
     decode steps: 8 / 16 / 24 / 32 / 48 / 64 / 96 MB give 0.6 / 1.0 / 1.2 / 1.2 / 1.1 / 0.6 / 0 % at 8 requests and
     the same at one; at the 14B sizes 16 and 24 MB are better than 32 (one request: 2 and 1 %).
     TESSWEAVE_OUTPUT_PREFETCH_MB overrides it; 0 switches it off."""
-    import os
-    mb = os.environ.get("TESSWEAVE_OUTPUT_PREFETCH_MB")
+    mb = setting("TESSWEAVE_OUTPUT_PREFETCH_MB")
     return OUTPUT_PRODUCT_PREFETCH_BYTES if mb is None else max(0, int(mb)) << 20
 
 
@@ -1058,8 +1053,7 @@ def product_prefetch_bytes() -> int:
     requests.  Before a product that is resident early (q/k/v behind the norm, the attention's output product)
     the same request makes the step slower, so only the feed-forward uses it.  TESSWEAVE_PRODUCT_PREFETCH_MB
     overrides it; 0 switches it off."""
-    import os
-    mb = os.environ.get("TESSWEAVE_PRODUCT_PREFETCH_MB")
+    mb = setting("TESSWEAVE_PRODUCT_PREFETCH_MB")
     return PRODUCT_PREFETCH_BYTES if mb is None else max(0, int(mb)) << 20
 
 
@@ -1067,15 +1061,13 @@ def weight_prefetch_min_cache_bytes() -> int:
     """The attention of a decode step prefetches weights only if it reads at least this much of the cache: a
     shorter kernel ends while the output product still fetches its own matrix, and the prefetch gets in its way
     (one request at 512 keys of a 7B-size layer: 1.4% slower with it).  TESSWEAVE_WEIGHT_PREFETCH_MIN_KB overrides."""
-    import os
-    kb = os.environ.get("TESSWEAVE_WEIGHT_PREFETCH_MIN_KB")
+    kb = setting("TESSWEAVE_WEIGHT_PREFETCH_MIN_KB")
     return (2 << 20) if kb is None else int(kb) << 10
 
 
 def fused_decode_enabled() -> bool:
     """TESSWEAVE_FUSED_DECODE=0 keeps bias, rotation and cache write of decode-only steps in a kernel of their own."""
-    import os
-    return os.environ.get("TESSWEAVE_FUSED_DECODE", "1") != "0"
+    return setting("TESSWEAVE_FUSED_DECODE", "1") != "0"
 
 
 def attention_decode_fused(out, source, bias, inv_freq, write_cache, seq_q_start, seq_q_len, seq_kv_len, seq_slot,
@@ -1140,8 +1132,7 @@ def decode_tma_supported(dtype: torch.dtype, head_dim: int, page_size: int, v_di
     """Whether single-token requests attend through ``attention_decode_tma``: bfloat16, a head size of 64, 128,
     192 or 256, and pages that are a whole fraction (at least 4 keys) or a whole multiple of a 64-key tile.
     TESSWEAVE_DECODE_TMA=0 keeps the kernel that loads keys through registers."""
-    import os
-    if os.environ.get("TESSWEAVE_DECODE_TMA", "1") == "0":
+    if setting("TESSWEAVE_DECODE_TMA", "1") == "0":
         return False
     return (dtype == torch.bfloat16 and all(d % 64 == 0 and 64 <= d <= 256 for d in (head_dim, v_dim or head_dim)) and page_size >= 4
             and (64 % page_size == 0 or page_size % 64 == 0))
@@ -1157,8 +1148,7 @@ def decode_tma_splits(n_seqs: int, n_kv_heads: int, group: int, max_kv_len: int)
     ms, with 12 or 16 3.4 to 3.5).  Few requests with long contexts take more slices and merge through scratch
     memory (16,384 keys, batch 2, 12 layers: 1.56 ms with 32 slices, 1.89 with 16).
     TESSWEAVE_DECODE_SPLITS forces a number."""
-    import os
-    forced = os.environ.get("TESSWEAVE_DECODE_SPLITS")
+    forced = setting("TESSWEAVE_DECODE_SPLITS")
     tiles = max(1, -(-max_kv_len // 64))
     most = min(tiles, DECODE_MAX_SPLITS, DECODE_SCRATCH_UNITS // max(1, n_seqs))
     if forced:
@@ -1190,8 +1180,7 @@ def decode_attention_resident_early(blocks: int, nsplit: int) -> bool:
     faster, 144 and 156 blocks (4 requests at 512 keys, 3 at 4,096) 1.7 and 1.1 % faster, 208 blocks (4 requests
     at 4,096 keys) 9 % slower, 256 blocks (8 requests) 5 to 10 % slower; launches that merge through scratch
     memory (no clusters) 1 % faster at 128 and at 256 blocks.  TESSWEAVE_DECODE_EARLY=0/1 forces it."""
-    import os
-    forced = os.environ.get("TESSWEAVE_DECODE_EARLY")
+    forced = setting("TESSWEAVE_DECODE_EARLY")
     if forced is not None:
         return forced == "1"
     return nsplit > DECODE_TMA_CLUSTER_SLICES or blocks * 10 <= _SM_COUNT * 11
@@ -1210,7 +1199,6 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
     ``gate``: as for ``attention_decode``; with ``q`` the values may have another size than the keys, or be the keys (the same
     pages), and ``sink`` (fp32 [Hq]) may join the denominator.  ``beside_prompts`` (with ``q``): the last kernel launched on this
     stream is ``attention_prefill_tcgen05`` of the same step with ``skip_single``, and this one runs beside it."""
-    import os
     _need(source is None or not beside_prompts, "attention_decode_tma: only with q given can it run beside the prompts' attention")
     width = (n_q_heads + 2 * n_kv_heads) * head_dim
     partial = dense = None
@@ -1235,7 +1223,7 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
           "attention_decode_tma: the sink must be fp32 [Hq], with q given")
     _need(source is None or k_pages.data_ptr() != v_pages.data_ptr(), "attention_decode_tma: values that are the keys go with q given")
     v_dim = v_pages.shape[3]
-    _need(decode_tma_supported(out.dtype, head_dim, k_pages.shape[2], v_dim) or os.environ.get("TESSWEAVE_DECODE_TMA") == "0",
+    _need(decode_tma_supported(out.dtype, head_dim, k_pages.shape[2], v_dim) or setting("TESSWEAVE_DECODE_TMA") == "0",
           f"attention_decode_tma does not take head size {head_dim} with pages of {k_pages.shape[2]} keys in {out.dtype}")
     _need(out.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16, "attention_decode_tma: bfloat16 only")
     _need(n_q_heads % n_kv_heads == 0, "attention: query heads must be a multiple of key/value heads")
@@ -1256,7 +1244,7 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
         _need(counters is not None and counters.dtype == torch.int32
               and counters.numel() >= n_seqs * n_kv_heads * ((n_q_heads // n_kv_heads + 7) // 8),
               "attention_decode: too few counters")
-    stages = stages or int(os.environ.get("TESSWEAVE_DECODE_STAGES", "0"))
+    stages = stages or int(setting("TESSWEAVE_DECODE_STAGES", "0"))
     code = _fn("attention_decode_tma", "tw_attn_decode_tma", head_size_defines(head_dim, v_dim))(
         _ptr(out), c_int(out.stride(0)), _ptr(q), c_int(q.stride(0) if q is not None else 0), _ptr(partial), c_int(nslices),
         ctypes.c_longlong(slice_stride), _ptr(dense), c_int(dense_stride), _ptr(bias), _ptr(inv_freq),
@@ -1311,10 +1299,9 @@ def prefer_latent_tcgen05(dtype: torch.dtype, head_dim: int, page_size: int, max
     start (28 heads over rows of 256 values: 13.4 us against 9.3 for a prompt of 64 tokens, 15.3 against 18.3 for 256, 40
     against 103 for a portion of 16 tokens behind 2,048).  TESSWEAVE_PREFILL_ATTENTION=mma|tcgen05 forces one
     of the two (the latter only for shapes the kernel takes)."""
-    import os
     if dtype != torch.bfloat16 or head_dim % 16 or not 16 <= head_dim <= 256 or latent_tcgen05_key_tile(page_size) is None:
         return False
-    forced = os.environ.get("TESSWEAVE_PREFILL_ATTENTION")
+    forced = setting("TESSWEAVE_PREFILL_ATTENTION")
     if forced in ("mma", "tcgen05"):
         return forced == "tcgen05"
     return max_keys >= LATENT_TCGEN05_MIN_KEYS
@@ -1537,8 +1524,7 @@ def pair_product_preferred(x: torch.Tensor, w: torch.Tensor, m: int) -> bool:
     the tiles do not fill whole rounds of pairs (1,280 rows: 271.9 against 260.7).  So: from 768 rows, and only
     where padding and rounds leave at least 93 % of the pairs' time useful.  TESSWEAVE_PAIR_GEMM=0 keeps the library,
     =force takes the pairs for every shape beyond 64 rows."""
-    import os
-    choice = os.environ.get("TESSWEAVE_PAIR_GEMM", "1")
+    choice = setting("TESSWEAVE_PAIR_GEMM", "1")
     if choice == "0":
         return False
     takes = (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[0] % 16 == 0
@@ -1591,11 +1577,10 @@ def stream_product_preferred(x: torch.Tensor, w: torch.Tensor, m: int) -> bool:
     (8.8 / 10.7 against 8.6 / 8.9) stay with the library, whose split over k is reduced inside its kernel.
     TESSWEAVE_STREAM_GEMM=0 keeps the library everywhere; TESSWEAVE_STREAM_MAX_M and TESSWEAVE_STREAM_MIN_WEIGHTS
     move the bounds."""
-    import os
-    if os.environ.get("TESSWEAVE_STREAM_GEMM", "1") == "0":
+    if setting("TESSWEAVE_STREAM_GEMM", "1") == "0":
         return False
-    top = min(STREAM_MAX_M, int(os.environ.get("TESSWEAVE_STREAM_MAX_M", "64")))
-    least = int(os.environ.get("TESSWEAVE_STREAM_MIN_WEIGHTS", str(STREAM_MIN_WEIGHTS)))
+    top = min(STREAM_MAX_M, int(setting("TESSWEAVE_STREAM_MAX_M", "64")))
+    least = int(setting("TESSWEAVE_STREAM_MIN_WEIGHTS", str(STREAM_MIN_WEIGHTS)))
     return (x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and STREAM_MIN_M <= m <= top
             and w.numel() >= least and w.shape[1] % 8 == 0 and x.is_contiguous() and w.is_contiguous()
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -1624,8 +1609,7 @@ def stream_split_gate_up_enabled() -> bool:
     runs on the persistent kernel in slices over k that the SiLU.mul kernel adds.  Off by default: measured at 14B
     layer sizes a decode step is 1 % shorter with it at batch 12 and 24 and 2.5 % longer at batch 32, where the
     library's product is at its best."""
-    import os
-    return os.environ.get("TESSWEAVE_STREAM_SPLIT_GATE_UP", "0") == "1"
+    return setting("TESSWEAVE_STREAM_SPLIT_GATE_UP", "0") == "1"
 
 
 def stream_split(n: int, k: int, allow: bool = True, sms: int | None = None) -> tuple[int, int]:
@@ -1890,10 +1874,9 @@ def state_space_chunks_supported(dtype: torch.dtype, state_dim: int, value_dim: 
     """Whether a step whose longest portion has ``max_q_len`` tokens runs the state-space recurrence in chunks on the
     tensor cores: bfloat16 rows, state sizes and values the tiles take, and more than a few tokens.
     TESSWEAVE_STATE_SPACE=tokens|chunks forces one of the two (the latter only for sizes the kernel takes)."""
-    import os
     if dtype != torch.bfloat16 or state_dim not in STATE_SPACE_CHUNK_STATES or value_dim % 16 or channels % 8:
         return False
-    forced = os.environ.get("TESSWEAVE_STATE_SPACE")
+    forced = setting("TESSWEAVE_STATE_SPACE")
     if forced in ("tokens", "chunks"):
         return forced == "chunks"
     return max_q_len >= STATE_SPACE_CHUNK_MIN_TOKENS

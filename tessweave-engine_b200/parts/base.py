@@ -19,7 +19,6 @@ comes next.
 """
 from __future__ import annotations
 
-import os
 from dataclasses import dataclass, field
 from typing import Any, Callable
 
@@ -27,6 +26,7 @@ import torch
 
 from ..csrc import ops
 from ..csrc.ops import SplitSum
+from ..csrc.settings import setting
 
 
 # ---------------------------------------------------------------------------
@@ -140,7 +140,7 @@ def poison_new_buffers() -> bool:
     number), so that a kernel that reads what nobody wrote gives NaN instead of whatever the memory held.
     Fresh device memory is often zero, or holds the same values an earlier run left there, and hides
     such a read."""
-    return os.environ.get("TESSWEAVE_POISON_BUFFERS", "0") == "1"
+    return setting("TESSWEAVE_POISON_BUFFERS", "0") == "1"
 
 
 def poisoned(t: torch.Tensor) -> torch.Tensor:
@@ -156,19 +156,26 @@ class Workspace:
     step does not grow with depth, and addresses stay fixed for CUDA graphs.
     """
 
+    MAX_VIEWS = 512
+
     def __init__(self, device: torch.device):
         self.device = device
         self._buffers: dict[str, torch.Tensor] = {}
+        self._views: dict[tuple, torch.Tensor] = {}     # of the buffers as they are, by (name, shape, type); at most MAX_VIEWS
         self.frozen = False
         self.prefix = ""        # put before every name: a part that runs several parts side by side gives each buffers of its own
 
     def get(self, name: str, shape: tuple[int, ...], dtype: torch.dtype, zero: bool = False) -> torch.Tensor:
         """The buffer ``name`` with at least ``shape`` elements.  ``zero`` fills it with zeros when it
         is (re)allocated -- for state that kernels keep zero between launches, such as counters."""
+        name = self.prefix + name
+        key = (name, shape, dtype)
+        view = self._views.get(key)
+        if view is not None:
+            return view
         numel = 1
         for s in shape:
             numel *= int(s)
-        name = self.prefix + name
         buf = self._buffers.get(name)
         if buf is None or buf.dtype != dtype or buf.numel() < numel:
             if self.frozen:
@@ -178,7 +185,11 @@ class Workspace:
             else:
                 buf = poisoned(torch.empty(max(numel, 1), dtype=dtype, device=self.device))
             self._buffers[name] = buf
-        return buf[:numel].view(*shape)
+            self._views.clear()             # (of the buffer that this one replaces, too)
+        if len(self._views) >= self.MAX_VIEWS:
+            self._views.clear()
+        view = self._views[key] = buf[:numel].view(*shape)
+        return view
 
     def reserve(self, name: str, shape: tuple[int, ...], dtype: torch.dtype) -> None:
         self.get(name, shape, dtype)
