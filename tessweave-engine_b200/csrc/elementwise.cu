@@ -1385,6 +1385,101 @@ norm_rotate_store_kernel(T* __restrict__ rows, int row_stride, NormSpans sp, T* 
     }
 }
 
+// The same for few rows of attention over latents in bfloat16: one head in each span, the cached row the second span and the rotated
+// values behind it, everything on 16-byte boundaries.  A decode step has a block per request and waits for its chain of loads, so
+// nothing is done one after the other here: the spans, the rotation and the gates have warps of their own, what depends on the
+// position and the weights alone is had before the wait for the product, and the cached row is written from registers.  The sums of
+// squares have the order of the kernel above (the same bits).  8 rows of 1,536 + 192 + 64 + 28 columns: 4.6 us inside a captured
+// step, 7.1 with the kernel above; steps with more rows hide that chain behind one another and stay with it.
+#define TW_LATENT_ROWS 64
+__global__ void __launch_bounds__(1024)
+latent_row_kernel(__nv_bfloat16* __restrict__ rows, int row_stride, NormSpans sp, __nv_bfloat16* __restrict__ dst0, float eps,
+                  int rot_dims, const float* __restrict__ inv_freq, int interleaved, float magnitude, const int* __restrict__ positions,
+                  const int* __restrict__ seq_of_token, const int* __restrict__ seq_slot, const int* __restrict__ block_table,
+                  int table_stride, __nv_bfloat16* __restrict__ cache, int page_size, int num_pages, int write_cache, int gate_col,
+                  int gate_heads, float* __restrict__ gate_out, int* status) {
+    __shared__ float sums[2][32];
+    const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s = seq_of_token[n];
+    if (s < 0) {
+        tw_grid_wait();
+        return;
+    }
+    const int pos = positions[n];
+    const int D0 = sp.dim[0], D1 = sp.dim[1], half = rot_dims >> 1;
+    const int nv0 = D0 >> 3, nv1 = D1 >> 3;
+    const int w0 = (nv0 + 31) >> 5, w1 = w0 + ((nv1 + 31) >> 5), w2 = w1 + ((half + 31) >> 5);     // warps of the spans, then of the rotation, then of the gates
+    const int span = warp < w0 ? 0 : 1, i = (int)threadIdx.x - (warp < w0 ? 0 : warp < w1 ? w0 : warp < w2 ? w1 : w2) * 32;
+    const bool normed = warp < w1 && i < (span ? nv1 : nv0), rotated = warp >= w1 && warp < w2 && i < half, gated = warp >= w2 && i < gate_heads;
+    __nv_bfloat16* row = rows + (size_t)n * row_stride;
+    __nv_bfloat16* place = nullptr;
+    bool missing = false;
+    if (write_cache) {
+        const int blk = pos / page_size;
+        const int page = blk < table_stride ? block_table[(size_t)seq_slot[s] * table_stride + blk] : -1;
+        if (page >= 0 && page < num_pages) place = cache + ((size_t)page * page_size + (pos - blk * page_size)) * (D1 + rot_dims);
+        else missing = true;
+    }
+    float4 wa = make_float4(0.f, 0.f, 0.f, 0.f), wb = wa;
+    float sn = 0.f, cs = 1.f;
+    if (normed) {
+        wa = reinterpret_cast<const float4*>(sp.weight[span])[2 * i];
+        wb = reinterpret_cast<const float4*>(sp.weight[span])[2 * i + 1];
+    }
+    if (rotated) {
+        sincosf((float)pos * inv_freq[i], &sn, &cs);
+        sn *= magnitude;
+        cs *= magnitude;
+    }
+    tw_grid_wait();
+    if (missing && threadIdx.x == 0) atomicOr(status, TW_ERR_PAGE);
+    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+    float ss = 0.f;
+    if (normed) {
+        raw = reinterpret_cast<const uint4*>(row + sp.col[span])[i];
+        const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(p2[e]);
+            ss += f.x * f.x + f.y * f.y;
+        }
+    } else if (rotated) {
+        __nv_bfloat16* r = row + sp.col[1] + D1;
+        const int a = interleaved ? 2 * i : i, b = interleaved ? 2 * i + 1 : i + half;
+        const float u = __bfloat162float(r[a]), v = __bfloat162float(r[b]);
+        const __nv_bfloat16 y = __float2bfloat16_rn(u * cs - v * sn), z = __float2bfloat16_rn(v * cs + u * sn);
+        r[a] = y;
+        r[b] = z;
+        if (place) {
+            place[D1 + a] = y;
+            place[D1 + b] = z;
+        }
+    } else if (gated) {
+        gate_out[(size_t)n * gate_heads + i] = 1.0f / (1.0f + expf(-__bfloat162float(row[gate_col + i])));
+    }
+    if (warp < w1) {
+        ss = tw_warp_sum(ss);
+        if (lane == 0) sums[span][warp - (span ? w0 : 0)] = ss;
+    }
+    __syncthreads();
+    if (warp >= w1) return;
+    float total = lane < (span ? w1 - w0 : w0) ? sums[span][lane] : 0.f;
+    total = tw_warp_sum(total);
+    if (!normed) return;
+    const float inv = 1.0f / sqrtf(total / (float)(span ? D1 : D0) + eps);
+    const float ww[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+    const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    uint4 packed;
+    __nv_bfloat162* q2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(p2[e]);
+        q2[e] = __floats2bfloat162_rn((f.x * inv) * ww[2 * e], (f.y * inv) * ww[2 * e + 1]);
+    }
+    reinterpret_cast<uint4*>(span == 0 && dst0 ? dst0 + (size_t)n * D0 : row + sp.col[span])[i] = packed;
+    if (span && place) reinterpret_cast<uint4*>(place)[i] = packed;
+}
+
 TW_EXPORT int tw_norm_rotate_store(void* rows, int row_stride, int n_tokens, int spans, int col0, int heads0, int dim0,
                                    const float* weight0, void* dst0, int col1, int heads1, int dim1, const float* weight1, float eps,
                                    int rot_col, int rot_dims, const float* inv_freq, int interleaved, float magnitude, int k_col,
@@ -1413,6 +1508,13 @@ TW_EXPORT int tw_norm_rotate_store(void* rows, int row_stride, int n_tokens, int
                  && (row_stride & 7) == 0 && (k_col & 7) == 0 && (Dk & 7) == 0 && (!v_cache || ((v_col & 7) == 0 && (Dv & 7) == 0))) ? 1 : 0;
     for (int sidx = 0; sidx < 2; ++sidx)
         if (sp.heads[sidx] && ((sp.col[sidx] & 7) || (sp.dim[sidx] & 7) || (block_wide && sp.dim[sidx] > 16 * threads))) vec16 = 0;
+    const int latent_threads = 32 * ((sp.dim[0] / 8 + 31) / 32 + (sp.dim[1] / 8 + 31) / 32 + (rot_dims / 2 + 31) / 32 + (gate_heads + 31) / 32);
+    if (vec16 && block_wide && n_tokens <= TW_LATENT_ROWS && spans == 2 && heads0 == 1 && heads1 == 1 && Hkv == 1 && !v_cache && k_cache
+        && k_col == col1 && rot_col == col1 + dim1 && Dk == dim1 + rot_dims && widest <= 2048 && latent_threads <= 1024)
+        return tw_launch<TW_READS_AHEAD>(latent_row_kernel, dim3(n_tokens), dim3(latent_threads), 0, stream, 1, (__nv_bfloat16*)rows, row_stride,
+                                         sp, (__nv_bfloat16*)dst0, eps, rot_dims, inv_freq, interleaved, magnitude, positions, seq_of_token,
+                                         seq_slot, block_table, table_stride, (__nv_bfloat16*)k_cache, page_size, num_pages, write_cache,
+                                         gate_col, gate_heads, gate_out, status);
     if (dtype == TW_F32)
         return tw_launch(norm_rotate_store_kernel<float>, dim3(n_tokens), dim3(threads), 0, stream, 1, (float*)rows, row_stride, sp,
                          (float*)dst0, eps, block_wide, 0, rot_col, rot_dims, inv_freq, interleaved, magnitude, k_col, v_col, positions, seq_of_token,

@@ -1,0 +1,48 @@
+"""Kernels of decode steps that run a row's chain in parallel, against the kernels of many rows."""
+import pytest
+import torch
+
+
+def ops():
+    from tessweave_engine_b200.csrc import ops as o
+    return o
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ranks,rot,gates", [((1536, 192), 64, 28), ((128, 8), 0, 0), ((2048, 264), 32, 40), ((136, 512), 72, 5)])
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("own_rows,write_cache", [(True, True), (False, False)])
+def test_rows_of_attention_over_latents(ranks, rot, gates, interleaved, own_rows, write_cache):
+    """Up to 64 rows (a warp or more for each span, the rotation and the gates) give the bits of steps with more: the norms, the rotated
+    part, the cached rows and the gates; a row of no request is left alone, a page that is not there is reported."""
+    o, few, many, page = ops(), 9, 70, 16
+    g = torch.Generator().manual_seed(sum(ranks) + rot)
+    q_rank, kv_rank = ranks
+    head = kv_rank + rot
+    width = -(-(q_rank + head + gates) // 8) * 8
+    rows = torch.randn(many, width, generator=g).bfloat16().cuda()
+    seq = torch.arange(many, dtype=torch.int32)
+    seq[few - 2] = -1
+    i32 = lambda t: t.to(torch.int32).cuda()        # noqa: E731
+    positions, slots = torch.randint(0, 5 * page, (many,), generator=g), torch.randperm(many, generator=g)
+    table = torch.arange(many * 5).view(many, 5)
+    table[slots[1]] = -1                            # request 1 holds no page
+    w0, w1 = torch.randn(q_rank, generator=g).cuda(), torch.randn(kv_rank, generator=g).cuda()
+    inv_freq = (10000.0 ** (-torch.arange(0, max(rot, 2), 2) / max(rot, 2))).float().cuda()
+
+    def run(n):
+        x = rows[:n].clone()
+        cache = torch.full((many * 5, 1, page, head), 9.0, dtype=torch.bfloat16, device="cuda")
+        first = torch.full((n, q_rank), 5.0, dtype=torch.bfloat16, device="cuda") if own_rows else None
+        gate = torch.full((n, gates), 5.0, device="cuda") if gates else None
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        o.norm_rotate_store(x, n, [(0, 1, q_rank, w0), (q_rank, 1, kv_rank, w1)], 1e-6, i32(positions[:n]), i32(seq[:n]), i32(slots), i32(table),
+                            cache, None, q_rank, q_rank, write_cache, status, dst0=first, rot_col=q_rank + kv_rank, rot_dims=rot,
+                            inv_freq=inv_freq if rot else None, interleaved=interleaved, magnitude=1.1, gate_col=q_rank + head, gate_out=gate)
+        held = cache[table.clamp_min(0)[slots[:few]].cuda()]       # the pages of the few rows' requests
+        return x[:few], None if first is None else first[:few], None if gate is None else gate[:few], held, int(status) if write_cache else 0
+
+    got, want = run(few), run(many)
+    for a, b in zip(got, want):
+        assert a == b if isinstance(a, int) else a is None and b is None or torch.equal(a, b)
+    assert got[4] == (2 if write_cache else 0)
