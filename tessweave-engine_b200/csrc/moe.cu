@@ -20,6 +20,8 @@
 // Expert matrices are stacked: gate/up [E, 2, F, width] (a gate matrix followed by its up matrix), down
 // [E, width, F].  Dot products accumulate in fp32; the weighted sum over experts is fp32.
 #include "moe_common.cuh"
+#include <algorithm>
+#include <type_traits>
 
 template <typename T>
 __device__ __forceinline__ float tw_dot_row(const T* __restrict__ w, const float* __restrict__ x, int n, int lane) {
@@ -56,6 +58,43 @@ __device__ __forceinline__ float tw_dot_row8(const __nv_bfloat16* __restrict__ w
     }
     for (; i < n; i += 256) a0 = tw_fma8(tw_stream16(w + i), x + i, a0);
     return tw_warp_sum((a0 + a1) + (a2 + a3));
+}
+
+// The same with the other row as it lies in memory, which 16-byte accesses may read: the next step's loads of both are under way
+// while this one is added up.
+__device__ __forceinline__ float tw_dot_rows8(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x, int n, int lane) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    uint4 m[4], r[4];
+    auto load = [&](int i) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool in = i + 256 * q < n;
+            m[q] = in ? tw_stream16(w + i + 256 * q) : make_uint4(0u, 0u, 0u, 0u);
+            r[q] = in ? *reinterpret_cast<const uint4*>(x + i + 256 * q) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    load(lane * 8);
+    for (int i = lane * 8; i < n; i += 1024) {
+        uint4 mc[4], rc[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { mc[q] = m[q]; rc[q] = r[q]; }
+        load(i + 1024);
+        const bool whole = i + 768 < n;                 // (what is behind the last whole step goes to the first sum)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (i + 256 * q >= n) continue;
+            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&rc[q]);
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 f = __bfloat1622float2(p[k]);
+                v[2 * k] = f.x; v[2 * k + 1] = f.y;
+            }
+            if (whole) a[q] = tw_fma8(mc[q], v, a[q]);
+            else a[0] = tw_fma8(mc[q], v, a[0]);
+        }
+    }
+    return tw_warp_sum((a[0] + a[1]) + (a[2] + a[3]));
 }
 
 // two rows of equal length at once (an expert's gate row and its up row): eight loads of a lane under way
@@ -213,28 +252,41 @@ __device__ __forceinline__ void moe_select(float* z, int row, int lane, bool has
     for (int j = 0; j < top; ++j) weight[(size_t)row * top + j] /= sum;
 }
 
-template <typename T>
+// DIRECT (bf16 on 16-byte boundaries, at most a row for every SM): the row is read where it lies instead of being staged as 32-bit
+// numbers; the same bits.  Without the 14 KB of shared memory (3,584 values) the kernel may also start on an SM that still runs a
+// product: a kernel that wants another split of L1 and shared memory waits until the SM is empty.  3,584 x 8 outputs, staged and
+// direct: 32 rows 9.3 and 6.6 us, 128 rows 9.5 and 6.8, 512 rows 11.1 and 20.8.
+#define TW_ROUTE_DIRECT_ROWS 148
+template <typename T, bool DIRECT>
 __global__ void __launch_bounds__(512)
 moe_route_kernel(int* __restrict__ chosen, float* __restrict__ weight, float* __restrict__ shared_gate,
                  const T* __restrict__ h, int h_stride, const T* __restrict__ wr, const float* __restrict__ br,
                  const T* __restrict__ ws, int width, int E, int top, int scoring, const float* __restrict__ correction,
-                 float weight_scale, int group_count, int group_keep) {
-    extern __shared__ float sm[];           // [width] the row, [E + 1] logits, [E] marks, [2 group_count]
-    tw_grid_wait();
+                 float weight_scale, int group_count, int group_keep, int beside) {
+    extern __shared__ float sm[];           // [width] the row (not DIRECT), [E + 1] logits, [E] marks, [2 group_count]
+    // `beside`: the kernel before this one reads the same rows and writes nothing that is read here; it lets this kernel start
+    // once the rows are there, and one block waits for it, at its end.
+    if (!beside) tw_grid_wait();
     tw_grid_launch_dependents();
     const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* x = sm;
-    float* z = sm + width;
-    stage_row(x, h + (size_t)row * h_stride, width);
-    __syncthreads();
+    float* z = DIRECT ? sm : sm + width;
+    if constexpr (!DIRECT) {
+        stage_row(x, h + (size_t)row * h_stride, width);
+        __syncthreads();
+    }
     const bool vec = (width & 7) == 0;
     for (int e = warp; e < E + (ws ? 1 : 0); e += (int)(blockDim.x >> 5)) {
-        const float d = tw_dot<T>(e < E ? wr + (size_t)e * width : ws, x, width, lane, vec);
+        const T* we = e < E ? wr + (size_t)e * width : ws;
+        float d;
+        if constexpr (DIRECT) d = tw_dot_rows8(we, h + (size_t)row * h_stride, width, lane);
+        else d = tw_dot<T>(we, x, width, lane, vec);
         if (lane == 0) z[e] = e < E ? d + (br ? br[e] : 0.f) : d;
     }
     __syncthreads();
     if (warp != 0) return;
     moe_select(z, row, lane, ws != nullptr, E, top, scoring, correction, weight_scale, group_count, group_keep, chosen, weight, shared_gate);
+    if (beside && blockIdx.x == 0) tw_grid_wait();
 }
 
 // Steps of many bf16 rows: a warp per row, sixteen rows to a block, which copies the router's matrix to shared memory once.  The dot
@@ -314,7 +366,7 @@ moe_route_rows_kernel(int* __restrict__ chosen, float* __restrict__ weight, floa
 
 TW_EXPORT int tw_moe_route(int* chosen, float* weight, float* shared_gate, const void* h, int h_stride, const void* wr,
                            const float* br, const void* ws, int rows, int width, int E, int top, int scoring,
-                           const float* correction, float weight_scale, int group_count, int group_keep, int dtype,
+                           const float* correction, float weight_scale, int group_count, int group_keep, int beside, int dtype,
                            cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (E <= 0 || top <= 0 || top > E || scoring < 0 || scoring > 2) return (int)cudaErrorInvalidValue;
@@ -334,12 +386,19 @@ TW_EXPORT int tw_moe_route(int* chosen, float* weight, float* shared_gate, const
     }
     const int threads = 32 * min(16, max(4, E + 1));        // a warp per expert (and one for the shared gate), up to 16
     if (dtype == TW_F32)
-        return tw_launch(moe_route_kernel<float>, dim3(rows), dim3(threads), smem, stream, 1, chosen, weight, shared_gate,
+        return tw_launch(moe_route_kernel<float, false>, dim3(rows), dim3(threads), smem, stream, 1, chosen, weight, shared_gate,
                          (const float*)h, h_stride, (const float*)wr, br, (const float*)ws, width, E, top, scoring, correction,
-                         weight_scale, group_count, group_keep);
-    return tw_launch(moe_route_kernel<__nv_bfloat16>, dim3(rows), dim3(threads), smem, stream, 1, chosen, weight, shared_gate,
-                     (const __nv_bfloat16*)h, h_stride, (const __nv_bfloat16*)wr, br, (const __nv_bfloat16*)ws, width, E, top,
-                     scoring, correction, weight_scale, group_count, group_keep);
+                         weight_scale, group_count, group_keep, 0);
+    const bool direct = rows <= TW_ROUTE_DIRECT_ROWS && (width & 7) == 0 && (h_stride & 7) == 0 && a16(h) && a16(wr) && a16(ws);
+    // (1 KB at least: with less the driver splits L1 and shared memory otherwise than for the product beside)
+    const size_t used = direct ? std::max<size_t>(smem - (size_t)width * sizeof(float), 1024) : smem;
+    auto kernel = direct ? moe_route_kernel<__nv_bfloat16, true> : moe_route_kernel<__nv_bfloat16, false>;
+    auto launch = [&](auto how) {
+        return tw_launch<decltype(how)::value>(kernel, dim3(rows), dim3(threads), used, stream, 1, chosen, weight, shared_gate,
+                                               (const __nv_bfloat16*)h, h_stride, (const __nv_bfloat16*)wr, br, (const __nv_bfloat16*)ws, width,
+                                               E, top, scoring, correction, weight_scale, group_count, group_keep, beside ? 1 : 0);
+    };
+    return beside ? launch(std::integral_constant<int, TW_OVERLAPS>()) : launch(std::integral_constant<int, TW_BY_SIZE>());
 }
 
 #define TW_MOE_WARPS 8

@@ -2052,13 +2052,15 @@ def kv_store(rows: torch.Tensor, k_col: int, v_col: int, positions: torch.Tensor
 def moe_route(chosen: torch.Tensor, weight: torch.Tensor, shared_gate: torch.Tensor | None, h: torch.Tensor, w_router: torch.Tensor,
               b_router: torch.Tensor | None, w_shared_gate: torch.Tensor | None, n_rows: int, top: int,
               score_all: bool = False, correction: torch.Tensor | None = None, weight_scale: float = 1.0,
-              renormalise: bool = False, groups: tuple[int, int] | None = None) -> None:
+              renormalise: bool = False, groups: tuple[int, int] | None = None, beside: bool = False) -> None:
     """Per row: the ``top`` experts with the largest fp32 logits ``w_router h + b_router`` (int32 [rows, top]), the
     softmax over those logits alone (fp32 [rows, top]), and ``sigmoid(w_shared_gate . h)`` (fp32 [rows]) if asked.
     With ``score_all`` the scores are the softmax over every router output, the choice goes by score + ``correction``
     (fp32 [outputs], may be None) and the weights are the chosen scores times ``weight_scale``, not renormalised -- or, with ``renormalise``, the chosen scores over their
     sum (+ 1e-20) times ``weight_scale``.  ``groups`` = (count, keep): the outputs form ``count`` groups of as many consecutive outputs
-    and only those of the ``keep`` groups with the largest best score may be chosen."""
+    and only those of the ``keep`` groups with the largest best score may be chosen.  ``beside`` (bfloat16, few rows): the last kernel
+    launched on this stream is a product of the same ``h`` with ``early_dependents``, and this one runs beside it."""
+    _need(not beside or (h.dtype == torch.bfloat16 and n_rows <= 64), "moe_route: only bfloat16 steps of few rows are routed beside a product")
     _cuda(chosen, weight, shared_gate, h, w_router, b_router, w_shared_gate, correction)
     experts, width = w_router.shape
     _need(correction is None or (score_all and correction.dtype == torch.float32 and correction.numel() == experts
@@ -2078,7 +2080,7 @@ def moe_route(chosen: torch.Tensor, weight: torch.Tensor, shared_gate: torch.Ten
     code = _fn("moe", "tw_moe_route")(_ptr(chosen), _ptr(weight), _ptr(shared_gate), _ptr(h), c_int(h.stride(0)), _ptr(w_router),
                                       _ptr(b_router), _ptr(w_shared_gate), c_int(n_rows), c_int(width), c_int(experts), c_int(top),
                                       c_int((2 if renormalise else 1) if score_all else 0), _ptr(correction), c_float(weight_scale),
-                                      c_int(count), c_int(keep),
+                                      c_int(count), c_int(keep), c_int(1 if beside else 0),
                                       c_int(dtype_code(h.dtype)), _stream())
     _check(code, "moe_route")
 

@@ -46,3 +46,40 @@ def test_rows_of_attention_over_latents(ranks, rot, gates, interleaved, own_rows
     for a, b in zip(got, want):
         assert a == b if isinstance(a, int) else a is None and b is None or torch.equal(a, b)
     assert got[4] == (2 if write_cache else 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,width,experts,stride", [(1, 8, 2, 8), (8, 3584, 8, 3584), (148, 1032, 5, 1040), (33, 264, 64, 264)])
+@pytest.mark.parametrize("shared,scored", [(True, False), (False, True)])
+def test_router_reads_rows_where_they_lie(rows, width, experts, stride, shared, scored):
+    """Few bf16 rows on 16-byte boundaries are routed without staging them, and beside a product: the bits of rows that are staged
+    (here: rows that start off a boundary)."""
+    o = ops()
+    g = torch.Generator().manual_seed(rows + width)
+    top, dev = min(2, experts), "cuda"
+    h = torch.randn(rows, width, generator=g).bfloat16()
+    wr, ws = torch.randn(experts, width, generator=g).bfloat16().to(dev), torch.randn(width, generator=g).bfloat16().to(dev)
+    br = torch.randn(experts, generator=g).to(dev)
+    weights = torch.randn(64, width, generator=g).bfloat16().to(dev)
+
+    def run(x, beside):
+        chosen, weight = torch.empty(rows, top, dtype=torch.int32, device=dev), torch.empty(rows, top, device=dev)
+        gate = torch.empty(rows, device=dev) if shared else None
+        if beside:
+            out = torch.empty(rows, 64, dtype=torch.bfloat16, device=dev)
+            o.gemm_small_m(out, x, weights, rows, early_dependents=True)
+        o.moe_route(chosen, weight, gate, x, wr, br, ws if shared else None, rows, top, score_all=scored, beside=beside)
+        return [t for t in (chosen, weight, gate) if t is not None] + ([out] if beside else [])
+
+    def laid(offset, row):
+        x = torch.zeros(rows * row + 8, dtype=torch.bfloat16, device=dev)[offset:offset + rows * row].view(rows, row)[:, :width]
+        x.copy_(h)
+        return x
+
+    want = run(laid(1, stride + 1), False)
+    assert all(torch.equal(a, b) for a, b in zip(run(laid(0, stride), False), want))
+    if rows <= 64 and stride == width:
+        for _ in range(3):
+            got = run(laid(0, stride), True)
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+            assert torch.allclose(got[-1].float(), (h.to(dev).float() @ weights.float().T), rtol=2e-2, atol=2e-2 * width ** 0.5)
