@@ -14,9 +14,8 @@
 //
 // What bounded the rule token by token is its chain (0.23 us a token, whatever the GPU could do beside it); now it is the
 // walk's, two products and two barriers a chunk, and the reads of W and K (96 KB a chunk and block) from L2.
-// 14 heads of 128 x 128 over 2,048 tokens: 482 us token by token, 207 in chunks (65 + 95 + 47 for the launches); portions of
-// 777, 1,024 and 201 tokens: 378 and 186; 14 heads of 64 x 64: 413 and 113.  Of the walk's 95 us a third goes when nothing
-// is copied and a third when few products are made; six sums for the small products instead of one change nothing.
+// 14 heads of 128 x 128 over 2,048 tokens: 482 us token by token, 202 in chunks (59 + 96 + 47 for the launches); portions of
+// 777, 1,024 and 201 tokens: 378 and 184 (58 + 77 + 49); 14 heads of 64 x 64, 2,048 tokens: 413 and 118 (37 + 57 + 21).
 // Against 64 bits: outputs 1.8e-7 (token by token 6.5e-7), state 2.0e-7 (6.1e-7).
 //
 // Precision: q, k, v, the state and everything in between are 32-bit numbers here.  They enter a product on the tensor
@@ -269,9 +268,10 @@ __global__ void __launch_bounds__(THREADS, 2) delta_solve_kernel(DcArgs a) {
 // operand; the W and K of the chunks stand in a ring of four places, or of three where the state takes more room, the next ones on
 // their way while one is used.
 //
-// What bounds it is the chain of a chunk (its products, on mma.sync, and two barriers), 3.0 us with 16 values and 4.6 with 32, so 32 are
-// taken where 16 would give more blocks than the GPU has SMs (one fits an SM): portions of 777, 1,024 and 201 tokens, 14 heads of
-// 128 x 128, 336 blocks in two rounds and 168 whose longest start first, 87 us and 75.
+// What bounds it is the chain of a chunk (its products, on mma.sync, and two barriers), 3.0 us with 16 values and 4.5 with 32 (keys of
+// 128), and one block fits an SM: 16 unless that gives more rounds of blocks than 32 by more than this (ops.delta_walk_values).  14 heads
+// of 128 x 128: portions of 777, 1,024 and 201 tokens 89 us and 77 (336 blocks in two rounds, 168 whose longest start first), of 2,048
+// tokens and 30 single ones 97 and 147, of 1,500 and 300 tokens 74 and 111.
 template <int DV, int VT>
 __global__ void __launch_bounds__(THREADS, 1) delta_walk_kernel(DcArgs a) {
     constexpr int NT = DK / 64;                             // tiles of 8 key channels per warp
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(THREADS, 1) delta_walk_kernel(DcArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int h = blockIdx.y, v0 = blockIdx.x * V;
     int s = blockIdx.z;
-    if (a.n_seqs <= 32) {                                   // the longest request's blocks start first
+    if (a.n_seqs <= 32) {                                   // the longest request's blocks start first (ops.DELTA_WALK_SORTED)
         const int mine = lane < a.n_seqs ? a.seq_q_len[lane] : -1;
         int rank = 0;
         for (int r = 0; r < a.n_seqs; ++r) {
@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(THREADS, 2) delta_outputs_kernel(DcArgs a) {
 }
 
 template <int DV>
-int launch_delta(const DcArgs& a, int max_q_len, cudaStream_t stream) {
+int launch_delta(const DcArgs& a, int max_q_len, int walk_values, cudaStream_t stream) {
     constexpr size_t terms = (size_t)3 * L * RS * 2;
     constexpr size_t smem1 = terms + (size_t)L * (L + 4) * 4, smem3 = 2 * terms;
     constexpr auto smem2 = [](int vt) constexpr { return (vt == 1 ? 4 : 3) * terms + (size_t)3 * 16 * vt * (DK + 8 + MS) * 2; };
@@ -665,8 +665,7 @@ int launch_delta(const DcArgs& a, int max_q_len, cudaStream_t stream) {
     const dim3 grid((max_q_len + L - 1) / L, a.H, a.n_seqs);
     int code = tw_launch(delta_solve_kernel<DV>, grid, dim3(THREADS), smem1, stream, 1, a);
     if (code) return code;
-    // (148 SMs: the same line on any part of the kind)
-    if ((long long)DV / 16 * a.H * a.n_seqs > 148)
+    if (walk_values == 32)
         code = tw_launch(delta_walk_kernel<DV, 2>, dim3(DV / 32, a.H, a.n_seqs), dim3(THREADS), smem2(2), stream, 1, a);
     else
         code = tw_launch(delta_walk_kernel<DV, 1>, dim3(DV / 16, a.H, a.n_seqs), dim3(THREADS), smem2(1), stream, 1, a);
@@ -679,17 +678,18 @@ int launch_delta(const DcArgs& a, int max_q_len, cudaStream_t stream) {
 // Requests with at least `min_len` rows (the others are left to tw_linear_recurrence).  Operands as tw_linear_recurrence has them
 // for the delta rule with a decay per head: q, k, v fp32 rows on 16-byte boundaries; Dk as compiled (64 or 128), Dv 64 or 128.
 // `scratch`: for each of `chunks` (at least the sum of ceil(rows / 64) over those requests)
-// H (Dk Dv + 64 Dv + 96 Dk + 128) + H / qk_group x 96 Dk floats.
+// H (Dk Dv + 64 Dv + 96 Dk + 128) + H / qk_group x 96 Dk floats.  `walk_values`: values a block of the walk takes, 16 or 32; the bits
+// do not depend on it.
 TW_EXPORT int tw_delta_chunks(float* out, const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
                               const float* pre, int pre_stride, const float* write, int write_stride, const float* rate_log,
                               const float* dt_bias, float q_scale, float k_scale, float* state, long long state_stride, const int* seq_slot,
                               const int* seq_q_start, const int* seq_q_len, int n_seqs, int H, int Dk, int Dv, int qk_group, int min_len,
-                              int max_q_len, int write_state, float* scratch, int chunks, cudaStream_t stream) {
+                              int max_q_len, int write_state, int walk_values, float* scratch, int chunks, cudaStream_t stream) {
     if (n_seqs <= 0 || H <= 0 || max_q_len <= 0) return 0;
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (Dk != DK || (Dk != 64 && Dk != 128) || (Dv != 64 && Dv != 128) || min_len < 1 || qk_group <= 0 || H % qk_group || (q_stride & 3)
         || (k_stride & 3) || !a16(q) || !a16(k) || !a16(scratch) || !pre || !write || !rate_log || !dt_bias || chunks < 1
-        || (reinterpret_cast<uintptr_t>(out) & 7) || n_seqs > 65535 || H > 65535)
+        || (reinterpret_cast<uintptr_t>(out) & 7) || n_seqs > 65535 || H > 65535 || (walk_values != 16 && walk_values != 32))
         return (int)cudaErrorInvalidValue;
     DcArgs a;
     a.out = out; a.q = q; a.k = k; a.v = v; a.q_stride = q_stride; a.k_stride = k_stride; a.v_stride = v_stride;
@@ -704,7 +704,7 @@ TW_EXPORT int tw_delta_chunks(float* out, const float* q, int q_stride, const fl
     a.decay = (float2*)(a.w + n * 3 * L * Dk);
     a.keys = (bf16*)(a.decay + n * L);
 #if TW_DK == 64 || TW_DK == 128
-    return Dv == 128 ? launch_delta<128>(a, max_q_len, stream) : launch_delta<64>(a, max_q_len, stream);
+    return Dv == 128 ? launch_delta<128>(a, max_q_len, walk_values, stream) : launch_delta<64>(a, max_q_len, walk_values, stream);
 #else
     return (int)cudaErrorInvalidValue;
 #endif

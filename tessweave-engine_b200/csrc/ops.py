@@ -8,7 +8,9 @@ they order with library matrix products and can be captured in CUDA graphs.
 """
 from __future__ import annotations
 
+import bisect
 import ctypes
+import functools
 from ctypes import c_void_p, c_int, c_float, c_long
 from dataclasses import dataclass
 
@@ -1839,13 +1841,56 @@ def delta_chunk_floats(heads: int, qk_group: int, key_dim: int, value_dim: int) 
     return heads * (key_dim * value_dim + RECURRENCE_CHUNK * (value_dim + 2) + terms) + heads // qk_group * terms
 
 
+# What a chunk takes a block of the walk that has 16 values of a head, and one that has 32, by the key size; and what a block takes besides.
+# us: 14 heads of 128 x 128, portions of 512, 1,024 and 2,048 tokens (8, 16, 32 chunks) 26.6, 49.7, 96.2 and 39.2, 74.9, 146.6; of 64 x
+# 64, 1,024 and 2,048 tokens 30.1, 57.4 and 43.4, 83.9.  The value size does not matter (128 x 64: 48.9, 95.1 and 74.1, 145.1).
+DELTA_WALK_CHUNK_US = {64: (1.71, 2.54), 128: (2.95, 4.48)}
+DELTA_WALK_START_US = 3.2
+DELTA_WALK_SORTED = 32                  # requests of a step whose blocks start in the order of their lengths, else in that of the step
+
+
+@functools.lru_cache(maxsize=256)
+def _blocks_end(lengths: tuple[float, ...], each: int) -> float:
+    """When the last block ends: ``each`` blocks of every length, in this order, each on the SM that is free first."""
+    free = [(0.0, _SM_COUNT)]                   # (from when, how many SMs), the earliest first
+    for length in lengths:
+        left = each
+        while left:
+            at, count = free.pop(0)
+            taken = min(count, left)
+            if taken < count:
+                free.insert(0, (at, count - taken))
+            bisect.insort(free, (at + length, taken))
+            left -= taken
+    return free[-1][0]
+
+
+def delta_walk_values(q_lens: list[int], heads: int, key_dim: int, value_dim: int) -> int:
+    """How many values of a head a block of the delta rule's walk takes in a step of requests with these row counts, 16 or 32.  A block
+    fits an SM alone.  With 32 there are half as many and each takes half as long again, which pays where blocks of 16 values
+    would come in more rounds than those of 32; so both are laid out over the SMs, the longest first, as the launch lays them out.
+    us of the walk with 16 and 32 values, 14 heads of 128 x 128: 2,048 tokens 96 and 147, beside one or thirty single tokens 97 and 146,
+    1,900 + 60 + 80 tokens 91 and 138, 1,500 + 300 74 and 111, 1,200 + 400 + 200 81 and 89, 3 x 600 94 and 94; 777 + 1,024 + 201 89 and 77,
+    1,000 + 1,000 98 and 76, 4 x 512 101 and 78, 8 x 1,024 335 and 293; 14 heads of 64 x 64: 2 x 1,024 31 and 44, 4 x 512 32 and 24."""
+    chunks = [-(-m // RECURRENCE_CHUNK) for m in q_lens if m >= RECURRENCE_CHUNK_MIN_ROWS]
+    blocks = heads * value_dim // 16            # of a request
+    if len(chunks) * blocks <= _SM_COUNT:
+        return 16
+    if len(q_lens) <= DELTA_WALK_SORTED:
+        chunks.sort(reverse=True)
+    narrow, wide = (_blocks_end(tuple(DELTA_WALK_START_US + c * us for c in chunks), blocks // n)
+                    for n, us in zip((1, 2), DELTA_WALK_CHUNK_US[key_dim]))
+    return 32 if wide < narrow else 16
+
+
 def delta_chunks(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, seq_slot: torch.Tensor,
                  seq_q_start: torch.Tensor, seq_q_len: torch.Tensor, n_seqs: int, heads: int, key_dim: int, value_dim: int,
                  max_q_len: int, scratch: torch.Tensor, write_state: bool, pre: torch.Tensor, p0: torch.Tensor, p1: torch.Tensor,
-                 write_pre: torch.Tensor, qk_group: int = 1, q_scale: float = 1.0, k_scale: float = 1.0) -> None:
+                 write_pre: torch.Tensor, qk_group: int = 1, q_scale: float = 1.0, k_scale: float = 1.0, walk_values: int = 16) -> None:
     """``linear_recurrence`` with the delta rule (a decay per head) of the requests that bring ``RECURRENCE_CHUNK_MIN_ROWS``
     rows or more, in chunks (csrc/delta_chunks.cu): same operands and state.  The other requests are left alone.  ``scratch``:
-    ``delta_chunk_floats`` fp32 numbers for each of ``recurrence_chunk_count`` chunks."""
+    ``delta_chunk_floats`` fp32 numbers for each of ``recurrence_chunk_count`` chunks.  ``walk_values``: see ``delta_walk_values``; the
+    bits do not depend on it."""
     _cuda(out, q, k, v, state, seq_slot, seq_q_start, seq_q_len, pre, p0, p1, write_pre, scratch)
     _need(delta_chunks_supported(q, k, key_dim, value_dim, False), "recurrence: the delta rule's chunk kernels do not take these sizes or rows")
     _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == heads * value_dim, "recurrence: out must be fp32 [rows, H * Dv]")
@@ -1862,7 +1907,7 @@ def delta_chunks(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.T
         _ptr(write_pre), c_int(write_pre.stride(0)), _ptr(p0), _ptr(p1), c_float(q_scale), c_float(k_scale), _ptr(state),
         ctypes.c_longlong(state.stride(0)), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), c_int(n_seqs), c_int(heads), c_int(key_dim),
         c_int(value_dim), c_int(qk_group), c_int(RECURRENCE_CHUNK_MIN_ROWS), c_int(max_q_len), c_int(1 if write_state else 0),
-        _ptr(scratch), c_int(chunks), _stream())
+        c_int(walk_values), _ptr(scratch), c_int(chunks), _stream())
     _check(code, "delta_chunks")
 
 

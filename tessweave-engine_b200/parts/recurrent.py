@@ -122,6 +122,7 @@ class MatrixStateMixer(Mixer):
             else:
                 if delta:
                     ops.delta_chunks(raw, q, k, v, cache.state, *common[2:], longest, scratch, write_state,
+                                     walk_values=ops.delta_walk_values(ctx.host_q_len, self.n_heads, self.key_dim, self.value_dim),
                                      **{name: value for name, value in rule_args.items() if name != "channel_decay"})
                 else:
                     ops.recurrence_chunks(self.rule, raw, den, q, k, v, *common, longest, *scratch, write_state, **rule_args)

@@ -1,4 +1,4 @@
-"""The walk of the gated delta rule's chunks with many requests: 32 values a block, the longest request first."""
+"""The walk of the gated delta rule's chunks with many requests: 16 or 32 values a block, the longest request first."""
 import pytest
 import torch
 
@@ -6,9 +6,10 @@ import torch
 @pytest.mark.gpu
 @pytest.mark.parametrize("heads,dk,dv,lens", [(2, 64, 64, [33, 64, 65, 64, 7, 129] * 6), (2, 128, 128, [64, 200, 64, 31, 130] * 5),
                                               (4, 64, 128, [65, 65, 65, 190, 32, 65])])
-def test_requests_together_and_alone(heads, dk, dv, lens):
-    """A step whose blocks take 32 values (more than a warp's 32 requests, requests of one length, short ones left to the token kernel)
-    gives the bits of every request alone, whose blocks take 16."""
+@pytest.mark.parametrize("values", [16, 32])
+def test_requests_together_and_alone(heads, dk, dv, lens, values):
+    """A step whose blocks take 16 or 32 values (more than a warp's 32 requests, requests of one length, short ones left to the token
+    kernel) gives the bits of every request alone, whose blocks take 16."""
     from tessweave_engine_b200.csrc import ops
     g = torch.Generator().manual_seed(heads * dk)
     n, half, count = sum(lens), heads // 2, len(lens)
@@ -22,7 +23,7 @@ def test_requests_together_and_alone(heads, dk, dv, lens):
     starts = [sum(lens[:i]) for i in range(count)]
     slots = torch.randperm(count, generator=g).tolist()
 
-    def run(st, which):
+    def run(st, which, values=16):
         rows = slice(starts[which[0]], starts[which[-1]] + lens[which[-1]])
         m = rows.stop - rows.start
         out = torch.full((m, heads * dv), -7.0, device="cuda")
@@ -30,11 +31,11 @@ def test_requests_together_and_alone(heads, dk, dv, lens):
         scratch = torch.full((chunks * ops.delta_chunk_floats(heads, 2, dk, dv),), float("nan"), device="cuda")
         ops.delta_chunks(out, q[rows], k[rows], v[rows], st, i32([slots[i] for i in which]), i32([starts[i] - rows.start for i in which]),
                          i32([lens[i] for i in which]), len(which), heads, dk, dv, max(lens[i] for i in which), scratch, True,
-                         pre=pre[rows], write_pre=write[rows], **args)
+                         pre=pre[rows], write_pre=write[rows], walk_values=values, **args)
         return out
 
     together, alone = state.clone(), state.clone()
-    got = run(together, list(range(count)))
+    got = run(together, list(range(count)), values)
     left = lambda m: torch.full((m, heads * dv), -7.0, device="cuda")          # noqa: E731
     want = torch.cat([run(alone, [i]) if m >= 32 else left(m) for i, m in enumerate(lens)])
     assert torch.equal(got, want) and torch.equal(together, alone)

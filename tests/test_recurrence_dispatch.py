@@ -85,3 +85,35 @@ def test_every_key_size_of_the_chunks_is_built_ahead():
     rows = torch.zeros(4, 256)
     sizes = [d for d in range(1, 257) if ops.delta_chunks_supported(rows, rows, d, 64, False)]
     assert [v["TW_DK"] for v in default_variants("delta_chunks")] == sizes
+
+
+@pytest.mark.parametrize("key_dim", [64, 128])
+@pytest.mark.parametrize("heads,value_dim", [(14, 128), (14, 64), (8, 128), (6, 64), (32, 128)])
+def test_width_of_the_delta_rules_walk(key_dim, heads, value_dim):
+    """A block of the walk takes 32 values only where the step's last block ends earlier so, laid out block by block over the SMs; in
+    particular never where blocks of 16 values all run at once, whatever else the step brings."""
+    def ends(lens, values):
+        free = [0.0] * 148
+        for m in sorted(lens, reverse=True) if len(lens) <= 32 else lens:
+            for _ in range(heads * value_dim // values if m >= ops.RECURRENCE_CHUNK_MIN_ROWS else 0):
+                at = free.index(min(free))
+                free[at] += ops.DELTA_WALK_START_US + ops.DELTA_WALK_CHUNK_US[key_dim][values // 32] * -(-m // 64)
+        return max(free)
+
+    for lens in ([2048], [2048, 1], [2048] + [1] * 30, [1] * 40 + [2048], [777, 1024, 201], [1900, 60, 80], [1500, 300], [1200, 400, 200], [1000, 1000],
+                 [31, 600, 600, 600], [512] * 4, [64] * 20 + [800], [800] + [33] * 40, [1024] * 8):
+        narrow, wide = ends(lens, 16), ends(lens, 32)
+        taken = ops.delta_walk_values(lens, heads, key_dim, value_dim)
+        assert abs(ends(lens, taken) - min(narrow, wide)) < 1e-6, lens
+        if sum(m >= ops.RECURRENCE_CHUNK_MIN_ROWS for m in lens) * heads * value_dim // 16 <= 148:
+            assert taken == 16
+
+
+def test_a_step_says_how_wide_its_walk_is(monkeypatch):
+    """(14 heads of 128 x 128 would take 32 values for the portions; the heads of the mixer here and its one long portion take 16)"""
+    assert ops.delta_walk_values([777, 1024, 201], 14, 128, 128) == 32 and ops.delta_walk_values([2048] + [1] * 30, 14, 128, 128) == 16
+    seen = []
+    with monkeypatch.context() as m:
+        m.setattr(ops, "delta_walk_values", lambda lens, *sizes: seen.append((lens, *sizes)) or 16)
+        recur("gated_delta", torch.bfloat16, [700, 1, 64], m)
+    assert seen == [([700, 1, 64], HEADS, DIM, DIM)]
