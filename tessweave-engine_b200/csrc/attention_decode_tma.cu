@@ -145,7 +145,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                        int num_pages, int window, float scale_log2e, int nsplit, int nstages,
                        float* __restrict__ partial_o, float* __restrict__ partial_ml, int* __restrict__ counters,
                        int* status, const FusedQkv fq, const float* __restrict__ gate, const float* __restrict__ sink,
-                       const int shared_kv, const int beside) {
+                       const int shared_kv, int* ready) {
     static_assert(!FUSED || SAME_DIMS, "the fused form packs q, k and v as heads of one size");
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[MAX_STAGES];
@@ -166,12 +166,15 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     TW_TIMELINE_SCOPE(TW_K_ATTN_DECODE);
     // The request arrays and the block table are written before the step's first kernel starts, not by the
     // kernel before this one: they are read before the wait for that kernel.
-    // `beside`: the kernel before this one is the prompts' attention of the same step.  It lets this kernel start once it has
+    // With `ready` the kernel before this one is the prompts' attention of the same step.  It lets this kernel start once it has
     // seen all that it reads itself (the rows of q and the cache), and neither reads what the other writes: only one block
     // waits for it, at its end, so that what follows comes after both.
+    const bool beside = ready != nullptr;
     const bool waits_last = beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+    if (beside) tw_wait_unless_ready(ready);
     if (seq_q_len[s] != 1) {
-        if (!beside || waits_last) tw_grid_wait();             // a block never finishes before the kernel before this one has
+        if (waits_last) tw_wait_and_clear(ready, threadIdx.x == 0);
+        else if (!beside) tw_grid_wait();                      // a block never finishes before the kernel before this one has
         return;
     }
     if constexpr (CLUSTER) cg::this_cluster().barrier_arrive();      // (waited for before the first store into a neighbour's memory)
@@ -274,7 +277,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 tw_prefetch_l2_share(fq.next_weights, fq.next_bytes);
             }
         }
-        if ((FUSED && fq.k_cache) || waits_last) tw_grid_wait();
+        if (waits_last) tw_wait_and_clear(ready, warp == CWARPS && lane == 0);
+        else if (FUSED && fq.k_cache) tw_grid_wait();
         return;
     } else {
         // ---- consumers
@@ -345,7 +349,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             for (int idx = threadIdx.x; idx < HEADS * (D / 8); idx += CTHREADS) {
                 const int head = idx / (D / 8), ch = idx - head * (D / 8);
                 uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (head < nheads) v = *reinterpret_cast<const uint4*>(q + (size_t)n * q_stride + (size_t)(kvh * G + h0 + head) * D + ch * 8);
+                // (past L1 and never ahead of the wait, whichever form this takes)
+                if (head < nheads)
+                    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                 : "l"(q + (size_t)n * q_stride + (size_t)(kvh * G + h0 + head) * D + ch * 8) : "memory");
                 *reinterpret_cast<uint4*>(s_q + head * D + ch * 8) = v;
             }
         }
@@ -727,8 +734,9 @@ TW_EXPORT int tw_attn_decode_tma_supported(int page_size) {
 // `scratch` and `counters` as for tw_attn_decode; they are used when the slices do not fit a cluster.
 // `gate` (fp32 [rows][Hq] or null): head h's output of a row is multiplied by its entry.  `sink` (fp32 [Hq] or null, with `q`
 // only): exp(sink[h]) joins head h's denominator.  v_cache may be k_cache (with `q` only): a position's value is its key, which
-// is copied once and read as both.  `flags`: 1 merges slices in scratch memory, 2 (with `q` only) runs beside the kernel launched
-// before, which must be the prompts' attention of the same step (tw_attn_prefill_tc5 with skip_single).
+// is copied once and read as both.  `flags`: 1 merges slices in scratch memory.  `ready` (or null; with `q` only): the word that the
+// kernel launched before, the prompts' attention of the same step (tw_attn_prefill_tc5 with skip_single), was given; this one runs
+// beside it then.
 TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q_stride, const float* partial, int nslices,
                                  long long slice_stride, const void* dense, int dense_stride, const float* bias,
                                  const float* inv_freq, int write_cache, const int* seq_q_start, const int* seq_q_len,
@@ -736,7 +744,7 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
                                  void* k_cache, void* v_cache, int n_seqs, int Hq, int Hkv, int page_size, int num_pages,
                                  int window, float scale, int nsplit, int nstages, int flags, float* scratch, int* counters,
                                  int* status, const void* next_weights, long long next_bytes, const float* gate,
-                                 const float* sink, cudaStream_t stream) {
+                                 const float* sink, int* ready, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     const bool fused = partial || dense;
     const bool shared_kv = k_cache == v_cache;
@@ -782,7 +790,7 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
     const size_t smem = smem_bytes(nstages, shared_kv);
     const float scale_log2e = scale * 1.4426950408889634f;
     const bool cluster = nsplit > 1 && !(flags & 1) && cluster_fits(nsplit, nstages, shared_kv);
-    const bool beside = (flags & 2) != 0;
+    const bool beside = ready != nullptr;
     if (beside && fused) return (int)cudaErrorInvalidValue;
 #define TW_DECODE_TMA_LAUNCH(CL, FU)                                                                                   \
     do {                                                                                                               \
@@ -791,7 +799,7 @@ TW_EXPORT int tw_attn_decode_tma(void* out, int out_stride, const void* q, int q
             return tw_launch<decltype(how)::value>(attn_decode_tma_kernel<CL, FU>, grid, dim3(THREADS), smem, stream, CL ? nsplit : 1, mk, mv,    \
                              (bf16*)out, out_stride, (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, \
                              block_table, table_stride, Hq, Hkv, page_size, num_pages, window, scale_log2e, nsplit, nstages, \
-                             partial_o, partial_ml, counters, status, fq, gate, sink, (int)shared_kv, (int)beside);    \
+                             partial_o, partial_ml, counters, status, fq, gate, sink, (int)shared_kv, ready);          \
         };                                                                                                             \
         return beside ? launch(std::integral_constant<int, TW_OVERLAPS>()) : launch(std::integral_constant<int, TW_READS_AHEAD>()); \
     } while (0)

@@ -98,12 +98,15 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                         const int* __restrict__ seq_kv_len, const int* __restrict__ seq_slot,
                         const int* __restrict__ block_table, int table_stride, int Hq, int Hkv, int page_size,
                         int num_pages, int window, float scale_log2e, int skip_single, const float* __restrict__ gate,
-                        int* status, int n_seqs) {
+                        int* status, int n_seqs, int* word) {
     extern __shared__ unsigned char smem_raw[];
     TW_TIMELINE_SCOPE(TW_K_ATTN_PREFILL);
     tw_grid_wait();
     // The decode attention of the same step writes other rows: it may run beside this kernel, on the SMs that have no block of it.
-    if (skip_single) tw_launch_dependents_now();
+    if (skip_single) {
+        tw_say_ready(word);
+        tw_launch_dependents_now();
+    }
     if (threadIdx.x == 0) TW_TRACE_AT(11, 0, 5);
     TW_TIMELINE_MARK();
     // Blocks start in the order of blockIdx.x, and a block's work grows with the position of its rows: x counts
@@ -582,12 +585,14 @@ TW_EXPORT int tw_attn_prefill_tc5_supported(int page_size) {
 // Attention for the requests of the batch that bring several tokens (with skip_single, requests
 // with one token are left to the decode kernel).  q [tokens, Hq * D] and out [tokens, Hq * D] are
 // bf16 with 16-byte aligned rows; the cache is [pages, Hkv, page_size, D] bf16 (values and out: heads of DV).  `row_tiles`: the sum of
-// ceil(rows x Hq / Hkv / 256) over the requests that are served, where the caller knows it, else 0.
+// ceil(rows x Hq / Hkv / 256) over the requests that are served, where the caller knows it, else 0.  `ready` (or null; with
+// skip_single): a word that tw_attn_decode_tma is given next, see tw_say_ready.
 TW_EXPORT int tw_attn_prefill_tc5(void* out, int out_stride, const void* q, int q_stride, const int* seq_q_start,
                                   const int* seq_q_len, const int* seq_kv_len, const int* seq_slot,
                                   const int* block_table, int table_stride, const void* k_cache, const void* v_cache,
                                   int n_seqs, int max_q_len, int Hq, int Hkv, int page_size, int num_pages, int window,
-                                  float scale, int skip_single, const float* gate, int row_tiles, int* status, cudaStream_t stream) {
+                                  float scale, int skip_single, const float* gate, int row_tiles, int* status, int* ready,
+                                  cudaStream_t stream) {
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
     if (Hkv <= 0 || Hq % Hkv || !tw_attn_prefill_tc5_supported(page_size) || scale <= 0.f) return (int)cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(q) & 15) || (out_stride & 7) || (q_stride & 7) ||
@@ -616,5 +621,5 @@ TW_EXPORT int tw_attn_prefill_tc5(void* out, int out_stride, const void* q, int 
     dim3 grid((unsigned)blocks, counted ? 1 : n_seqs);
     return tw_launch(attn_prefill_tc5_kernel, grid, dim3(THREADS), (size_t)SMEM, stream, 1, mk, mv, (bf16*)out, out_stride,
                      (const bf16*)q, q_stride, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table, table_stride,
-                     Hq, Hkv, page_size, num_pages, window, scale * 1.4426950408889634f, skip_single, gate, status, counted ? n_seqs : 0);
+                     Hq, Hkv, page_size, num_pages, window, scale * 1.4426950408889634f, skip_single, gate, status, counted ? n_seqs : 0, ready);
 }

@@ -152,15 +152,22 @@ TW_EXPORT int tw_timeline_set(void* buffer) {
 #endif
 
 // ---------------------------------------------------------------------------------------
-// Programmatic dependent launch.  Every kernel of this engine starts with tw_grid_wait():
-// nothing it reads that an earlier kernel wrote, and nothing it writes, is touched before.
-// Kernels are launched with the programmatic-serialization attribute, so inside a CUDA graph
-// the next kernel's launch overlaps the tail of the one before (measured on B200: 2 % off a
-// decode step).  Letting the next kernel become resident even earlier with an explicit
-// griddepcontrol.launch_dependents -- at the top of short kernels or after the main loop of long
-// ones -- made the step slower (up to 8 %), so tw_grid_launch_dependents() compiles to nothing
-// unless TW_PDL_TRIGGERS is defined.  TESSWEAVE_PDL=0 in the environment launches every kernel
-// the ordinary way.
+// Programmatic dependent launch.  Kernels captured into a CUDA graph, and large plain launches (see tw_launch), carry the
+// programmatic-serialization attribute: the next kernel's launch overlaps the tail of the one before (measured on B200: 2 %
+// off a decode step).  What this rests on: a kernel starts with tw_grid_wait(), and before it touches nothing that an earlier
+// kernel wrote and writes nothing.  Three kinds of kernel do otherwise, each under a condition of its own:
+//   * those launched with TW_READS_AHEAD read, before they wait, what stood before their step's first kernel (request arrays, block
+//     tables, weights).  A graph's first kernel comes after all of that; plain launches of them carry no attribute.
+//   * those that run beside the kernel before them (attn_decode_tma_kernel and moe_route_kernel, with a `ready` word) pass
+//     tw_wait_unless_ready() instead: see there.
+//   * whichever of the two it is, a block that leaves early still waits first where nothing else makes sure that its kernel
+//     ends after the one before.
+// A new kernel launched by tw_launch's default that reads ahead of its wait is a race on large plain launches.
+//
+// Letting the next kernel become resident even earlier with an explicit griddepcontrol.launch_dependents -- at the top of
+// short kernels or after the main loop of long ones -- made the step slower (up to 8 %), so tw_grid_launch_dependents()
+// compiles to nothing unless TW_PDL_TRIGGERS is defined.  TESSWEAVE_PDL=0 in the environment launches every kernel the
+// ordinary way.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void tw_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void tw_grid_launch_dependents() {
@@ -172,6 +179,30 @@ __device__ __forceinline__ void tw_grid_launch_dependents_late() { tw_grid_launc
 // The exception, measured to pay: kernels whose successor is small (or whose own blocks are few) let it
 // become resident at once.  Used by the clustered norm and, on request, by the small-M product.
 __device__ __forceinline__ void tw_launch_dependents_now() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Two kernels side by side, the second reading what the first one read.  That the second starts only once every block of the first has
+// triggered, behind its own wait, orders them in time; what memory looks like is only promised behind a wait.  So the first
+// (behind its wait, before its trigger, one thread of its last block, the one that triggers last) says in a word of memory that
+// everything before it is there, and a warp of the second that finds the word set goes on: release and acquire order it behind
+// all that the first kernel's wait had made visible, and the fence extends that to copies by TMA.  A warp that does not find it set
+// waits like any other, so a second kernel launched behind anything else is ordinary.  One block of the second waits for the
+// first at its end, so that what follows comes after both, and clears the word.
+__device__ __forceinline__ void tw_say_ready(int* ready) {
+    if (ready && threadIdx.x == 0 && blockIdx.x + 1 == gridDim.x && blockIdx.y + 1 == gridDim.y && blockIdx.z + 1 == gridDim.z)
+        asm volatile("st.release.gpu.global.s32 [%0], 1;" ::"l"(ready) : "memory");
+}
+// (a whole warp)
+__device__ __forceinline__ void tw_wait_unless_ready(const int* ready) {
+    int set;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(set) : "l"(ready) : "memory");
+    if (__all_sync(0xffffffffu, set != 0)) asm volatile("fence.proxy.async.global;" ::: "memory");
+    else tw_grid_wait();
+}
+// (the threads that wait at the end of the second kernel's one block; `one` of them clears the word)
+__device__ __forceinline__ void tw_wait_and_clear(int* ready, bool one) {
+    tw_grid_wait();
+    if (one) *(volatile int*)ready = 0;
+}
 
 // A hint to bring this block's share of [ptr, ptr + bytes) into L2: what the next kernel will stream (its
 // weights), asked for while this kernel's last blocks finish and the memory system has little to do.  One
@@ -226,7 +257,7 @@ static inline int tw_allow_shared() {
 // attention 160.8 and 157.7, 32-bit attention 320.5 and 316.5).  Smaller ones belong to steps that the host bounds, and there
 // the attribute costs 1 to 2 % of a step.  TW_READS_AHEAD: the kernel reads some of its step's inputs before it waits, which is
 // sound where they were there before the graph's first kernel, so it waits for everything before it on plain launches.
-// TW_OVERLAPS: with the attribute whatever its size.
+// TW_OVERLAPS: with the attribute whatever its size (kernels that run beside the one before).
 #define TW_PDL_THREADS (148 * 128)
 enum : int { TW_BY_SIZE = 0, TW_READS_AHEAD = 1, TW_OVERLAPS = 2 };
 template <int HOW = TW_BY_SIZE, typename... KArgs, typename... Args>

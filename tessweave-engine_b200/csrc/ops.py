@@ -71,6 +71,11 @@ def _cuda(*tensors: torch.Tensor | None) -> None:
             raise KernelError("kernel operands must live on a CUDA device; this engine has no CPU path")
 
 
+def _ready_check(ready: torch.Tensor | None) -> None:
+    _need(ready is None or (ready.is_cuda and ready.dtype == torch.int32 and ready.numel() >= 1), "the word between two kernels that run beside "
+          "each other must be int32 on the GPU")
+
+
 def _check(code: int, what: str) -> None:
     if code != 0:
         raise KernelError(f"{what}: CUDA error {code} at launch "
@@ -1192,7 +1197,7 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
                          block_table, k_pages, v_pages, n_seqs, n_q_heads, n_kv_heads, head_dim, window, scale, nsplit,
                          scratch, counters, status, merge_in_scratch: bool = False, prefetch: torch.Tensor | None = None,
                          stages: int = 0, gate: torch.Tensor | None = None, sink: torch.Tensor | None = None,
-                         beside_prompts: bool = False) -> None:
+                         beside_prompts: bool = False, ready: torch.Tensor | None = None) -> None:
     """Split-KV attention for the requests of the batch that bring one token, keys and values brought in by TMA.
     Either ``q`` (bf16 [rows, Hq D], 16-byte aligned rows) or ``source`` -- the step's untouched q/k/v product, a
     ``SplitSum`` or a bf16 [rows, (Hq + 2 Hkv) D] tensor, which the kernel biases, rotates and (``write_cache``)
@@ -1200,8 +1205,10 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
     ``stages`` is the depth of a block's ring of 64-key tiles (0: chosen from the size of the launch).  ``window`` and
     ``gate``: as for ``attention_decode``; with ``q`` the values may have another size than the keys, or be the keys (the same
     pages), and ``sink`` (fp32 [Hq]) may join the denominator.  ``beside_prompts`` (with ``q``): the last kernel launched on this
-    stream is ``attention_prefill_tcgen05`` of the same step with ``skip_single``, and this one runs beside it."""
+    stream is ``attention_prefill_tcgen05`` of the same step with ``skip_single``, and this one runs beside it if both were given
+    ``ready`` (int32 [1], zero and zero again afterwards), through which the first tells this one that all that both read is there."""
     _need(source is None or not beside_prompts, "attention_decode_tma: only with q given can it run beside the prompts' attention")
+    _ready_check(ready)
     width = (n_q_heads + 2 * n_kv_heads) * head_dim
     partial = dense = None
     nslices = slice_stride = dense_stride = 0
@@ -1253,17 +1260,21 @@ def attention_decode_tma(out, q, source, bias, inv_freq, write_cache, seq_q_star
         c_int(1 if write_cache else 0), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(seq_slot),
         _ptr(block_table), c_int(block_table.shape[1]), _ptr(k_pages), _ptr(v_pages), c_int(n_seqs), c_int(n_q_heads),
         c_int(n_kv_heads), c_int(k_pages.shape[2]), c_int(k_pages.shape[0]), c_int(window), c_float(scale), c_int(nsplit),
-        c_int(stages), c_int((1 if merge_in_scratch else 0) + (2 if beside_prompts else 0)), _ptr(scratch), _ptr(counters), _ptr(status), _ptr(prefetch),
-        ctypes.c_longlong(prefetch.numel() * prefetch.element_size() if prefetch is not None else 0), _ptr(gate), _ptr(sink), _stream())
+        c_int(stages), c_int(1 if merge_in_scratch else 0), _ptr(scratch), _ptr(counters), _ptr(status), _ptr(prefetch),
+        ctypes.c_longlong(prefetch.numel() * prefetch.element_size() if prefetch is not None else 0), _ptr(gate), _ptr(sink),
+        _ptr(ready if beside_prompts else None), _stream())
     _check(code, "attention_decode_tma")
 
 
 def attention_prefill_tcgen05(out, q, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table, k_pages, v_pages, n_seqs,
                               max_q_len, n_q_heads, n_kv_heads, head_dim, window, scale, skip_single, status,
-                              gate: torch.Tensor | None = None, host_q_len: list[int] | None = None) -> None:
+                              gate: torch.Tensor | None = None, host_q_len: list[int] | None = None,
+                              ready: torch.Tensor | None = None) -> None:
     """The same as ``attention_prefill`` on the 5th-generation tensor cores (TMA, tcgen05.mma,
     accumulators in tensor memory), for the shapes ``tcgen05_attention_supported`` names and a positive scale.  ``host_q_len``
-    (the requests' row counts, where the host knows them): the launch then has no blocks but those with rows to serve."""
+    (the requests' row counts, where the host knows them): the launch then has no blocks but those with rows to serve.
+    ``ready`` (with ``skip_single``): for the ``attention_decode_tma`` that is launched next and runs beside this kernel."""
+    _ready_check(ready)
     _cuda(out, q, seq_q_start, seq_q_len, seq_kv_len, seq_slot, block_table, k_pages, v_pages, status, gate)
     _gate_check(gate, 0, n_q_heads)
     _attn_common_checks(out, q, block_table, k_pages, v_pages, n_q_heads, n_kv_heads, head_dim)
@@ -1280,7 +1291,7 @@ def attention_prefill_tcgen05(out, q, seq_q_start, seq_q_len, seq_kv_len, seq_sl
         _ptr(seq_kv_len), _ptr(seq_slot), _ptr(block_table), c_int(block_table.shape[1]), _ptr(k_pages), _ptr(v_pages),
         c_int(n_seqs), c_int(max_q_len), c_int(n_q_heads), c_int(n_kv_heads), c_int(k_pages.shape[2]),
         c_int(k_pages.shape[0]), c_int(window), c_float(scale), c_int(1 if skip_single else 0), _ptr(gate), c_int(row_tiles),
-        _ptr(status), _stream())
+        _ptr(status), _ptr(ready), _stream())
     _check(code, "attention_prefill_tcgen05")
 
 

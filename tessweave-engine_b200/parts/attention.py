@@ -35,12 +35,15 @@ class PagedSoftmaxMixer(Mixer):
     def _prefetch_plan(self, ctx: StepContext):
         return None, None
 
+    def _decode_tma(self, cache: PagedView) -> bool:
+        # (a table by distance is what the kernel fed by TMA does not know.  8 requests of 4,096 cached rows of 256 that are keys and
+        # values of 28 heads: 28.5 us with keys loaded through registers, 16.6 through TMA)
+        return self.bias_rows is None and ops.decode_tma_supported(self.runtime.dtype, self.head_dim, cache.page_size, self.v_dim)
+
     def _decode_launch(self, ctx: StepContext, cache: PagedView) -> tuple[bool, int, int]:
         """(fed by TMA?, slices per request, blocks) of the decode attention this step will launch."""
         group = self.n_heads // self.n_kv_heads
-        # (a table by distance is what the kernel fed by TMA does not know.  8 requests of 4,096 cached rows of 256 that are keys and
-        # values of 28 heads: 28.5 us with keys loaded through registers, 16.6 through TMA)
-        tma = self.bias_rows is None and ops.decode_tma_supported(self.runtime.dtype, self.head_dim, cache.page_size, self.v_dim)
+        tma = self._decode_tma(cache)
         # (the keys a request can see: a window or a chunk bounds them, and the kernels cut those into the slices)
         seen = min(ctx.max_kv_len, self.span) if self.span else ctx.max_kv_len
         nsplit = (ops.decode_tma_splits(ctx.n_seqs, self.n_kv_heads, group, seen) if tma
@@ -66,8 +69,9 @@ class PagedSoftmaxMixer(Mixer):
                     and ops.prefer_tcgen05_attention(self.runtime.dtype, self.head_dim, cache.k_pages.shape[2], ctx.max_q_len, self.v_dim)):
                 prefill, beside = ops.attention_prefill_tcgen05, True
                 more["host_q_len"] = None if ctx.fixed_shape else ctx.host_q_len or None
-                if singles:     # (the scratch may be cleared when it is made: not between two kernels that run side by side)
-                    self._decode_buffers(ctx)
+                if singles:     # (the buffers may be cleared when they are made: not between two kernels that run side by side)
+                    ready = self._decode_buffers(ctx)[2]
+                    more["ready"] = ready if self._decode_tma(cache) else None
             prefill(out, q, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.seq_slot,
                                   cache.block_table, cache.k_pages, cache.v_pages, ctx.n_seqs, ctx.max_q_len,
                                   self.n_heads, self.n_kv_heads, self.head_dim, self.reach, self.scale, singles, ctx.status,
@@ -75,11 +79,13 @@ class PagedSoftmaxMixer(Mixer):
         if singles:
             self._decode(ctx, out, q, cache, gate=gate, beside_prompts=beside)
 
-    def _decode_buffers(self, ctx: StepContext) -> tuple[torch.Tensor, torch.Tensor]:
+    def _decode_buffers(self, ctx: StepContext) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+        """(scratch for slices, counters, the word between the prompts' kernel and this one)"""
         group = self.n_heads // self.n_kv_heads
         return (ctx.workspace.get("attn.decode_scratch", (ops.decode_scratch_floats(self.n_heads, self.v_dim),), torch.float32),
                 ctx.workspace.get("attn.decode_counters", (ops.decode_counter_ints(ctx.n_seqs, self.n_kv_heads, group),), torch.int32,
-                                  zero=True))
+                                  zero=True),
+                ctx.workspace.get("attn.ready", (1,), torch.int32, zero=True))
 
     def _decode(self, ctx: StepContext, out: torch.Tensor, q: torch.Tensor | None, cache: PagedView, fused=None,
                 gate: torch.Tensor | None = None, beside_prompts: bool = False) -> None:
@@ -89,7 +95,7 @@ class PagedSoftmaxMixer(Mixer):
         other by its longest blocks' chains).  Head sizes that are
         multiples of 64 take the kernel that is fed by TMA, the others the one that loads keys through registers."""
         tma, nsplit, _ = self._decode_launch(ctx, cache)
-        scratch, counters = self._decode_buffers(ctx)
+        scratch, counters, ready = self._decode_buffers(ctx)
         window = self.reach
         product, table, write_cache = fused if fused is not None else (None, None, False)
         prefetch = self._prefetch_plan(ctx)[0] if fused is not None else None
@@ -98,7 +104,8 @@ class PagedSoftmaxMixer(Mixer):
                                      ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.seq_slot, cache.block_table,
                                      cache.k_pages, cache.v_pages, ctx.n_seqs, self.n_heads, self.n_kv_heads, self.head_dim,
                                      window, self.scale, nsplit, scratch, counters, ctx.status, prefetch=prefetch, gate=gate,
-                                     sink=self.sink if self.score_terms else None, beside_prompts=beside_prompts)
+                                     sink=self.sink if self.score_terms else None, beside_prompts=beside_prompts,
+                                     ready=ready)
         elif fused is not None:
             ops.attention_decode_fused(out, product, self.b_qkv, table, write_cache, ctx.seq_q_start, ctx.seq_q_len,
                                        ctx.seq_kv_len, ctx.seq_slot, cache.block_table, cache.k_pages, cache.v_pages,

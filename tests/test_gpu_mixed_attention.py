@@ -48,6 +48,87 @@ def test_prompt_and_decode_attention_side_by_side(hq, hkv, d, window, order):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("captured", [False, True])
+def test_what_the_kernel_before_both_wrote_is_seen(captured):
+    """The queries, and every request's newest keys and values, written into fresh pages by the kernel right before the prompts'
+    attention: the decode attention beside it (the word between the two set) gives the bits of the one that waits, plainly and in a
+    graph, and the word is zero again."""
+    o, hq, hkv, d, rows = ops(), 28, 4, 128, [300, 1, 1, 260] + [1] * 28
+    n, held = len(rows), [(i * 53) % 900 for i in range(len(rows))]
+    total = [a + b for a, b in zip(rows, held)]
+    g = torch.Generator().manual_seed(9)
+    setup = paged_setup(total, 16, hkv, d, torch.bfloat16, seed=3)
+    starts = [sum(rows[:i]) for i in range(n)]
+    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))     # noqa: E731
+    meta = (i32(starts), i32(rows), i32(total), i32(setup["slots"]), setup["table"], setup["k_pages"], setup["v_pages"], n)
+    positions = i32([p for i in range(n) for p in range(held[i], total[i])])
+    seq = i32([i for i in range(n) for _ in range(rows[i])])
+    scratch = torch.zeros(o.decode_scratch_floats(hq, d), device="cuda")
+    counters = torch.zeros(o.decode_counter_ints(n, hkv, hq // hkv), dtype=torch.int32, device="cuda")
+    ready = torch.zeros(1, dtype=torch.int32, device="cuda")
+    made = dev(torch.randn(2, sum(rows), (hq + 2 * hkv) * d, generator=g), torch.bfloat16)     # two steps' products
+    inv_freq = dev((1e4 ** (-torch.arange(0, d, 2) / d)).float())
+    st = status()
+
+    def step(which, word):
+        out, qkv = torch.zeros(sum(rows), hq * d, dtype=torch.bfloat16, device="cuda"), made[which] + 0
+        o.rope_kv_write(qkv, None, positions, seq, meta[3], setup["table"], inv_freq, setup["k_pages"], setup["v_pages"], sum(rows), hq, hkv,
+                        d, True, st)
+        q = qkv[:, :hq * d]
+        o.attention_prefill_tcgen05(out, q, *meta, max(rows), hq, hkv, d, 0, d ** -0.5, True, st, host_q_len=rows, ready=word)
+        o.attention_decode_tma(out, q, None, None, None, False, *meta, hq, hkv, d, 0, d ** -0.5, 2, scratch, counters, st,
+                               beside_prompts=word is not None, ready=word)
+        return out
+
+    def both(word):
+        for _ in range(3):
+            outs = [step(0, word), step(1, word)]       # (the second step writes over the first one's keys and values)
+        return [t + 0 for t in outs]
+
+    want = both(None)
+    if captured:
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            both(ready)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = both(ready)
+        for _ in range(3):
+            graph.replay()
+    else:
+        got = both(ready)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and not torch.equal(want[0], want[1])
+    assert int(ready) == 0 and int(st) == 0
+
+
+@pytest.mark.gpu
+def test_behind_anything_else_it_waits():
+    """A decode attention whose word nobody set waits for the kernel before it, here one that lets it start long before its own
+    results, the queries, are written."""
+    o, hq, hkv, d, n, k = ops(), 28, 4, 128, 40, 8192
+    g = torch.Generator().manual_seed(5)
+    total = [1 + (i * 37) % 300 for i in range(n)]
+    setup = paged_setup(total, 16, hkv, d, torch.bfloat16, seed=2)
+    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))     # noqa: E731
+    meta = (i32(range(n)), i32([1] * n), i32(total), i32(setup["slots"]), setup["table"], setup["k_pages"], setup["v_pages"], n)
+    scratch = torch.zeros(o.decode_scratch_floats(hq, d), device="cuda")
+    counters = torch.zeros(o.decode_counter_ints(n, hkv, hq // hkv), dtype=torch.int32, device="cuda")
+    ready, st = torch.zeros(1, dtype=torch.int32, device="cuda"), status()
+    x, w = dev(torch.randn(n, k, generator=g), torch.bfloat16), dev(torch.randn(hq * d, k, generator=g) / 90, torch.bfloat16)
+
+    def run(beside):
+        q, out = torch.full((n, hq * d), 3.0, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, hq * d, dtype=torch.bfloat16, device="cuda")
+        o.gemm_small_m(q, x, w, n, early_dependents=True)
+        o.attention_decode_tma(out, q, None, None, None, False, *meta, hq, hkv, d, 0, d ** -0.5, 2, scratch, counters, st, beside_prompts=beside,
+                               ready=ready)
+        return out
+
+    want = run(False)
+    assert all(torch.equal(run(True), want) for _ in range(5)) and int(ready) == 0 and int(st) == 0
+
+
+@pytest.mark.gpu
 def test_only_a_decode_attention_with_q_given_runs_beside():
     o = ops()
     setup = paged_setup([40], 16, 1, 64, torch.bfloat16)
