@@ -169,7 +169,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     // With `ready` the kernel before this one is the prompts' attention of the same step.  It lets this kernel start once it has
     // seen all that it reads itself (the rows of q and the cache), and neither reads what the other writes: only one block
     // waits for it, at its end, so that what follows comes after both.
-    const bool beside = ready != nullptr;
+    const bool beside = !FUSED && ready != nullptr;
     const bool waits_last = beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
     if (beside) tw_wait_unless_ready(ready);
     if (seq_q_len[s] != 1) {

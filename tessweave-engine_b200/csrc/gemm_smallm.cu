@@ -27,6 +27,7 @@
 #include "common.cuh"
 
 #include <cooperative_groups.h>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -72,11 +73,12 @@ struct Frag {          // 16 consecutive values of k of one row
 // EPI: the sums get a bias or an activation other than SiLU on gates (kept apart, since it takes registers from the
 // stream of the plain form).
 // MERGE: the grid is (slices, row tiles) and the slices of a row tile a cluster that merges its sums (up to 8 rows).
-template <int NT, int KS, bool EPI, bool MERGE>
+// READY: a kernel that reads x too runs beside this one (of its own, so that the other forms stay as they are).
+template <int NT, int KS, bool EPI, bool MERGE, bool READY>
 __global__ void __launch_bounds__(WARPS * 32, (NT == 1 ? 5 : 0))
 gemm_smallm_kernel(const bf16* __restrict__ w, const bf16* __restrict__ x, int M, int N, int K, int kper,
                    void* __restrict__ out, int out_mode, int out_stride, const TwEpilogue ep, const void* next_weights,
-                   long long next_bytes) {
+                   long long next_bytes, int* ready) {
     constexpr int TILES = WARPS / KS;                  // 16-row tiles of a block
     __shared__ float s_part[KS > 1 ? TILES * 32 * NT * 4 : 1];
     constexpr int TILE_ROWS = TILES * 16;
@@ -90,7 +92,10 @@ gemm_smallm_kernel(const bf16* __restrict__ w, const bf16* __restrict__ x, int M
     // for this kernel's results itself).  That pays when the next kernel is small, like the residual add +
     // norm after the o_proj and down products (measured: 0.5 % of a decode step); before the attention or
     // another large product it costs more than it gives, so the caller decides.
-    if (out_mode & OUT_EARLY_DEPENDENTS) tw_launch_dependents_now();
+    if (out_mode & OUT_EARLY_DEPENDENTS) {
+        if constexpr (READY) tw_say_ready(ready);
+        tw_launch_dependents_now();
+    }
     out_mode &= ~OUT_EARLY_DEPENDENTS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;
@@ -353,11 +358,13 @@ __global__ void reduce_partial_kernel(T* __restrict__ out, const float* __restri
 // out_mode 0: bf16 [M, out_stride]; 1: fp32 [M, out_stride]; 2: fp32 partial sums [ksplit, M, out_stride]
 // (then kper < K); with kper < K, at most 8 slices, at most 8 rows and no `act`, 0 and 1 are added up in clusters; 3: bf16 [M, out_stride] = act(gate) * up for weights whose rows alternate between eight
 // gate rows and their eight up rows (N a multiple of 16, no split).  K must be a multiple of 8; kper of 32.
-// `bias` (bf16 [N], in the order of the rows, or null) and `act`: see TwEpilogue.
+// `bias` (bf16 [N], in the order of the rows, or null) and `act`: see TwEpilogue.  `ready` (or null; with OUT_EARLY_DEPENDENTS): the word
+// for a kernel that reads x beside this one, see tw_say_ready.
 TW_EXPORT int tw_gemm_smallm(const void* w, const void* x, int M, int N, int K, int kper, void* out, int out_mode,
                              int out_stride, const void* bias, int act, const void* next_weights, long long next_bytes,
-                             cudaStream_t stream) {
+                             int* ready, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
+    if (ready && !(out_mode & OUT_EARLY_DEPENDENTS)) return (int)cudaErrorInvalidValue;
     if ((uintptr_t)next_weights & 15) return (int)cudaErrorMisalignedAddress;
     if (!next_weights || next_bytes < 0) next_bytes = 0;
     if (M > 64 || K <= 0 || (K & 7) || kper <= 0 || (kper & 31) || (out_mode & ~OUT_EARLY_DEPENDENTS) < 0 || (out_mode & ~OUT_EARLY_DEPENDENTS) > 3 || ((out_mode & ~OUT_EARLY_DEPENDENTS) == OUT_GATED && (N & 15)) ||
@@ -381,19 +388,23 @@ TW_EXPORT int tw_gemm_smallm(const void* w, const void* x, int M, int N, int K, 
     const bool epi = bias || act != ((out_mode & ~OUT_EARLY_DEPENDENTS) == OUT_GATED ? TW_ACT_SILU : TW_ACT_NONE);
     if (pair_warps) grid.x = (N + (WARPS / 2) * 16 - 1) / ((WARPS / 2) * 16);
     if (merge) {
-        auto merging = pair_warps ? (epi ? gemm_smallm_kernel<1, 2, true, true> : gemm_smallm_kernel<1, 2, false, true>)
-                                  : (epi ? gemm_smallm_kernel<1, 1, true, true> : gemm_smallm_kernel<1, 1, false, true>);
+        if (ready) return (int)cudaErrorInvalidValue;
+        auto merging = pair_warps ? (epi ? gemm_smallm_kernel<1, 2, true, true, false> : gemm_smallm_kernel<1, 2, false, true, false>)
+                                  : (epi ? gemm_smallm_kernel<1, 1, true, true, false> : gemm_smallm_kernel<1, 1, false, true, false>);
         return tw_launch(merging, dim3(ksplit, grid.x), dim3(WARPS * 32), 0, stream, ksplit, wp, xp, M, N, K, kper, out, out_mode, out_stride, ep,
-                         next_weights, next_bytes);
+                         next_weights, next_bytes, ready);
     }
-    auto kernel = pair_warps ? (epi ? gemm_smallm_kernel<1, 2, true, false> : gemm_smallm_kernel<1, 2, false, false>)
-                : M <= 8     ? (epi ? gemm_smallm_kernel<1, 1, true, false> : gemm_smallm_kernel<1, 1, false, false>)
-                : M <= 16    ? (epi ? gemm_smallm_kernel<2, 1, true, false> : gemm_smallm_kernel<2, 1, false, false>)
-                : M <= 32    ? (epi ? gemm_smallm_kernel<4, 1, true, false> : gemm_smallm_kernel<4, 1, false, false>)
-                             : (epi ? gemm_smallm_kernel<8, 1, true, false> : gemm_smallm_kernel<8, 1, false, false>);
-    tw_launch(kernel, dim3(grid), dim3(WARPS * 32), 0, stream, 1, wp, xp, M, N, K, kper, out, out_mode, out_stride, ep,
-              next_weights, next_bytes);
-    return TW_LAUNCH_CHECK();
+    auto launch = [&](auto beside) {
+        constexpr bool R = decltype(beside)::value;
+        auto kernel = pair_warps ? (epi ? gemm_smallm_kernel<1, 2, true, false, R> : gemm_smallm_kernel<1, 2, false, false, R>)
+                    : M <= 8     ? (epi ? gemm_smallm_kernel<1, 1, true, false, R> : gemm_smallm_kernel<1, 1, false, false, R>)
+                    : M <= 16    ? (epi ? gemm_smallm_kernel<2, 1, true, false, R> : gemm_smallm_kernel<2, 1, false, false, R>)
+                    : M <= 32    ? (epi ? gemm_smallm_kernel<4, 1, true, false, R> : gemm_smallm_kernel<4, 1, false, false, R>)
+                                 : (epi ? gemm_smallm_kernel<8, 1, true, false, R> : gemm_smallm_kernel<8, 1, false, false, R>);
+        return tw_launch(kernel, dim3(grid), dim3(WARPS * 32), 0, stream, 1, wp, xp, M, N, K, kper, out, out_mode, out_stride, ep,
+                         next_weights, next_bytes, ready);
+    };
+    return ready ? launch(std::true_type()) : launch(std::false_type());
 }
 
 // bf16 operands, rows of x `x_stride` apart on 16-byte boundaries, w [N, K] contiguous, N <= 64, K a multiple of 8; out fp32.

@@ -262,11 +262,12 @@ __global__ void __launch_bounds__(512)
 moe_route_kernel(int* __restrict__ chosen, float* __restrict__ weight, float* __restrict__ shared_gate,
                  const T* __restrict__ h, int h_stride, const T* __restrict__ wr, const float* __restrict__ br,
                  const T* __restrict__ ws, int width, int E, int top, int scoring, const float* __restrict__ correction,
-                 float weight_scale, int group_count, int group_keep, int beside) {
+                 float weight_scale, int group_count, int group_keep, int* ready) {
     extern __shared__ float sm[];           // [width] the row (not DIRECT), [E + 1] logits, [E] marks, [2 group_count]
-    // `beside`: the kernel before this one reads the same rows and writes nothing that is read here; it lets this kernel start
+    // With `ready` the kernel before this one reads the same rows and writes nothing that is read here; it lets this kernel start
     // once the rows are there, and one block waits for it, at its end.
-    if (!beside) tw_grid_wait();
+    if (ready) tw_wait_unless_ready(ready);
+    else tw_grid_wait();
     tw_grid_launch_dependents();
     const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* x = sm;
@@ -286,7 +287,7 @@ moe_route_kernel(int* __restrict__ chosen, float* __restrict__ weight, float* __
     __syncthreads();
     if (warp != 0) return;
     moe_select(z, row, lane, ws != nullptr, E, top, scoring, correction, weight_scale, group_count, group_keep, chosen, weight, shared_gate);
-    if (beside && blockIdx.x == 0) tw_grid_wait();
+    if (ready && blockIdx.x == 0) tw_wait_and_clear(ready, lane == 0);
 }
 
 // Steps of many bf16 rows: a warp per row, sixteen rows to a block, which copies the router's matrix to shared memory once.  The dot
@@ -364,11 +365,14 @@ moe_route_rows_kernel(int* __restrict__ chosen, float* __restrict__ weight, floa
     moe_select(z, row, lane, ws != nullptr, E, top, scoring, correction, weight_scale, group_count, group_keep, chosen, weight, shared_gate);
 }
 
+// `ready` (or null; bf16, few rows): the word that the kernel launched before, a product of the same rows (tw_gemm_smallm with
+// OUT_EARLY_DEPENDENTS), was given; this one runs beside it then.
 TW_EXPORT int tw_moe_route(int* chosen, float* weight, float* shared_gate, const void* h, int h_stride, const void* wr,
                            const float* br, const void* ws, int rows, int width, int E, int top, int scoring,
-                           const float* correction, float weight_scale, int group_count, int group_keep, int beside, int dtype,
+                           const float* correction, float weight_scale, int group_count, int group_keep, int* ready, int dtype,
                            cudaStream_t stream) {
     if (rows <= 0) return 0;
+    if (ready && (dtype == TW_F32 || rows >= TW_ROUTE_MIN_ROWS)) return (int)cudaErrorInvalidValue;
     if (E <= 0 || top <= 0 || top > E || scoring < 0 || scoring > 2) return (int)cudaErrorInvalidValue;
     if (group_count < 0 || (group_count > 0 && (scoring == 0 || E % group_count || group_keep < 1 || group_keep > group_count
                                                 || group_keep * (E / group_count) < top)))
@@ -388,7 +392,7 @@ TW_EXPORT int tw_moe_route(int* chosen, float* weight, float* shared_gate, const
     if (dtype == TW_F32)
         return tw_launch(moe_route_kernel<float, false>, dim3(rows), dim3(threads), smem, stream, 1, chosen, weight, shared_gate,
                          (const float*)h, h_stride, (const float*)wr, br, (const float*)ws, width, E, top, scoring, correction,
-                         weight_scale, group_count, group_keep, 0);
+                         weight_scale, group_count, group_keep, nullptr);
     const bool direct = rows <= TW_ROUTE_DIRECT_ROWS && (width & 7) == 0 && (h_stride & 7) == 0 && a16(h) && a16(wr) && a16(ws);
     // (1 KB at least: with less the driver splits L1 and shared memory otherwise than for the product beside)
     const size_t used = direct ? std::max<size_t>(smem - (size_t)width * sizeof(float), 1024) : smem;
@@ -396,9 +400,9 @@ TW_EXPORT int tw_moe_route(int* chosen, float* weight, float* shared_gate, const
     auto launch = [&](auto how) {
         return tw_launch<decltype(how)::value>(kernel, dim3(rows), dim3(threads), used, stream, 1, chosen, weight, shared_gate,
                                                (const __nv_bfloat16*)h, h_stride, (const __nv_bfloat16*)wr, br, (const __nv_bfloat16*)ws, width,
-                                               E, top, scoring, correction, weight_scale, group_count, group_keep, beside ? 1 : 0);
+                                               E, top, scoring, correction, weight_scale, group_count, group_keep, ready);
     };
-    return beside ? launch(std::integral_constant<int, TW_OVERLAPS>()) : launch(std::integral_constant<int, TW_BY_SIZE>());
+    return ready ? launch(std::integral_constant<int, TW_OVERLAPS>()) : launch(std::integral_constant<int, TW_BY_SIZE>());
 }
 
 #define TW_MOE_WARPS 8

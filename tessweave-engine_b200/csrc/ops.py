@@ -1413,7 +1413,7 @@ def small_m_split(n: int, k: int, max_slices: int = 12, sms: int | None = None) 
 def gemm_small_m(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, kper: int | None = None,
                  silu_mul_pairs: bool = False, early_dependents: bool = False,
                  prefetch: torch.Tensor | None = None, bias: torch.Tensor | None = None, act: int | None = None,
-                 merge: bool = False) -> None:
+                 merge: bool = False, ready: torch.Tensor | None = None) -> None:
     """out[:m] = x[:m] @ w.T for m <= 64 rows.  ``out`` is bf16 or fp32 [>=m, n]; or, when the
     product is split over k (kper < k), fp32 slices [slices, m, n] (with ``merge``, for up to 8 rows and 8 slices, their
     sum in the order ``SplitSum.dense`` adds them: ``out`` as without a split); or, with ``silu_mul_pairs``
@@ -1422,8 +1422,11 @@ def gemm_small_m(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, kp
     ``act`` is applied to every value (not to slices).
     ``early_dependents``: the kernel launched next may become resident while this one runs (it waits for
     the result itself); worth it when that kernel is small.  ``prefetch``: a contiguous, 16-byte aligned tensor
-    that the kernel after this one streams; the blocks ask for it to be brought into L2 when their own stream ends."""
+    that the kernel after this one streams; the blocks ask for it to be brought into L2 when their own stream ends.
+    ``ready`` (with ``early_dependents``): for the kernel that is launched next and runs beside this one (``moe_route``)."""
     _cuda(out, x, w, bias)
+    _ready_check(ready)
+    _need(ready is None or early_dependents, "gemm_small_m: only with early_dependents does a kernel run beside it")
     if prefetch is not None:
         _need(prefetch.is_cuda and prefetch.is_contiguous(), "gemm_small_m: the tensor to prefetch must be contiguous")
     n, k = w.shape
@@ -1451,7 +1454,7 @@ def gemm_small_m(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, m: int, kp
     code = _fn("gemm_smallm", "tw_gemm_smallm")(_ptr(w), _ptr(x), c_int(m), c_int(n), c_int(k), c_int(kper), _ptr(out),
                                                 c_int(mode), c_int(stride), _ptr(bias), c_int(act), _ptr(prefetch),
                                                 ctypes.c_longlong(prefetch.numel() * prefetch.element_size()
-                                                                  if prefetch is not None else 0), _stream())
+                                                                  if prefetch is not None else 0), _ptr(ready), _stream())
     _check(code, "gemm_small_m")
 
 
@@ -2108,14 +2111,17 @@ def kv_store(rows: torch.Tensor, k_col: int, v_col: int, positions: torch.Tensor
 def moe_route(chosen: torch.Tensor, weight: torch.Tensor, shared_gate: torch.Tensor | None, h: torch.Tensor, w_router: torch.Tensor,
               b_router: torch.Tensor | None, w_shared_gate: torch.Tensor | None, n_rows: int, top: int,
               score_all: bool = False, correction: torch.Tensor | None = None, weight_scale: float = 1.0,
-              renormalise: bool = False, groups: tuple[int, int] | None = None, beside: bool = False) -> None:
+              renormalise: bool = False, groups: tuple[int, int] | None = None, beside: bool = False,
+              ready: torch.Tensor | None = None) -> None:
     """Per row: the ``top`` experts with the largest fp32 logits ``w_router h + b_router`` (int32 [rows, top]), the
     softmax over those logits alone (fp32 [rows, top]), and ``sigmoid(w_shared_gate . h)`` (fp32 [rows]) if asked.
     With ``score_all`` the scores are the softmax over every router output, the choice goes by score + ``correction``
     (fp32 [outputs], may be None) and the weights are the chosen scores times ``weight_scale``, not renormalised -- or, with ``renormalise``, the chosen scores over their
     sum (+ 1e-20) times ``weight_scale``.  ``groups`` = (count, keep): the outputs form ``count`` groups of as many consecutive outputs
     and only those of the ``keep`` groups with the largest best score may be chosen.  ``beside`` (bfloat16, few rows): the last kernel
-    launched on this stream is a product of the same ``h`` with ``early_dependents``, and this one runs beside it."""
+    launched on this stream is a product of the same ``h`` with ``early_dependents``, and this one runs beside it if both were given
+    ``ready`` (int32 [1], zero and zero again afterwards), through which the first tells this one that the rows are there."""
+    _ready_check(ready)
     _need(not beside or (h.dtype == torch.bfloat16 and n_rows <= 64), "moe_route: only bfloat16 steps of few rows are routed beside a product")
     _cuda(chosen, weight, shared_gate, h, w_router, b_router, w_shared_gate, correction)
     experts, width = w_router.shape
@@ -2136,7 +2142,7 @@ def moe_route(chosen: torch.Tensor, weight: torch.Tensor, shared_gate: torch.Ten
     code = _fn("moe", "tw_moe_route")(_ptr(chosen), _ptr(weight), _ptr(shared_gate), _ptr(h), c_int(h.stride(0)), _ptr(w_router),
                                       _ptr(b_router), _ptr(w_shared_gate), c_int(n_rows), c_int(width), c_int(experts), c_int(top),
                                       c_int((2 if renormalise else 1) if score_all else 0), _ptr(correction), c_float(weight_scale),
-                                      c_int(count), c_int(keep), c_int(1 if beside else 0),
+                                      c_int(count), c_int(keep), _ptr(ready if beside else None),
                                       c_int(dtype_code(h.dtype)), _stream())
     _check(code, "moe_route")
 

@@ -76,14 +76,14 @@ class GatedMLP(FeedForward):
         """Whether ``gate_up`` of a step of ``n`` rows is one launch of the weight-streaming kernel."""
         return self.interleaved and ops.small_m_supported(h, self.w_gate_up, n)
 
-    def gate_up(self, ctx: StepContext, h: torch.Tensor, consumer_early: bool = False) -> torch.Tensor:
-        """act(gate) * up, by whichever kernel takes the step's number of rows.  ``consumer_early``: as for ``linear``, where
-        ``one_streamed_product``."""
+    def gate_up(self, ctx: StepContext, h: torch.Tensor, ready: torch.Tensor | None = None) -> torch.Tensor:
+        """act(gate) * up, by whichever kernel takes the step's number of rows.  ``ready``: as for ``ops.gemm_small_m``, for a kernel that
+        runs beside, where ``one_streamed_product``."""
         n, ws, dt = ctx.n_tokens, ctx.workspace, self.runtime.dtype
         act = ws.get("ffn.act", (n, self.intermediate), dt)
         how = {"act": self.act, "bias": self.b_gate_up}
         if self.one_streamed_product(h, n):
-            ops.gemm_small_m(act, h, self.w_gate_up, n, silu_mul_pairs=True, early_dependents=consumer_early, **how,
+            ops.gemm_small_m(act, h, self.w_gate_up, n, silu_mul_pairs=True, early_dependents=ready is not None, ready=ready, **how,
                              prefetch=ops.weight_head(self.w_down, ops.product_prefetch_bytes()))
         elif (self.interleaved and ops.stream_product_preferred(h, self.w_gate_up, n)
               and (ops.stream_whole_k_balanced(2 * self.intermediate) or ops.stream_split_gate_up_enabled())):
@@ -267,25 +267,27 @@ class RoutedExperts(FeedForward):
         return (ws.get("moe.chosen", (n, self.top), torch.int32), ws.get("moe.weight", (n, self.top), torch.float32),
                 ws.get("moe.shared_gate", (n,), torch.float32) if self.w_shared_gate is not None else None)
 
-    def route(self, ctx: StepContext, h: torch.Tensor, beside: bool = False):
-        """(chosen int32 [rows, top], weights fp32 [rows, top], gate of the shared expert fp32 [rows] or None).  ``beside``: the
-        shared expert's first product has just been launched, and the router runs beside it."""
+    def route(self, ctx: StepContext, h: torch.Tensor, ready: torch.Tensor | None = None):
+        """(chosen int32 [rows, top], weights fp32 [rows, top], gate of the shared expert fp32 [rows] or None).  ``ready``: the shared
+        expert's first product has just been launched with this word, and the router runs beside it."""
         n = ctx.n_tokens
         chosen, weight, gate = self._route_buffers(ctx)
         ops.moe_route(chosen, weight, gate, h, self.w_router, self.b_router,
                       self.w_shared_gate.view(-1) if self.w_shared_gate is not None else None, n, self.top,
                       score_all=self.score_all, correction=self.correction, weight_scale=self.weight_scale,
-                      renormalise=self.renormalise, groups=self.groups, beside=beside)
+                      renormalise=self.renormalise, groups=self.groups, beside=ready is not None, ready=ready)
         return chosen, weight, gate
 
     def forward(self, ctx: StepContext, h: torch.Tensor):
         n, ws, dt = ctx.n_tokens, ctx.workspace, self.runtime.dtype
         shared = None
+        # (asked for in every step, so that the workspace has all of its buffers after the first one)
+        ready = ws.get("moe.ready", (1,), torch.int32, zero=True) if self.shared is not None else None
         if isinstance(self.shared, GatedMLP) and dt == torch.bfloat16 and n <= 64 and self.shared.one_streamed_product(h, n):
             # few rows: the router, a chain of latencies on as many SMs as there are rows, beside the shared expert's first product
             self._route_buffers(ctx)            # (a new buffer may be filled when it is made: not between the two)
-            act = self.shared.gate_up(ctx, h, consumer_early=True)
-            chosen, weight, gate = self.route(ctx, h, beside=True)
+            act = self.shared.gate_up(ctx, h, ready)
+            chosen, weight, gate = self.route(ctx, h, ready)
             shared = dense_delta(ctx, self.shared.down(ctx, act), dt, "moe.shared")
         else:
             chosen, weight, gate = self.route(ctx, h)

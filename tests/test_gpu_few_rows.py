@@ -62,13 +62,17 @@ def test_router_reads_rows_where_they_lie(rows, width, experts, stride, shared, 
     br = torch.randn(experts, generator=g).to(dev)
     weights = torch.randn(64, width, generator=g).bfloat16().to(dev)
 
+    ready = torch.zeros(1, dtype=torch.int32, device=dev)
+
     def run(x, beside):
         chosen, weight = torch.empty(rows, top, dtype=torch.int32, device=dev), torch.empty(rows, top, device=dev)
         gate = torch.empty(rows, device=dev) if shared else None
         if beside:
             out = torch.empty(rows, 64, dtype=torch.bfloat16, device=dev)
-            o.gemm_small_m(out, x, weights, rows, early_dependents=True)
-        o.moe_route(chosen, weight, gate, x, wr, br, ws if shared else None, rows, top, score_all=scored, beside=beside)
+            if beside == "rows made just before":
+                x = x + 0
+            o.gemm_small_m(out, x, weights, rows, early_dependents=True, ready=ready)
+        o.moe_route(chosen, weight, gate, x, wr, br, ws if shared else None, rows, top, score_all=scored, beside=bool(beside), ready=ready)
         return [t for t in (chosen, weight, gate) if t is not None] + ([out] if beside else [])
 
     def laid(offset, row):
@@ -79,7 +83,31 @@ def test_router_reads_rows_where_they_lie(rows, width, experts, stride, shared, 
     want = run(laid(1, stride + 1), False)
     assert all(torch.equal(a, b) for a, b in zip(run(laid(0, stride), False), want))
     if rows <= 64 and stride == width:
-        for _ in range(3):
-            got = run(laid(0, stride), True)
+        for i in range(4):
+            got = run(laid(0, stride), "rows made just before" if i & 1 else True)
+            assert int(ready) == 0
             assert all(torch.equal(a, b) for a, b in zip(got, want))
             assert torch.allclose(got[-1].float(), (h.to(dev).float() @ weights.float().T), rtol=2e-2, atol=2e-2 * width ** 0.5)
+
+
+@pytest.mark.gpu
+def test_router_behind_anything_else_waits():
+    """A router whose word nobody set waits for the kernel before it, here one that lets it start long before its own results, the
+    router's rows, are written; a product without a kernel beside it takes no word."""
+    o, rows, width, k = ops(), 40, 3584, 8192
+    g = torch.Generator().manual_seed(8)
+    make = lambda *shape: torch.randn(*shape, generator=g).bfloat16().cuda()        # noqa: E731
+    x, w, wr, ready = make(rows, k), make(width, k) / 90, make(8, width), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run(beside):
+        h = torch.full((rows, width), 3.0, dtype=torch.bfloat16, device="cuda")
+        chosen, weight = torch.empty(rows, 2, dtype=torch.int32, device="cuda"), torch.empty(rows, 2, device="cuda")
+        o.gemm_small_m(h, x, w, rows, early_dependents=True)
+        o.moe_route(chosen, weight, None, h, wr, None, None, rows, 2, beside=beside, ready=ready)
+        return chosen, weight
+
+    want = run(False)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(run(True), want)) and int(ready) == 0
+    with pytest.raises(Exception, match="beside"):
+        o.gemm_small_m(torch.empty(rows, width, dtype=torch.bfloat16, device="cuda"), x, w, rows, ready=ready)
