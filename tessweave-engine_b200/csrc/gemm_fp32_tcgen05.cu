@@ -13,7 +13,8 @@
 //   * four warps add the accumulator of the last 64 values to their registers (tcgen05.ld), a row of the tile per thread.
 //
 // A sum that is not finite is made again as a chain of plain fp32 multiply-adds: an infinite number has no three terms, and a
-// finite one above the largest bf16 would give infinities.  Numbers below 2^-100 lose their last bits as their terms underflow.
+// finite one above the largest bf16 would give infinities.  The block's cutting warps make the whole tile again then, so that a
+// matrix full of NaN takes a few times the product's time and not a thousand times.  Numbers below 2^-100 lose their last bits as their terms underflow.
 //
 // What bounds it is the data port of shared memory and L1: the MMAs' operands take 48 KB of it per 16 values of k, the terms' stores
 // and the loads half as much again, and 64 values of k take 3,100 cycles of which the tensor pipe is busy for 1,540.  (N = 256 for x_h
@@ -71,15 +72,69 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& a, uint32_t& 
     c = round2(less(v, b));
 }
 
+// Sums of the tile that are not finite, again, by the cutting warps: every sum of the tile on the FMA units, in one chain over k
+// (fmaf(x, w, sum) from zero on), and those that were not finite take the place of what stands in `sums` (see the kernel).
+// 128 rows of 32 values of k of x and of w at a time in `area`, transposed; a warp has eight rows, a lane four columns.
+constexpr int AGAIN_K = 32, AGAIN_STRIDE = 128 + 4;
+static_assert(128 * 512 <= STAGE && 2 * AGAIN_K * AGAIN_STRIDE * 4 <= STAGE && CUTTERS * 8 == 128, "the sums take the first stage, their factors the second");
+__device__ __forceinline__ void cutters_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CUTTERS * 32) : "memory"); }
+__device__ __forceinline__ unsigned char* sum_place(unsigned char* sums, int row, int col4) {
+    return sums + (row >> 5) * (32 * 512) + (row & 31) * 512 + ((col4 ^ (row & 31)) << 4);
+}
+__device__ __forceinline__ void make_again(unsigned char* sums, float* area, const float* __restrict__ x, int x_stride, const float* __restrict__ w,
+                                        int w_stride, int row0, int col0, int M, int N, int K) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* xs = area;
+    float* ws = area + AGAIN_K * AGAIN_STRIDE;
+    float acc[8][4];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+    for (int k0 = 0; k0 < K; k0 += AGAIN_K) {
+        cutters_sync();                                     // nobody reads the values before these any more
+        for (int half = 0; half < 2; ++half)
+            for (int i = threadIdx.x; i < 128 * (AGAIN_K / 4); i += CUTTERS * 32) {
+                const int r = i / (AGAIN_K / 4), q = i % (AGAIN_K / 4) * 4, at = (half ? col0 : row0) + r;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k0 + q < K && at < (half ? N : M))
+                    v = *reinterpret_cast<const float4*>((half ? w + (size_t)at * w_stride : x + (size_t)at * x_stride) + k0 + q);
+                float* p = (half ? ws : xs) + q * AGAIN_STRIDE + r;
+                p[0] = v.x; p[AGAIN_STRIDE] = v.y; p[2 * AGAIN_STRIDE] = v.z; p[3 * AGAIN_STRIDE] = v.w;
+            }
+        cutters_sync();
+        const int most = min(AGAIN_K, K - k0);
+        for (int k = 0; k < most; ++k) {
+            const float4 xa = *reinterpret_cast<const float4*>(xs + k * AGAIN_STRIDE + warp * 8);
+            const float4 xb = *reinterpret_cast<const float4*>(xs + k * AGAIN_STRIDE + warp * 8 + 4);
+            const float4 wv = *reinterpret_cast<const float4*>(ws + k * AGAIN_STRIDE + lane * 4);
+            const float xr[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w}, wc[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(xr[r], wc[c], acc[r][c]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        float* p = reinterpret_cast<float*>(sum_place(sums, warp * 8 + r, lane));
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (!isfinite(p[c])) p[c] = acc[r][c];
+    }
+}
+// the sums stand in shared memory: the adding warps say so, the cutting warps wait for it
+__device__ __forceinline__ void sums_there() { asm volatile("bar.arrive 2, %0;" ::"n"((CUTTERS + ADDERS) * 32) : "memory"); }
+__device__ __forceinline__ void wait_for_sums() { asm volatile("bar.sync 2, %0;" ::"n"((CUTTERS + ADDERS) * 32) : "memory"); }
+
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_fp32_kernel(float* __restrict__ out, int out_stride, const float* __restrict__ x, int x_stride, const float* __restrict__ w,
                  int w_stride, int M, int N, int K, int* status) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full[2], done[2], read[2];
+    __shared__ __align__(8) uint64_t full[2], done[2], read[2], made_again;
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_aborted;
+    __shared__ int s_aborted, s_again;
     unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     volatile int* aborted = &s_aborted;
+    volatile int* again = &s_again;
     tw_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_m = (M + BM - 1) / BM;
@@ -87,7 +142,8 @@ gemm_fp32_kernel(float* __restrict__ out, int out_stride, const float* __restric
     const int num_kb = (K + BK - 1) / BK;
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) { mbar_init(&full[s], CUTTERS); mbar_init(&done[s], 1); mbar_init(&read[s], ADDERS); }
-        s_aborted = 0;
+        mbar_init(&made_again, CUTTERS);
+        s_aborted = s_again = 0;
         mbar_fence_init();
     }
     if (warp == MMA_WARP) tmem_alloc(&tmem_slot, TMEM_COLS);
@@ -186,6 +242,13 @@ gemm_fp32_kernel(float* __restrict__ out, int out_stride, const float* __restric
             if (lane == 0) mbar_arrive(&full[s]);
         }
         if (!ok) *aborted = 1;
+        __syncwarp();
+        wait_for_sums();
+        if (*again) {
+            make_again(stages, reinterpret_cast<float*>(stages + STAGE), x, x_stride, w, w_stride, row0, col0, M, N, K);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&made_again);
+        }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ADD_REGS));
         // a thread adds up the sums of one row
@@ -203,7 +266,7 @@ gemm_fp32_kernel(float* __restrict__ out, int out_stride, const float* __restric
                 for (int e = 0; e < 16; ++e) acc[c + e] += __uint_as_float(t[e]);
             }
         };
-        bool ok = true;
+        bool ok = true, finite = true;
         for (int kb = 0; kb < num_kb; ++kb) {
             const int s = kb & 1;
             ok = !*aborted && mbar_wait(&done[s], (kb >> 1) & 1, status);
@@ -218,34 +281,24 @@ gemm_fp32_kernel(float* __restrict__ out, int out_stride, const float* __restric
             *aborted = 1;
         } else {
             add(mine + LOW_COL);
-            const int row = row0 + quarter * 32 + lane;
-            bool finite = true;
 #pragma unroll
             for (int e = 0; e < BN; ++e) finite = finite && isfinite(acc[e]);
-            if (!finite && row < M) {
-                for (int e = 0; e < BN && col0 + e < N; ++e) {
-                    float value = 0.f;
-#pragma unroll
-                    for (int i = 0; i < BN; ++i) value = i == e ? acc[i] : value;
-                    if (isfinite(value)) continue;
-                    value = 0.f;
-                    for (int k = 0; k < K; ++k) value = fmaf(x[(size_t)row * x_stride + k], w[(size_t)(col0 + e) * w_stride + k], value);
-#pragma unroll
-                    for (int i = 0; i < BN; ++i) acc[i] = i == e ? value : acc[i];
-                }
-            }
+            if (!finite) *again = 1;                        // (what is behind the last row or column has the numbers of one that is not)
             // through shared memory (every MMA has retired), so that a warp writes whole rows: 32 rows of 128 sums a warp
-            unsigned char* own = stages + quarter * (32 * 512);
 #pragma unroll
             for (int c = 0; c < BN / 4; ++c)
-                *reinterpret_cast<float4*>(own + lane * 512 + ((c ^ (lane & 31)) << 4)) = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
-            __syncwarp();
+                *reinterpret_cast<float4*>(sum_place(stages, quarter * 32 + lane, c)) = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+        }
+        __syncwarp();
+        sums_there();
+        if (__any_sync(0xffffffffu, !finite) && !mbar_wait(&made_again, 0, status)) ok = false;
+        if (ok) {
             const int gcol = col0 + 4 * lane;
             const bool wide = (N & 3) == 0 && (out_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
 #pragma unroll 8
             for (int r = 0; r < 32; ++r) {
                 const int grow = row0 + quarter * 32 + r;
-                const float4 o = *reinterpret_cast<const float4*>(own + r * 512 + ((lane ^ r) << 4));
+                const float4 o = *reinterpret_cast<const float4*>(sum_place(stages, quarter * 32 + r, lane));
                 if (grow >= M || gcol >= N) continue;
                 float* dst = out + (size_t)grow * out_stride + gcol;
                 if (wide) {

@@ -57,6 +57,57 @@ def test_numbers_without_three_terms():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,x_more", [(333, 260, 132, 4), (128, 128, 32, 0), (130, 390, 1000, 0), (5, 3, 4, 0)])
+def test_many_sums_that_are_not_finite(m, n, k, x_more):
+    """Rows of x and of w with infinities and NaN throughout, at both ends and at edges of tiles: every sum that is not finite in 64 bits
+    is the same kind of number here, every other one within the bound, and nothing behind the last row or column is written."""
+    o = ops()
+    g = torch.Generator().manual_seed(m)
+    x, w = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g)
+    bad = (float("inf"), -float("inf"), float("nan"))
+    for t, step in ((x, 3), (w, 41)):
+        for i in {*range(0, t.shape[0], step), t.shape[0] - 1}:
+            t[i, (i * 7) % k] = bad[i % 3]
+    w[0, :: 2] = 0.0                            # (an infinity times zero is no number)
+    xd = torch.zeros(m, k + x_more, device="cuda")[:, :k]
+    xd.copy_(x)
+    out, status = torch.full((m + 1, n), 7.0, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    o.gemm_fp32(out[:m], xd, w.cuda(), m, status)
+    want, got = x.double() @ w.double().T, out[:m].cpu().double()
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    clean = lambda t: t.double().nan_to_num(0, 0, 0).abs()      # noqa: E731
+    assert bool(((got - want).abs() <= 2.0 ** -17 * (clean(x) @ clean(w).T))[finite].all())
+    assert bool((out[m] == 7.0).all()) and int(status) == 0
+
+
+@pytest.mark.gpu
+def test_numbers_that_are_not_finite_cost_little():
+    """A matrix full of NaN (a model that has diverged): a few times the product's time, here at most 20 times; sum by sum, by one thread
+    for a row, it was hundreds of times."""
+    o = ops()
+    m, n, k = 777, 896, 4864
+    x, w, out = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda"), torch.empty(m, n, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def us(rows):
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            o.gemm_fp32(out, rows, w, m, status)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return min(times)
+
+    plain = us(x)
+    worst = us(torch.full_like(x, float("nan")))
+    assert bool(torch.isnan(out).all()) and worst < 20 * plain, (plain, worst)
+    print(f"finite {plain:.1f} us, NaN {worst:.1f} us")
+
+
+@pytest.mark.gpu
 def test_which_products_and_what_is_refused():
     o = ops()
     assert o.prefer_gemm_fp32(777, 896, 896) and not o.prefer_gemm_fp32(512, 1152, 896) and not o.prefer_gemm_fp32(64, 151936, 896)
