@@ -14,14 +14,18 @@
 //
 // A sum that is not finite is made again as a chain of plain fp32 multiply-adds: an infinite number has no three terms, and a
 // finite one above the largest bf16 would give infinities.  The block's cutting warps make the whole tile again then, so that a
-// matrix full of NaN takes a few times the product's time and not a thousand times.  Numbers below 2^-100 lose their last bits as their terms underflow.
+// matrix full of NaN takes a few times the product's time and not a thousand times.  Numbers are taken times 2^16 on the
+// way in, so that the last bits of the smallest ones do not fall below what a term can hold.
 //
 // What bounds it is the data port of shared memory and L1: the MMAs' operands take 48 KB of it per 16 values of k, the terms' stores
 // and the loads half as much again, and 64 values of k take 3,100 cycles of which the tensor pipe is busy for 1,540.  (N = 256 for x_h
 // against two terms of w at once, and eight warps instead of sixteen, change nothing.)  us here and in the library's fp32 product, which
-// runs on the FMA units: 1,814 rows by 896 x 1,152 33 and 80, by 896 x 896 33 and 70, by 1,536 x 2,048 92 and 238, by 4,864 x 896 135
-// and 328; 777 rows by 896 x 1,152 33 and 45.  Relative error against 64 bits (2-norms), here and there: k = 896 1.0e-7 and 5.4e-7,
-// k = 1,536 1.2e-7 and 7.0e-7, k = 4,864 1.9e-7 and 1.3e-6.
+// runs on the FMA units: 1,814 rows by 896 x 1,152 28 and 77, by 896 x 896 28 and 68, by 1,536 x 2,048 84 and 236, by 4,864 x 896 125
+// and 324; 777 rows by 896 x 1,152 28 and 42 (caches warm).  A matrix of NaN: 777 rows by 4,864 x 896 0.92 ms, the library 0.20.
+// Relative error against 64 bits (2-norms), here and there: k = 896 1.0e-7 and 5.4e-7, k = 1,536 1.2e-7 and 7.0e-7, k = 4,864 1.9e-7 and
+// 6.3e-7; numbers spread over 60 powers of two: k = 256 9.4e-8 and 9.0e-8, k = 896 1.1e-7 and 1.6e-7, k = 4,864 1.8e-7 and 1.9e-7, k =
+// 8,960 2.4e-7 and 2.1e-7; numbers of 2^-126: 9.0e-8 and 4.1e-7 (not scaled 2.3e-3).  (Halving what grows with k, by a second level of sums
+// in tensor memory, costs 2 to 5 % of the time.)
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets TW_ERR_WAIT in the status word, every role stops, and the block
 // frees its tensor memory and returns.
@@ -64,8 +68,20 @@ __device__ __forceinline__ uint32_t round2(float2 v) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// (x, y) times 2^UP.  The smallest 32-bit number's last bit, 2^-149, becomes 2^-133 so, the smallest that a bf16 number has; a number
+// or a sum that this takes out of range is not finite and made again.  The sums are taken back by 2^-2 UP.
+constexpr int UP = 16;
+__device__ __forceinline__ float2 scaled(float x, float y) {
+    float2 d;
+    asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %4};\n\t"
+        "mul.rn.f32x2 rd, ra, rb;\n\t"
+        "mov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(x), "f"(y), "f"((float)(1 << UP)));
+    return d;
+}
 __device__ __forceinline__ void split3(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
-    float2 v = make_float2(x, y);
+    float2 v = scaled(x, y);
     a = round2(v);
     v = less(v, a);
     b = round2(v);
@@ -281,6 +297,8 @@ gemm_fp32_kernel(float* __restrict__ out, int out_stride, const float* __restric
             *aborted = 1;
         } else {
             add(mine + LOW_COL);
+#pragma unroll
+            for (int e = 0; e < BN; ++e) acc[e] *= 1.f / (1ll << 2 * UP);
 #pragma unroll
             for (int e = 0; e < BN; ++e) finite = finite && isfinite(acc[e]);
             if (!finite) *again = 1;                        // (what is behind the last row or column has the numbers of one that is not)

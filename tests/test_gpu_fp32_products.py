@@ -37,6 +37,38 @@ def test_product(m, n, k, x_more, out_more, spread):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("k", [512, 896, 1536])
+@pytest.mark.parametrize("spread", [4, 15, 30])
+def test_numbers_of_many_sizes(k, spread):
+    """At a size that goes through here, with numbers spread over 8 to 60 powers of two: the error as a whole is no larger than that of plain
+    32-bit sums (0.2 to 0.85 of it)."""
+    o, m, n = ops(), 640, 1152
+    g = torch.Generator().manual_seed(k + spread)
+    make = lambda r: torch.randn(r, k, generator=g) * torch.exp2(torch.randint(-spread, spread + 1, (r, k), generator=g).float())   # noqa: E731
+    x, w, out = make(m).cuda(), make(n).cuda(), torch.empty(m, n, device="cuda")
+    assert o.prefer_gemm_fp32(m, n, k)
+    o.gemm_fp32(out, x, w, m, torch.zeros(1, dtype=torch.int32, device="cuda"))
+    want = x.double() @ w.double().T
+    assert float((out.double() - want).norm()) <= float((torch.mm(x, w.T).double() - want).norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("small", ["x", "w"])
+@pytest.mark.parametrize("power", [-100, -112, -120, -126, -135])
+def test_the_smallest_numbers(small, power):
+    """Operands whose last bits lie below what a bf16 number holds, down to numbers that have lost bits themselves: the error is no larger
+    than that of plain 32-bit sums."""
+    o, m, n, k = ops(), 130, 260, 512
+    g = torch.Generator().manual_seed(-power)
+    make = lambda rows, tiny: (torch.randn(rows, k, generator=g).double() * 2.0 ** (power if tiny else 3)).float()      # noqa: E731
+    x, w = make(m, small == "x"), make(n, small == "w")
+    out, status = torch.empty(m, n, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    o.gemm_fp32(out, x.cuda(), w.cuda(), m, status)
+    want, plain = x.double() @ w.double().T, torch.mm(x.cuda(), w.cuda().T).cpu().double()
+    assert float((out.cpu().double() - want).norm()) <= float((plain - want).norm()) and int(status) == 0
+
+
+@pytest.mark.gpu
 def test_numbers_without_three_terms():
     """Infinities, NaN and numbers above the largest bf16 give what plain 32-bit sums give, and reach no other row or column."""
     o = ops()
