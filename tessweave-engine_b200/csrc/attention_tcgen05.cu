@@ -582,6 +582,10 @@ TW_EXPORT int tw_attn_prefill_tc5_supported(int page_size) {
     return (BN % page_size == 0 || page_size % BN == 0) ? 1 : 0;
 }
 
+// 1 if the compiler gave the kernel the registers that its roles are split from, 0 if not (the shape belongs to the mma.sync kernel then),
+// a negative number if the driver could not say.
+TW_EXPORT int tw_attn_prefill_tc5_built() { return tw_registers_are<attn_prefill_tc5_kernel>(LAUNCH_REGS); }
+
 // Attention for the requests of the batch that bring several tokens (with skip_single, requests
 // with one token are left to the decode kernel).  q [tokens, Hq * D] and out [tokens, Hq * D] are
 // bf16 with 16-byte aligned rows; the cache is [pages, Hkv, page_size, D] bf16 (values and out: heads of DV).  `row_tiles`: the sum of
@@ -602,10 +606,8 @@ TW_EXPORT int tw_attn_prefill_tc5(void* out, int out_stride, const void* q, int 
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return (int)e;
-        cudaFuncAttributes built;
-        e = cudaFuncGetAttributes(&built, attn_prefill_tc5_kernel);
-        if (e != cudaSuccess) return (int)e;
-        if (built.numRegs != LAUNCH_REGS) return (int)cudaErrorInvalidConfiguration;       // the warps would wait for registers that are not there
+        const int built = tw_attn_prefill_tc5_built();
+        if (built != 1) return built < 0 ? -built : (int)cudaErrorInvalidConfiguration;
         attr_set = true;
     }
     const int box_rows = page_size < BN ? page_size : BN;

@@ -249,6 +249,17 @@ static inline int tw_allow_shared() {
     return 0;
 }
 
+// Whether the compiler gave a kernel the registers a thread that its roles are split from (setmaxnreg): with others its warps would wait
+// for registers that are not there.  1, 0, or the driver's error as a negative number.
+template <auto KERNEL>
+static inline int tw_registers_are(int wanted) {
+    cudaFuncAttributes built;
+    const cudaError_t e = cudaFuncGetAttributes(&built, KERNEL);
+    if (e == cudaSuccess) return built.numRegs == wanted ? 1 : 0;
+    cudaGetLastError();
+    return -(int)e;
+}
+
 // Launch `kernel` on `stream`, allowing it to be scheduled before its predecessor has finished
 // (the kernel itself waits where it must), optionally as clusters of `cluster_x` blocks.
 //

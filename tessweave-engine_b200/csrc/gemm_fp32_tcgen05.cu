@@ -338,6 +338,10 @@ gemm_fp32_kernel(float* __restrict__ out, int out_stride, const float* __restric
 
 }  // namespace
 
+// 1 if the compiler gave the kernel the registers that its roles are split from, 0 if not (the product belongs to the library then), a
+// negative number if the driver could not say.
+TW_EXPORT int tw_gemm_fp32_built() { return tw_registers_are<gemm_fp32_kernel>(LAUNCH_REGS); }
+
 // out[m, n] = x[m, k] @ w[n, k].T, fp32; rows of x and w on 16-byte boundaries, k a multiple of 4.
 TW_EXPORT int tw_gemm_fp32(float* out, int out_stride, const float* x, int x_stride, const float* w, int w_stride, int m, int n, int k,
                            int* status, cudaStream_t stream) {
@@ -347,11 +351,12 @@ TW_EXPORT int tw_gemm_fp32(float* out, int out_stride, const float* x, int x_str
     const long long blocks = ((long long)(m + BM - 1) / BM) * ((n + BN - 1) / BN);
     if (blocks > 0x7fffffffll) return (int)cudaErrorInvalidValue;
     if (const int e = tw_allow_shared<gemm_fp32_kernel, SMEM>()) return e;
-    static const int built = [] {
-        cudaFuncAttributes a;
-        return cudaFuncGetAttributes(&a, gemm_fp32_kernel) == cudaSuccess ? a.numRegs : 0;
-    }();
-    if (built != LAUNCH_REGS) return (int)cudaErrorInvalidConfiguration;        // the warps would wait for registers that are not there
+    static std::atomic<bool> known{false};
+    if (!known.load(std::memory_order_relaxed)) {
+        const int built = tw_gemm_fp32_built();
+        if (built != 1) return built < 0 ? -built : (int)cudaErrorInvalidConfiguration;
+        known.store(true, std::memory_order_relaxed);
+    }
     return tw_launch(gemm_fp32_kernel, dim3((unsigned)blocks), dim3(THREADS), (size_t)SMEM, stream, 1, out, out_stride, x, x_stride, w,
                      w_stride, m, n, k, status);
 }

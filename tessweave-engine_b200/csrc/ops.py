@@ -54,6 +54,22 @@ def _ptr(t: torch.Tensor | None) -> c_void_p:
     return c_void_p(0 if t is None else t.data_ptr())
 
 
+_built: dict[tuple, bool] = {}
+
+
+def _built_as_wanted(lib_name: str, fn_name: str, defines=None) -> bool:
+    """Whether the compiler that built a library gave its kernel the registers that the kernel's roles are split from (asked of the
+    library once).  Where it did not the kernel cannot run and what it would serve goes another way."""
+    key = (fn_name, lib_name, timeline_enabled(), *(defines.items() if defines else ()))
+    known = _built.get(key)
+    if known is None:
+        answer = getattr(load_library(lib_name, defines), fn_name)()
+        if answer < 0:
+            return True         # (the driver could not say: the launch will tell why)
+        known = _built[key] = answer == 1
+    return known
+
+
 def _stream() -> c_void_p:
     # the raw handle of torch's current stream (what torch.cuda.current_stream().cuda_stream gives, without
     # building a Stream object for every launch)
@@ -882,6 +898,11 @@ def tcgen05_attention_supported(dtype: torch.dtype, head_dim: int, page_size: in
             and (128 % page_size == 0 or page_size % 128 == 0))
 
 
+def tcgen05_attention_built(head_dim: int, v_dim: int) -> bool:
+    """Whether the tcgen05 prefill attention of these head sizes, as it was compiled here, can run."""
+    return _built_as_wanted("attention_tcgen05", "tw_attn_prefill_tc5_built", head_size_defines(head_dim, v_dim))
+
+
 TCGEN05_ATTENTION_MIN_TOKENS = 128
 
 
@@ -1498,6 +1519,11 @@ def prefer_gemm_fp32(m: int, n: int, k: int) -> bool:
     rows 51 and 72; 128 rows 3,584 x 4,608 118 and 115, 256 rows 117 and 154; 64 rows 896 x 9,728 37 and 45, 256 rows 63 and 115;
     256 rows 4,864 x 896 137 and 127, 777 rows 135 and 202."""
     return m >= 128 and m * n >= 640 * 1024 and k >= 256
+
+
+def gemm_fp32_built() -> bool:
+    """Whether ``gemm_fp32``, as it was compiled here, can run."""
+    return _built_as_wanted("gemm_fp32_tcgen05", "tw_gemm_fp32_built")
 
 
 def gemm_fp32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:

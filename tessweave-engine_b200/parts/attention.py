@@ -66,7 +66,8 @@ class PagedSoftmaxMixer(Mixer):
             # does not take, stay on the mma.sync kernel, which starts faster
             prefill, more = ops.attention_prefill, self._terms()
             if (not self.score_terms and self.scale > 0
-                    and ops.prefer_tcgen05_attention(self.runtime.dtype, self.head_dim, cache.k_pages.shape[2], ctx.max_q_len, self.v_dim)):
+                    and ops.prefer_tcgen05_attention(self.runtime.dtype, self.head_dim, cache.k_pages.shape[2], ctx.max_q_len, self.v_dim)
+                    and ops.tcgen05_attention_built(self.head_dim, self.v_dim)):
                 prefill, beside = ops.attention_prefill_tcgen05, True
                 more["host_q_len"] = None if ctx.fixed_shape else ctx.host_q_len or None
                 if singles:     # (the buffers may be cleared when they are made: not between two kernels that run side by side)

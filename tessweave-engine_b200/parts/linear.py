@@ -112,7 +112,7 @@ def linear(ctx, name: str, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dt
         ops.gemm_narrow(out, x, w, m)
         return out
     if (x.dtype == torch.float32 and dtype == torch.float32 and bias is None and x.is_cuda and ops.prefer_gemm_fp32(m, n, w.shape[1])
-            and ops.gemm_fp32_supported(x, w)):
+            and ops.gemm_fp32_supported(x, w) and ops.gemm_fp32_built()):
         out = ctx.workspace.get(name, (m, n), dtype)
         ops.gemm_fp32(out, x, w, m, ctx.status)
         return out
