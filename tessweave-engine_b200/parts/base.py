@@ -169,7 +169,7 @@ class Workspace:
         """The buffer ``name`` with at least ``shape`` elements.  ``zero`` fills it with zeros when it
         is (re)allocated -- for state that kernels keep zero between launches, such as counters."""
         name = self.prefix + name
-        key = (name, shape, dtype)
+        key = (name, tuple(shape), dtype)
         view = self._views.get(key)
         if view is not None:
             return view

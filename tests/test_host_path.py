@@ -28,5 +28,7 @@ def test_workspace_views_follow_their_buffers():
     for n in range(1, 3 * Workspace.MAX_VIEWS):
         ws.get("y", (n,), torch.float32)
     assert len(ws._views) <= Workspace.MAX_VIEWS
+    listed = ws.get("w", [2, 3], torch.float32)                     # a shape in a list, or a torch.Size
+    assert listed.shape == (2, 3) and ws.get("w", listed.shape, torch.float32).data_ptr() == listed.data_ptr()
     zeros = ws.get("z", (4,), torch.int32, zero=True)
     assert int(zeros.sum()) == 0
