@@ -12,6 +12,8 @@ def test_settings_follow_the_environment(monkeypatch):
     assert setting("TESSWEAVE_PDL", "1") == "0"
     monkeypatch.setenv("TESSWEAVE_PDL", "")
     assert setting("TESSWEAVE_PDL", "1") == ""
+    monkeypatch.setattr("os.environ", {"TESSWEAVE_PDL": "2"})       # another mapping in the environment's place
+    assert setting("TESSWEAVE_PDL", "1") == "2" and setting("PATH") is None
 
 
 def test_workspace_views_follow_their_buffers():
