@@ -66,7 +66,7 @@ constexpr int Q_BYTES = NQ * KB * BLK;
 constexpr int K_STAGE_BYTES = KB * BLK, V_STAGE_BYTES = VB * BLK;
 constexpr int SMEM_TILES = Q_BYTES + KV_STAGES * (K_STAGE_BYTES + V_STAGE_BYTES);
 constexpr int SMEM = SMEM_TILES + 1024 /* alignment slack */ + 256 /* barriers */;
-constexpr int THREADS = 384;                  // warps 0-3 / 4-7: softmax of tile 0 / 1, warps 8 / 9: copies of K / V, warps 10 / 11: MMAs of tile 0 / 1
+constexpr int THREADS = 384;                  // warps 0-3 / 4-7: softmax of tile 0 / 1, warps 8 / 9: copies of K / V, warp 10: every MMA; warp 11 helps with the query rows and fills up the group that gives registers back
 constexpr int K_WARP = 8, V_WARP = 9, MMA_WARP = 10;
 // A softmax thread holds a row of 128 scores; the others need few registers.  256 x 200 + 128 x 104 = 384 x 168, which the
 // block is launched with.
@@ -80,7 +80,7 @@ constexpr float RESCALE_THRESHOLD = 8.f;      // log2 units
 // -DTW_TRACE: block (0, 0, 0) records clock64() at the hand-over points of its roles, for a
 // timeline of one block (tw_attn_tc5_trace_ptr gives the buffer).  Off in the product.
 #ifdef TW_TRACE
-constexpr int TRACE_SLOTS = 12, TRACE_TILES = 80, TRACE_ROLES = 12;     // a role: a softmax warp, 8 both MMA warps, 9 and 10 the copies, 11 the block
+constexpr int TRACE_SLOTS = 12, TRACE_TILES = 80, TRACE_ROLES = 12;     // a role: a softmax warp, 8 the MMA warp, 9 and 10 the copies, 11 the block
 __device__ long long g_trace[TRACE_ROLES * TRACE_TILES * TRACE_SLOTS];
 #define TW_TRACE_AT(role, tile, slot)                                                              \
     do {                                                                                           \
